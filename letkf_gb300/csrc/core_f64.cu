@@ -1,5 +1,10 @@
 // core_f64.cu -- FP64 plain form of letkf_core on the GPU.
 //
+// For k <= 64 core_f64_ns.cu answers every point whose spectrum allows it and
+// this kernel takes the ones left (few or none; their share is what the ring,
+// SPEEDY and regional workloads measure as 5 to 11 us of an idle launch); for
+// k > 64 it takes all.
+//
 // One CTA per grid point (persistent over the batch).  The k x k work matrix
 // lives in shared memory; the steps are those of common/common_letkf.f90:50-243:
 //   hdxb_rinv weighting (:101-113) and the Gram DGEMM (:117) accumulated in
@@ -134,7 +139,8 @@ __global__ void __launch_bounds__(F64_NT) core_f64_kernel(int n, int npts, const
                                                            const double* __restrict__ rloc,
                                                            const double* __restrict__ dep, double* parm_infl,
                                                            double* trans, double* transm, double* pao,
-                                                           int rdiag_wloc, double minfl, int* status) {
+                                                           int rdiag_wloc, double minfl, int* status,
+                                                           int pending_only) {
   extern __shared__ __align__(16) double sm[];
   double* Zm = sm;               // n*n, column-major, ld = n
   double* d = Zm + n * n;        // n
@@ -157,6 +163,8 @@ __global__ void __launch_bounds__(F64_NT) core_f64_kernel(int n, int npts, const
 #define E(i) e[(i)-1]
 
   for (int p = blockIdx.x; p < npts; p += gridDim.x) {
+    if (pending_only && status[p] != LETKF_PENDING) continue;
+    __syncthreads();  // every thread has read the status before it is set
     const int64_t r0 = offs[p];
     const int L = (int)(offs[p + 1] - r0);
     double infl = parm_infl[p];
@@ -441,11 +449,22 @@ __global__ void __launch_bounds__(F64_NT) core_f64_kernel(int n, int npts, const
 #undef E
 }
 
+int launch_core_f64_ns(int, int, const int64_t*, const double*, const double*, const double*, const double*, double*,
+                       double*, double*, double*, int, double, int*, cudaStream_t);
+
 int launch_core_f64(int ne, int npts, const int64_t* offs, const double* rows, const double* rdiag,
                     const double* rloc, const double* dep, double* parm_infl, double* trans, double* transm,
                     double* pao, int rdiag_wloc, double minfl, int* status, cudaStream_t stream) {
   if (ne < 2 || ne > LETKF_MAX_NE || npts < 0) return ne > LETKF_MAX_NE ? LETKF_ERR_CAPACITY : LETKF_ERR_ARG;
   if (npts == 0) return LETKF_OK;
+  // k <= 64: the eigensolver only takes the points that the first launch leaves
+  // to it.  Above, that kernel's three FP64 matrices leave one CTA per SM or none.
+  const int ns = ne <= 64;
+  if (ns) {
+    const int st = launch_core_f64_ns(ne, npts, offs, rows, rdiag, rloc, dep, parm_infl, trans, transm, pao, rdiag_wloc,
+                                      minfl, status, stream);
+    if (st != LETKF_OK) return st;
+  }
   const size_t smem = f64_smem_doubles(ne) * sizeof(double);
   cudaError_t err = cudaFuncSetAttribute(core_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (err != cudaSuccess) return cuda_status(err);
@@ -457,7 +476,7 @@ int launch_core_f64(int ne, int npts, const int64_t* offs, const double* rows, c
   int grid = nsm * per_sm;
   if (grid > npts) grid = npts;
   core_f64_kernel<<<grid, F64_NT, smem, stream>>>(ne, npts, offs, rows, rdiag, rloc, dep, parm_infl, trans, transm,
-                                                   pao, rdiag_wloc, minfl, status);
+                                                   pao, rdiag_wloc, minfl, status, ns);
   note_launch();
   return cuda_status(cudaGetLastError());
 }
