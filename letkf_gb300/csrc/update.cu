@@ -1,94 +1,38 @@
-// update.cu -- ensemble update with the analysis weights (FP64 plain form).
+// update.cu -- ensemble update with the analysis weights (FP64 plain form) and
+// the relaxed update of the SCALE driver.
 //
 //   mean(p,v) = (x(p,1,v) + ... + x(p,ne,v)) / ne      speedy/common/common_speedy.f90:335-370
 //   xa(p,m,v) = mean + sum_k (x(p,k,v) - mean) * (trans(k,m) + transm(k))
 //                                                     speedy/letkf/letkf_tools.f90:164-170,
 //                                                     scale/letkf/letkf_tools.f90:237-251 (beta = 1)
-// One CTA per point; the sum over k runs in the reference order.
+// and with relaxation (scale/letkf/letkf_tools.f90:215-268), per point and
+// variable, W_rlx = RTPP (1-a) W + a I (:1224-1237) or RTPS infl W with infl =
+// a sqrt(var_g / (var_a (k-1))) - a + 1 (:1240-1268), T = (W_rlx + transm 1^T)
+// beta + (1 - beta) I, xa = mean + xb' T; beta == 0 leaves mean + xb'; optional
+// clipping of the relative spread of one variable (Q_SPRD_MAX).
+//
+// One CTA per point, one kernel for both entry points (mode 0 with beta = 1 is
+// the plain update bit for bit).  The factors that do not depend on k stay out
+// of the sum: t(m) = sum_k x(k) W(k,m) and sum_k x(k) transm(k) once, then xa =
+// mean + beta (fac t + tx) + (1 - beta) x(m): one multiply-add per element of W
+// and variable where forming each weight first took five FP64 operations, and
+// increments added up before they meet the mean.
+//
+// Bound: the FP64 pipe (1.2 TFLOP/s; a warp instruction takes 16 cycles of an
+// SM), so lanes are kept full: outputs (variable, member) are flattened over
+// the lanes, W is kept k-major with an odd row length (consecutive lanes read
+// consecutive members and the transposing stores spread over the banks), and
+// the quadratic form of RTPS goes over unordered pairs: x' Pa x = sum_d sum_i
+// x(i) D(d,i) x(i+d mod k), D(d,i) = Pa(i,i+d) + Pa(i+d,i), d = 0..k/2, formed
+// once per point for all variables, half the products of the full form and
+// every lane busy.  RTPS, 20,000 points, k = 50, 11 variables: 7.77 -> 2.89 ms
+// (FP64 pipe 78 % busy).
 #include "letkf_common.cuh"
 
 namespace letkf {
 
 constexpr int UPD_NT = 128;
-
-// Points p0 .. p0+cnt-1 of arrays holding npts_total points; trans / transm
-// are indexed from p0.
-__global__ void __launch_bounds__(UPD_NT) update_f64_kernel(int n, int npts_total, int p0, int cnt, int nv,
-                                                             const double* __restrict__ xb,
-                                                             const double* __restrict__ trans,
-                                                             const double* __restrict__ transm, double* xa) {
-  extern __shared__ __align__(16) double su[];
-  double* W = su;            // n*n
-  double* tm = W + n * n;    // n
-  double* xp = tm + n;       // nv*n
-  double* mean = xp + nv * n;  // nv
-  const int tid = threadIdx.x;
-  for (int pl = blockIdx.x; pl < cnt; pl += gridDim.x) {
-    const int p = p0 + pl;
-    __syncthreads();
-    for (int idx = tid; idx < n * n; idx += UPD_NT) W[idx] = trans[(size_t)pl * n * n + idx];
-    for (int k = tid; k < n; k += UPD_NT) tm[k] = transm ? transm[(size_t)pl * n + k] : 0.0;
-    for (int t = tid; t < nv * n; t += UPD_NT) {
-      const int v = t / n, m = t - v * n;
-      xp[t] = xb[((size_t)v * npts_total + p) * n + m];
-    }
-    __syncthreads();
-    for (int v = tid; v < nv; v += UPD_NT) {
-      double s = xp[v * n];
-      for (int m = 1; m < n; m++) s = s + xp[v * n + m];
-      mean[v] = s / (double)n;
-    }
-    __syncthreads();
-    for (int t = tid; t < nv * n; t += UPD_NT) xp[t] = xp[t] - mean[t / n];
-    __syncthreads();
-    for (int t = tid; t < nv * n; t += UPD_NT) {
-      const int v = t / n, m = t - v * n;
-      double a = mean[v];
-      if (transm) {
-        for (int k = 0; k < n; k++) a = a + xp[v * n + k] * (W[(size_t)m * n + k] + tm[k]);
-      } else {
-        for (int k = 0; k < n; k++) a = a + xp[v * n + k] * W[(size_t)m * n + k];
-      }
-      xa[((size_t)v * npts_total + p) * n + m] = a;
-    }
-  }
-}
-
-int launch_update_f64_range(int ne, int npts_total, int p0, int cnt, int nv, const double* xb, const double* trans,
-                            const double* transm, double* xa, cudaStream_t stream) {
-  if (ne < 2 || npts_total < 0 || p0 < 0 || cnt < 0 || p0 + cnt > npts_total || nv < 1) return LETKF_ERR_ARG;
-  if (ne > LETKF_MAX_NE) return LETKF_ERR_CAPACITY;
-  if (cnt == 0) return LETKF_OK;
-  const int npts = cnt;
-  const size_t smem = sizeof(double) * ((size_t)ne * ne + ne + (size_t)nv * ne + nv);
-  cudaError_t err = cudaFuncSetAttribute(update_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (err != cudaSuccess) return cuda_status(err);
-  int dev = 0, nsm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  int grid = nsm * 8;
-  if (grid > npts) grid = npts;
-  update_f64_kernel<<<grid, UPD_NT, smem, stream>>>(ne, npts_total, p0, cnt, nv, xb, trans, transm, xa);
-  note_launch();
-  return cuda_status(cudaGetLastError());
-}
-
-int launch_update_f64(int ne, int npts, int nv, const double* xb, const double* trans, const double* transm,
-                      double* xa, cudaStream_t stream) {
-  return launch_update_f64_range(ne, npts, 0, npts, nv, xb, trans, transm, xa, stream);
-}
-
-}  // namespace letkf
-
-// ---------------------------------------------------------------------------
-// Relaxed update of the SCALE driver (scale/letkf/letkf_tools.f90:215-268):
-// per point and variable, W_rlx = RTPP (1-a) W + a I  (:1224-1237) or
-// RTPS infl W with infl = a sqrt(var_g / (var_a (k-1))) - a + 1 (:1240-1268),
-// T = (W_rlx + transm 1^T) beta + (1 - beta) I, xa = mean + xb' T; beta == 0
-// leaves mean + xb'; optional clipping of the relative spread of one variable
-// (Q_SPRD_MAX).  Each element is formed with the reference's operations in
-// its order, so mode 0 with beta = 1 equals update_f64_kernel bit for bit.
-namespace letkf {
+constexpr int UPD_VC = 16;  // variables handled at a time
 
 struct RelaxArgs {
   int mode;           // 0 none, 1 RTPP, 2 RTPS
@@ -99,108 +43,225 @@ struct RelaxArgs {
   double* rtps_infl;  // [nv][npts] or NULL
 };
 
-__global__ void __launch_bounds__(UPD_NT) update_relax_f64_kernel(int n, int npts, int nv, const double* __restrict__ xb,
-                                                                   const double* __restrict__ trans,
-                                                                   const double* __restrict__ transm,
-                                                                   const double* __restrict__ pao, RelaxArgs r,
-                                                                   double* xa) {
+// doubles of shared memory: W, D (RTPS), transm, x and the products of a chunk
+// of variables, mean / factor / beta / x . transm, the clipped variable
+__host__ __device__ inline size_t upd_smem_doubles(int n, int nv, int mode) {
+  const int vc = nv < UPD_VC ? nv : UPD_VC;
+  const size_t d = mode == 2 ? (size_t)(n / 2 + 1) * n + (size_t)vc * n : 0;
+  return (size_t)n * (n | 1) + d + n + (size_t)vc * n + 4 * (size_t)vc + n;
+}
+
+// Points p0 .. p0+cnt-1 of arrays holding npts points; trans / transm / pao
+// are indexed from p0.
+__global__ void __launch_bounds__(UPD_NT) update_f64_kernel(int n, int npts, int p0, int cnt, int nv,
+                                                             const double* __restrict__ xb,
+                                                             const double* __restrict__ trans,
+                                                             const double* __restrict__ transm,
+                                                             const double* __restrict__ pao, RelaxArgs r, double* xa) {
   extern __shared__ __align__(16) double su[];
-  double* W = su;                  // n*n
-  double* Pa = W + n * n;          // n*n (RTPS)
-  double* tm = Pa + n * n;         // n
-  double* xp = tm + n;             // nv*n
-  double* mean = xp + nv * n;      // nv
-  double* fac = mean + nv;         // nv: RTPS inflation
-  double* bet = fac + nv;          // nv
-  double* outv = bet + nv;         // nv*n analysis (for the spread clip)
-  const int tid = threadIdx.x;
-  for (int p = blockIdx.x; p < npts; p += gridDim.x) {
+  const int ld = n | 1, nh = n / 2, vcm = nv < UPD_VC ? nv : UPD_VC;
+  double* W = su;                          // [k][ld]
+  double* D = W + (size_t)n * ld;          // [nh + 1][n] (RTPS)
+  double* prod = D + (r.mode == 2 ? (size_t)(nh + 1) * n : 0);  // [vcm][n] (RTPS)
+  double* tm = prod + (r.mode == 2 ? (size_t)vcm * n : 0);      // [n]
+  double* xp = tm + n;                     // [vcm][n]
+  double* mean = xp + (size_t)vcm * n;     // [vcm] each
+  double* fac = mean + vcm;
+  double* bet = fac + vcm;
+  double* tx = bet + vcm;
+  double* qv = tx + vcm;                   // [n]
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  for (int pl = blockIdx.x; pl < cnt; pl += gridDim.x) {
+    const int p = p0 + pl;
     __syncthreads();
+    const double* Tp = trans + (size_t)pl * n * n;
+#pragma unroll 4
     for (int idx = tid; idx < n * n; idx += UPD_NT) {
-      W[idx] = trans[(size_t)p * n * n + idx];
-      if (r.mode == 2) Pa[idx] = pao[(size_t)p * n * n + idx];
+      const int m = idx / n, k = idx - m * n;
+      W[k * ld + m] = Tp[idx];
     }
-    for (int k = tid; k < n; k += UPD_NT) tm[k] = transm ? transm[(size_t)p * n + k] : 0.0;
-    for (int t = tid; t < nv * n; t += UPD_NT) {
-      const int v = t / n, m = t - v * n;
-      xp[t] = xb[((size_t)v * npts + p) * n + m];
+    if (transm)
+      for (int k = tid; k < n; k += UPD_NT) tm[k] = transm[(size_t)pl * n + k];
+    if (r.mode == 2) {
+      // first the element of each pair that starts it, then the other one onto it
+      const double* Pp = pao + (size_t)pl * n * n;
+#pragma unroll 4
+      for (int idx = tid; idx < n * n; idx += UPD_NT) {
+        const int i = idx / n, j = idx - i * n;
+        const int d = j >= i ? j - i : j - i + n;
+        if (2 * d < n || (2 * d == n && i < j)) D[d * n + i] = Pp[idx];
+        if (2 * d == n && i > j) D[d * n + i] = 0.0;
+      }
+      __syncthreads();
+#pragma unroll 4
+      for (int idx = tid; idx < n * n; idx += UPD_NT) {
+        const int i = idx / n, j = idx - i * n;
+        const int d = i >= j ? i - j : i - j + n;
+        if (d != 0 && (2 * d < n || (2 * d == n && j < i))) D[d * n + j] += Pp[idx];
+      }
     }
-    __syncthreads();
-    for (int v = tid; v < nv; v += UPD_NT) {
-      double s = xp[v * n];
-      for (int m = 1; m < n; m++) s = s + xp[v * n + m];
-      mean[v] = s / (double)n;
-      bet[v] = r.beta ? r.beta[(size_t)v * npts + p] : 1.0;
-    }
-    __syncthreads();
-    for (int t = tid; t < nv * n; t += UPD_NT) xp[t] = xp[t] - mean[t / n];
-    __syncthreads();
-    // RTPS factor, one warp per variable: lanes split k so the Pa(k, m) reads of
-    // a column are consecutive; beta == 0 skips weight_RTPS (factor 1)
-    {
-      const int lane = tid & 31;
-      for (int v = tid >> 5; v < nv; v += UPD_NT / 32) {
-        double f = 1.0;
-        if (r.mode == 2 && bet[v] != 0.0) {
+    for (int v0 = 0; v0 < nv; v0 += UPD_VC) {
+      const int vc = min(UPD_VC, nv - v0), total = vc * n;
+      if (v0) __syncthreads();
+      for (int t = tid; t < total; t += UPD_NT) {
+        const int v = t / n;
+        xp[t] = xb[((size_t)(v0 + v) * npts + p) * n + (t - v * n)];
+      }
+      __syncthreads();
+      for (int v = tid; v < vc; v += UPD_NT) {
+        double s = xp[v * n];
+        for (int m = 1; m < n; m++) s = s + xp[v * n + m];
+        mean[v] = s / (double)n;
+        bet[v] = r.beta ? r.beta[(size_t)(v0 + v) * npts + p] : 1.0;
+        fac[v] = 1.0;
+      }
+      __syncthreads();
+      for (int t = tid; t < total; t += UPD_NT) xp[t] = xp[t] - mean[t / n];
+      __syncthreads();
+      const int nch = (total + 31) / 32;  // 32 outputs (variable, member) a chunk, chunks over the warps
+      if (r.mode == 2) {
+        for (int c = wid; c < nch; c += UPD_NT / 32) {
+          const int t = min(32 * c + lane, total - 1);
+          const int v = t / n, i = t - v * n;
           const double* x = xp + v * n;
-          double var_a = 0.0, var_g = 0.0;
-          for (int m = 0; m < n; m++) {
-            double part = 0.0;
-            for (int k = lane; k < n; k += 32) part = part + x[k] * Pa[(size_t)m * n + k];
-            var_a = var_a + part * x[m];
+          double a = 0.0;
+          int j = i;
+#pragma unroll 4
+          for (int d = 0; d <= nh; d++) {
+            a = fma(D[d * n + i], x[j], a);
+            j = j + 1 == n ? 0 : j + 1;
           }
-          for (int m = lane; m < n; m += 32) var_g = var_g + x[m] * x[m];
-          var_a = warp_sum(var_a);
-          var_g = warp_sum(var_g);
-          if (var_g > 0.0 && var_a > 0.0) f = r.alpha * sqrt(var_g / (var_a * (double)(n - 1))) - r.alpha + 1.0;
+          if (32 * c + lane < total) prod[t] = a * x[i];
         }
-        if (lane == 0) {
-          if (r.mode == 2 && r.rtps_infl) r.rtps_infl[(size_t)v * npts + p] = f;
-          fac[v] = f;
+        __syncthreads();
+      }
+      // sums over the members by eight lanes per variable (a full warp would
+      // spend more FP64 slots on the reduction than on the sum)
+      if (transm || r.mode == 2) {
+        for (int vb = 4 * wid; vb < vc; vb += UPD_NT / 8) {
+          const int v = min(vb + (lane >> 3), vc - 1);
+          const double* x = xp + v * n;
+          double sx = 0.0, va = 0.0, vg = 0.0;
+          if (transm)
+            for (int k = lane & 7; k < n; k += 8) sx = fma(x[k], tm[k], sx);
+          if (r.mode == 2)
+            for (int k = lane & 7; k < n; k += 8) {
+              va = va + prod[v * n + k];
+              vg = fma(x[k], x[k], vg);
+            }
+#pragma unroll
+          for (int o = 4; o > 0; o >>= 1) {
+            if (transm) sx += __shfl_xor_sync(0xffffffffu, sx, o);
+            if (r.mode == 2) {
+              va += __shfl_xor_sync(0xffffffffu, va, o);
+              vg += __shfl_xor_sync(0xffffffffu, vg, o);
+            }
+          }
+          if ((lane & 7) == 0 && vb + (lane >> 3) < vc) {
+            tx[v] = sx;
+            if (r.mode == 2) {  // beta == 0 skips weight_RTPS (factor 1)
+              double f = 1.0;
+              if (bet[v] != 0.0 && vg > 0.0 && va > 0.0)
+                f = r.alpha * sqrt(vg / (va * (double)(n - 1))) - r.alpha + 1.0;
+              fac[v] = f;
+              if (r.rtps_infl) r.rtps_infl[(size_t)(v0 + v) * npts + p] = f;
+            }
+          }
         }
       }
-    }
-    __syncthreads();
-    for (int t = tid; t < nv * n; t += UPD_NT) {
-      const int v = t / n, m = t - v * n;
-      const double b = bet[v];
-      double a = mean[v];
-      if (b == 0.0) {
-        a = a + xp[t];
-      } else {
-        for (int k = 0; k < n; k++) {
-          double w = W[(size_t)m * n + k];
-          if (r.mode == 1) {
-            w = (1.0 - r.alpha) * w;
-            if (k == m) w = w + r.alpha;
-          } else if (r.mode == 2) {
-            w = w * fac[v];
+      __syncthreads();
+      const bool clip = r.q_sprd_max > 0.0 && r.q_var >= v0 && r.q_var < v0 + vc;
+      constexpr int U = 4;
+      for (int c0 = wid; c0 < nch; c0 += U * (UPD_NT / 32)) {
+        const int nu = min(U, (nch - c0 + UPD_NT / 32 - 1) / (UPD_NT / 32));
+        double a[U];
+        int vv[U], mm[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+          const int t = min(32 * (c0 + u * (UPD_NT / 32)) + lane, total - 1);
+          vv[u] = t / n;
+          mm[u] = t - vv[u] * n;
+          a[u] = 0.0;
+        }
+#pragma unroll 2
+        for (int k = 0; k < n; k++)
+#pragma unroll
+          for (int u = 0; u < U; u++)
+            if (u < nu) a[u] = fma(xp[vv[u] * n + k], W[k * ld + mm[u]], a[u]);
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+          if (u >= nu || 32 * (c0 + u * (UPD_NT / 32)) + lane >= total) continue;
+          const int v = vv[u], m = mm[u];
+          const double b = bet[v], x = xp[v * n + m];
+          double inc;
+          if (b == 0.0) {
+            inc = x;
+          } else {
+            inc = a[u];
+            if (r.mode == 1) inc = (1.0 - r.alpha) * inc + r.alpha * x;
+            if (r.mode == 2) inc = fac[v] * inc;
+            if (transm) inc = inc + tx[v];
+            if (b != 1.0) inc = b * inc + (1.0 - b) * x;
           }
-          w = (w + tm[k]) * b;
-          if (k == m) w = w + (1.0 - b);
-          a = a + xp[v * n + k] * w;
+          const double y = mean[v] + inc;
+          if (clip && v0 + v == r.q_var)
+            qv[m] = y;
+          else
+            xa[((size_t)(v0 + v) * npts + p) * n + m] = y;
         }
       }
-      outv[t] = a;
-    }
-    __syncthreads();
-    if (r.q_sprd_max > 0.0 && r.q_var >= 0 && r.q_var < nv && tid == 0) {
-      double* q = outv + r.q_var * n;
-      double qm = q[0];
-      for (int m = 1; m < n; m++) qm = qm + q[m];
-      qm = qm / (double)n;
-      double sp = 0.0;
-      for (int m = 0; m < n; m++) sp = sp + (q[m] - qm) * (q[m] - qm);
-      sp = sqrt(sp / (double)(n - 1)) / qm;
-      if (sp > r.q_sprd_max)
-        for (int m = 0; m < n; m++) q[m] = qm + (q[m] - qm) * r.q_sprd_max / sp;
-    }
-    __syncthreads();
-    for (int t = tid; t < nv * n; t += UPD_NT) {
-      const int v = t / n, m = t - v * n;
-      xa[((size_t)v * npts + p) * n + m] = outv[t];
+      if (clip) {
+        __syncthreads();
+        if (wid == 0) {
+          double s = 0.0;
+          for (int m = lane; m < n; m += 32) s = s + qv[m];
+          const double qm = warp_sum(s) / (double)n;
+          double sp = 0.0;
+          for (int m = lane; m < n; m += 32) sp = fma(qv[m] - qm, qv[m] - qm, sp);
+          sp = sqrt(warp_sum(sp) / (double)(n - 1)) / qm;
+          const double f = r.q_sprd_max / sp;
+          for (int m = lane; m < n; m += 32) {
+            double y = qv[m];
+            if (sp > r.q_sprd_max) y = qm + (y - qm) * f;
+            xa[((size_t)r.q_var * npts + p) * n + m] = y;
+          }
+        }
+      }
     }
   }
+}
+
+static int launch_update(int ne, int npts, int p0, int cnt, int nv, const double* xb, const double* trans,
+                         const double* transm, const double* pao, const RelaxArgs& r, double* xa,
+                         cudaStream_t stream) {
+  const size_t smem = sizeof(double) * upd_smem_doubles(ne, nv, r.mode);
+  const cudaError_t err =
+      cudaFuncSetAttribute(update_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (err != cudaSuccess) return cuda_status(err);
+  int dev = 0, nsm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  // resident CTAs: shared memory, at most 8 (32 warps cover the FP64 unit's latency)
+  int per_sm = (int)((size_t)(220 * 1024) / (smem + 1024));
+  per_sm = per_sm < 1 ? 1 : per_sm > 8 ? 8 : per_sm;
+  const int grid = cnt < nsm * per_sm ? cnt : nsm * per_sm;
+  update_f64_kernel<<<grid, UPD_NT, smem, stream>>>(ne, npts, p0, cnt, nv, xb, trans, transm, pao, r, xa);
+  note_launch();
+  return cuda_status(cudaGetLastError());
+}
+
+int launch_update_f64_range(int ne, int npts_total, int p0, int cnt, int nv, const double* xb, const double* trans,
+                            const double* transm, double* xa, cudaStream_t stream) {
+  if (ne < 2 || npts_total < 0 || p0 < 0 || cnt < 0 || p0 + cnt > npts_total || nv < 1) return LETKF_ERR_ARG;
+  if (ne > LETKF_MAX_NE) return LETKF_ERR_CAPACITY;
+  if (cnt == 0) return LETKF_OK;
+  const RelaxArgs r = {0, 0.0, nullptr, -1, 0.0, nullptr};
+  return launch_update(ne, npts_total, p0, cnt, nv, xb, trans, transm, nullptr, r, xa, stream);
+}
+
+int launch_update_f64(int ne, int npts, int nv, const double* xb, const double* trans, const double* transm,
+                      double* xa, cudaStream_t stream) {
+  return launch_update_f64_range(ne, npts, 0, npts, nv, xb, trans, transm, xa, stream);
 }
 
 // relax_beta (scale/letkf/letkf_tools.f90:1182-1220): 0 for the q variables
@@ -248,17 +309,7 @@ extern "C" int letkf_update_relax_f64(int ne, int npts, int nv, const double* xb
   r.q_var = rd->q_var;
   r.q_sprd_max = rd->q_sprd_max;
   r.rtps_infl = rtps_infl;
-  const size_t smem = sizeof(double) * (2 * (size_t)ne * ne + ne + 2 * (size_t)nv * ne + 3 * (size_t)nv);
-  cudaError_t err =
-      cudaFuncSetAttribute(update_relax_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (err != cudaSuccess) return cuda_status(err);
-  int dev = 0, nsm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  const int grid = npts < nsm * 8 ? npts : nsm * 8;
-  update_relax_f64_kernel<<<grid, UPD_NT, smem, (cudaStream_t)stream>>>(ne, npts, nv, xb, trans, transm, pao, r, xa);
-  note_launch();
-  return cuda_status(cudaGetLastError());
+  return launch_update(ne, npts, 0, npts, nv, xb, trans, transm, pao, r, xa, (cudaStream_t)stream);
 }
 
 extern "C" int letkf_relax_beta(int npts, int nv, const double* ri, const double* rj, const double* rlev, int q_lo,
