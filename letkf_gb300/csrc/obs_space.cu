@@ -13,63 +13,94 @@
 namespace letkf {
 
 constexpr int OSA_NT = 128;
+constexpr int OSA_T = 64;       // members and weights of a staged tile
+constexpr int OSA_LD = OSA_T + 1;
 constexpr int EFSO_MAX_TERM = 8;
 constexpr int EFSO_MAX_NV = 16;
+constexpr int EFSO_MC = 16;     // members of a staged tile of 32 observations
+constexpr int EFSO_GROUP = 8;   // grid points of a CTA at most
 
+// One CTA per observation location.  Bound: HBM for trans (k^2 doubles, read
+// once), as long as the reads are whole lines: tiles of 64 weights x 64
+// members go through shared memory (rows of trans are read along the weights,
+// the odd row length spreads the transposing stores over the banks), then a
+// thread sums half a tile of one member's weights.  A thread walking its own
+// member's row in global memory read 32 lines per warp instruction: 20,000
+// locations of k = 64 took 0.91 ms, now 0.23.
 __global__ void __launch_bounds__(OSA_NT) obs_analysis_kernel(int ne, int n, const double* __restrict__ trans,
                                                                const double* __restrict__ ybar,
                                                                const double* __restrict__ hdxf, double alpha,
                                                                const int* __restrict__ mode, double q_sprd_max,
                                                                double* anal, double* amean) {
   extern __shared__ double so[];
-  double* h = so;         // [ne] obshdxf(n, :)
-  double* a = so + ne;    // [ne] analysis members
-  const int tid = threadIdx.x;
+  double* h = so;               // [ne] obshdxf(n, :)
+  double* a = h + ne;           // [ne] analysis members
+  double* tile = a + ne;        // [OSA_T][OSA_LD] weight k0 + kk of member m0 + m
+  double* part = tile + OSA_T * OSA_LD;  // [OSA_T] second half's sums
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int m = tid % OSA_T, half = tid / OSA_T;
   for (int p = blockIdx.x; p < n; p += gridDim.x) {
-    __syncthreads();
-    for (int m = tid; m < ne; m += OSA_NT) h[m] = hdxf[(size_t)p * ne + m];
-    __syncthreads();
     const int md = mode ? mode[p] : 0;
     const double yb = ybar[p];
     const double* tp = trans + (size_t)p * ne * ne;
-    // thread per member m: it walks column m of trans (contiguous, stays in L1)
-    for (int m = tid; m < ne; m += OSA_NT) {
-      double v;
-      if (md == 1) {
-        v = yb + h[m];
-      } else {
-        v = yb;
-        for (int k = 0; k < ne; k++) {
-          double w = tp[(size_t)m * ne + k];
-          if (alpha != 0.0) {
-            w = (1.0 - alpha) * w;
-            if (k == m) w = w + alpha;
+    __syncthreads();
+    for (int i = tid; i < ne; i += OSA_NT) h[i] = hdxf[(size_t)p * ne + i];
+    if (md == 1) {
+      __syncthreads();
+      for (int i = tid; i < ne; i += OSA_NT) a[i] = yb + h[i];
+    } else {
+      for (int m0 = 0; m0 < ne; m0 += OSA_T) {
+        const int nm = min(OSA_T, ne - m0);
+        double v = 0.0;
+        for (int k0 = 0; k0 < ne; k0 += OSA_T) {
+          const int nk = min(OSA_T, ne - k0);
+          // all of a thread's part in flight before the tile's last readers are waited for
+          double r[OSA_T * OSA_T / OSA_NT];
+          const int kk = tid % OSA_T, mm = tid / OSA_T;
+          const double* src = tp + (size_t)(m0 + mm) * ne + k0 + kk;
+#pragma unroll
+          for (int i = 0; i < OSA_T * OSA_T / OSA_NT; i++) {
+            const int mi = mm + i * (OSA_NT / OSA_T);
+            r[i] = (kk < nk && mi < nm) ? src[(size_t)i * (OSA_NT / OSA_T) * ne] : 0.0;
           }
-          v = v + h[k] * w;
+          __syncthreads();
+#pragma unroll
+          for (int i = 0; i < OSA_T * OSA_T / OSA_NT; i++) tile[kk * OSA_LD + mm + i * (OSA_NT / OSA_T)] = r[i];
+          __syncthreads();
+          const int kb = half * (OSA_T / 2), ke = min(nk, kb + OSA_T / 2);
+          if (m < nm)
+#pragma unroll 4
+            for (int kk = kb; kk < ke; kk++) v = fma(h[k0 + kk], tile[kk * OSA_LD + m], v);
+        }
+        if (half == 1) part[m] = v;
+        __syncthreads();
+        // RTPP (:959-970) outside the sum: (1 - a) sum_k h(k) w(k, m) + a h(m)
+        if (half == 0 && m < nm) {
+          v = v + part[m];
+          if (alpha != 0.0) v = (1.0 - alpha) * v + alpha * h[m0 + m];
+          a[m0 + m] = yb + v;
         }
       }
-      a[m] = v;
     }
     __syncthreads();
-    if (tid == 0) {
-      double s = 0.0;
-      if (md == 1) {
-        s = yb;
-      } else {
-        for (int m = 0; m < ne; m++) s = s + a[m];
-        s = s / (double)ne;
+    if (tid < 32) {
+      double s = yb;
+      if (md != 1) {
+        double t = 0.0;
+        for (int i = lane; i < ne; i += 32) t = t + a[i];
+        s = warp_sum(t) / (double)ne;
         if (md == 2) {
           double sp = 0.0;
-          for (int m = 0; m < ne; m++) sp = sp + (a[m] - s) * (a[m] - s);
-          sp = sqrt(sp / (double)(ne - 1)) / s;
+          for (int i = lane; i < ne; i += 32) sp = fma(a[i] - s, a[i] - s, sp);
+          sp = sqrt(warp_sum(sp) / (double)(ne - 1)) / s;
           if (sp > q_sprd_max)
-            for (int m = 0; m < ne; m++) a[m] = s + (a[m] - s) * q_sprd_max / sp;
+            for (int i = lane; i < ne; i += 32) a[i] = s + (a[i] - s) * q_sprd_max / sp;
         }
       }
-      if (amean) amean[p] = s;
+      if (amean && lane == 0) amean[p] = s;
     }
     __syncthreads();
-    for (int m = tid; m < ne; m += OSA_NT) anal[(size_t)p * ne + m] = a[m];
+    for (int i = tid; i < ne; i += OSA_NT) anal[(size_t)p * ne + i] = a[i];
   }
 }
 
@@ -77,8 +108,19 @@ struct EfsoTerms {
   int term[EFSO_MAX_NV];
 };
 
-// one CTA per grid point: work1 in shared memory, one local observation per thread
-__global__ void __launch_bounds__(OSA_NT) efso_djdy_kernel(int ne, int npts, int nv, int nterm, EfsoTerms tv,
+// One CTA per group of neighbouring grid points: their work1 in shared memory
+// and the entries of all their lists flattened over the lanes, so short lists
+// fill the warps.  A lane sums one entry's products over the members (FP64
+// pipe: one multiply-add per member and term; the entry's rloc / rdiag is
+// applied to the sums), and the rows of the 32 observations of a warp go
+// through a tile of 16 members in shared memory, read as whole lines with the
+// next tile's loads in flight.  Bound: the FP64 pipe (1.2 TFLOP/s).  A thread
+// walking its own observation's row, one point per CTA, two more products per
+// member: 30,000 points with 50 local observations of k = 64 and 3 terms took
+// 2.55 ms, now 0.78 (FP64 pipe 69 % busy).
+template <int NTERM>
+__global__ void __launch_bounds__(OSA_NT) efso_djdy_kernel(int ne, int npts, int nv, int group,
+                                                            const __grid_constant__ EfsoTerms tv,
                                                             const int64_t* __restrict__ offs,
                                                             const int* __restrict__ idx,
                                                             const double* __restrict__ rdiag,
@@ -86,38 +128,100 @@ __global__ void __launch_bounds__(OSA_NT) efso_djdy_kernel(int ne, int npts, int
                                                             const double* __restrict__ hdxa,
                                                             const double* __restrict__ fcst,
                                                             const double* __restrict__ fcer, double* djdy) {
-  extern __shared__ double w1[];  // [nterm][ne]
-  const int tid = threadIdx.x;
-  for (int p = blockIdx.x; p < npts; p += gridDim.x) {
-    const int64_t l0 = offs[p], l1 = offs[p + 1];
-    if (l1 == l0) continue;
+  extern __shared__ double w1[];  // [group][NTERM][ne], then the warps' tiles [EFSO_MC][33]
+  __shared__ int64_t lo[EFSO_GROUP + 1];
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  double* tile = w1 + (size_t)group * NTERM * ne + wid * EFSO_MC * 33;
+  const int ngroup = (npts + group - 1) / group;
+  for (int g = blockIdx.x; g < ngroup; g += gridDim.x) {
+    const int p0 = g * group, np = min(group, npts - p0);
     __syncthreads();
-    for (int i = tid; i < nterm * ne; i += OSA_NT) w1[i] = 0.0;
-    __syncthreads();
-    for (int m = tid; m < ne; m += OSA_NT)
+    if (tid <= np) lo[tid] = offs[p0 + tid];
+    for (int t = tid; t < np * ne; t += OSA_NT) {
+      const int q = t / ne, m = t - q * ne;
+      double s[NTERM];
+#pragma unroll
+      for (int i = 0; i < NTERM; i++) s[i] = 0.0;
       for (int v = 0; v < nv; v++) {
-        const int t = tv.term[v];
-        if (t < 0) continue;
-        w1[t * ne + m] = w1[t * ne + m] + fcst[((size_t)v * npts + p) * ne + m] * fcer[(size_t)v * npts + p];
+        const double f = fcst[((size_t)v * npts + p0 + q) * ne + m] * fcer[(size_t)v * npts + p0 + q];
+#pragma unroll
+        for (int i = 0; i < NTERM; i++)
+          if (tv.term[v] == i) s[i] = s[i] + f;
       }
+#pragma unroll
+      for (int i = 0; i < NTERM; i++) w1[((size_t)q * NTERM + i) * ne + m] = s[i];
+    }
     __syncthreads();
-    for (int64_t l = l0 + tid; l < l1; l += OSA_NT) {
-      const int ob = idx[l];
-      const double rinv = 1.0 / rdiag[l], rl = rloc[l];  // one division per observation, not per member
-      double acc[EFSO_MAX_TERM];
+    const int64_t l0 = lo[0], l1 = lo[np];
+    for (int64_t lb = l0 + 32 * wid; lb < l1; lb += OSA_NT) {
+      const int64_t l = lb + lane;
+      const bool on = l < l1;
+      const int ob = on ? idx[l] : -1;
+      int q = 0;
+      while (q + 1 < np && l >= lo[q + 1]) q++;
+      const double* w = w1 + (size_t)q * NTERM * ne;
+      double acc[NTERM];
 #pragma unroll
-      for (int t = 0; t < EFSO_MAX_TERM; t++) acc[t] = 0.0;
-      for (int m = 0; m < ne; m++) {
-        const double hr = hdxa[(size_t)ob * ne + m] * rinv * rl;
+      for (int i = 0; i < NTERM; i++) acc[i] = 0.0;
+      // rows 2 r and 2 r + 1 of the tile by the two half warps, lane % 16 the member
+      double nx[16];
+      auto load = [&](int m0) {
 #pragma unroll
-        for (int t = 0; t < EFSO_MAX_TERM; t++)
-          if (t < nterm) acc[t] = acc[t] + w1[t * ne + m] * hr;
+        for (int r = 0; r < 16; r++) {
+          const int o = __shfl_sync(0xffffffffu, ob, 2 * r + (lane >> 4));
+          const int m = m0 + (lane & 15);
+          nx[r] = (o >= 0 && m < ne) ? hdxa[(size_t)o * ne + m] : 0.0;
+        }
+      };
+      load(0);
+      for (int m0 = 0; m0 < ne; m0 += EFSO_MC) {
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < 16; r++) tile[(lane & 15) * 33 + 2 * r + (lane >> 4)] = nx[r];
+        __syncwarp();
+        if (m0 + EFSO_MC < ne) load(m0 + EFSO_MC);
+        const int nm = min(EFSO_MC, ne - m0);
+#pragma unroll 4
+        for (int m = 0; m < nm; m++) {
+          const double h = tile[m * 33 + lane];
+#pragma unroll
+          for (int i = 0; i < NTERM; i++) acc[i] = fma(w[i * ne + m0 + m], h, acc[i]);
+        }
       }
+      if (on) {
+        const double s = 1.0 / rdiag[l] * rloc[l];
 #pragma unroll
-      for (int t = 0; t < EFSO_MAX_TERM; t++)
-        if (t < nterm) atomicAdd(&djdy[(size_t)ob * nterm + t], acc[t]);
+        for (int i = 0; i < NTERM; i++) atomicAdd(&djdy[(size_t)ob * NTERM + i], acc[i] * s);
+      }
     }
   }
+}
+
+template <int NTERM>
+static int launch_efso(int ne, int npts, int nv, const EfsoTerms& tv, const int64_t* offs, const int* idx,
+                       const double* rdiag, const double* rloc, const double* hdxa, const double* fcst,
+                       const double* fcer, double* djdy, cudaStream_t s) {
+  const size_t one = sizeof(double) * (size_t)NTERM * ne;
+  // as many points as 24 KB of work1 hold, fewer where that would leave SMs without a group
+  int dev = 0, nsm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  int group = (int)(24 * 1024 / one);
+  group = group < 1 ? 1 : group > EFSO_GROUP ? EFSO_GROUP : group;
+  const int fill = npts / (nsm * 8);
+  if (group > fill) group = fill < 1 ? 1 : fill;
+  const size_t smem = group * one + sizeof(double) * (OSA_NT / 32) * EFSO_MC * 33;
+  if (smem > 48 * 1024) {
+    const cudaError_t e =
+        cudaFuncSetAttribute(efso_djdy_kernel<NTERM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return cuda_status(e);
+  }
+  const int ngroup = (npts + group - 1) / group;
+  const int grid = ngroup < nsm * 8 ? ngroup : nsm * 8;
+  efso_djdy_kernel<NTERM><<<grid, OSA_NT, smem, s>>>(ne, npts, nv, group, tv, offs, idx, rdiag, rloc, hdxa, fcst,
+                                                     fcer, djdy);
+  note_launch();
+  return cuda_status(cudaGetLastError());
 }
 
 __global__ void efso_sense_kernel(int64_t n, int nterm, const double* __restrict__ djdy,
@@ -152,7 +256,7 @@ extern "C" int letkf_obs_analysis(int ne, int n, const double* trans, const doub
   if (ne < 2 || ne > 4096 || n < 0 || (n > 0 && (!trans || !ybar || !hdxf || !anal))) return LETKF_ERR_ARG;
   if (!have_device()) return LETKF_ERR_NOGPU;
   if (n == 0) return LETKF_OK;
-  const size_t smem = sizeof(double) * 2 * (size_t)ne;
+  const size_t smem = sizeof(double) * (2 * (size_t)ne + OSA_T * OSA_LD + OSA_T);
   if (smem > 48 * 1024) {
     const cudaError_t e =
         cudaFuncSetAttribute(obs_analysis_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -181,16 +285,19 @@ extern "C" int letkf_efso(int ne, int npts, int nv, int nterm, const int* term, 
   if (nobs == 0) return LETKF_OK;
   int st = cuda_status(cudaMemsetAsync(djdy, 0, sizeof(double) * (size_t)nobs * nterm, s));
   if (st == LETKF_OK && npts > 0) {
-    const size_t smem = sizeof(double) * (size_t)nterm * ne;
-    if (smem > 48 * 1024) {
-      const cudaError_t e =
-          cudaFuncSetAttribute(efso_djdy_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return cuda_status(e);
+#define EFSO_CASE(T) \
+  case T: st = launch_efso<T>(ne, npts, nv, tv, offs, idx, rdiag, rloc, hdxa, fcst, fcer, djdy, s); break
+    switch (nterm) {
+      EFSO_CASE(1);
+      EFSO_CASE(2);
+      EFSO_CASE(3);
+      EFSO_CASE(4);
+      EFSO_CASE(5);
+      EFSO_CASE(6);
+      EFSO_CASE(7);
+      EFSO_CASE(8);
     }
-    efso_djdy_kernel<<<grid_for(npts), OSA_NT, smem, s>>>(ne, npts, nv, nterm, tv, offs, idx, rdiag, rloc, hdxa,
-                                                          fcst, fcer, djdy);
-    note_launch();
-    st = cuda_status(cudaGetLastError());
+#undef EFSO_CASE
   }
   if (st == LETKF_OK) {
     const int64_t tot = (int64_t)nobs * nterm;

@@ -1,0 +1,133 @@
+"""The FP64 updates, the obs-space analysis and EFSO at the sizes where their
+tiles and chunks end: odd and even ensembles around the lane counts and the
+64-wide tile, more variables than one chunk holds, the clipped variable in any
+chunk, every number of EFSO terms, lists that leave a warp partly empty.
+
+Reference: the formulas of scale/letkf/letkf_tools.f90:215-268 and
+gfs/letkf/letkf_tools.f90:466-497,547-679 in numpy.  Tolerance 1e-12 of the
+largest value: sums of at most 130 products of O(1) terms in another order."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+RTOL = 1e-12
+
+
+def _t(a, dev, dt=None):
+    import torch
+
+    return torch.as_tensor(np.ascontiguousarray(a), dtype=dt or torch.float64, device=dev)
+
+
+def _close(a, b):
+    assert np.abs(a - b).max() <= RTOL * np.abs(b).max()
+
+
+@pytest.mark.parametrize("ne,nv,mode,q_var", [(2, 1, 2, 0), (3, 5, 1, 4), (7, 17, 2, 16), (8, 16, 2, 0), (15, 33, 0, 20),
+                                              (31, 4, 2, 3), (32, 3, 1, 1), (33, 11, 2, 2), (50, 18, 2, 17),
+                                              (64, 6, 2, 0), (65, 2, 1, 1), (101, 11, 2, 5), (128, 1, 0, 0)])
+def test_relaxed_update_edges(cuda, ne, nv, mode, q_var):
+    from letkf_gb300.core import update_relax_f64
+
+    rng = np.random.default_rng(100 * ne + nv)
+    npts, alpha, q_max = 23, 0.7, 0.05
+    w = rng.standard_normal((npts, ne, ne)) / ne + np.eye(ne)      # [p][m][k]
+    pa = rng.standard_normal((npts, ne, ne)) * 0.1 / ne + np.eye(ne) / ne  # not symmetric: every element counts
+    tm = rng.standard_normal((npts, ne)) * 0.1
+    xb = rng.standard_normal((nv, npts, ne)) + 3.0
+    beta = rng.uniform(0, 1, (nv, npts))
+    beta[:, ::5] = 1.0
+    beta[:, 1::7] = 0.0
+    xa, infl = update_relax_f64(_t(xb, cuda), _t(w, cuda), _t(tm, cuda), _t(pa, cuda), mode=mode, alpha=alpha,
+                                beta=_t(beta, cuda), q_var=q_var, q_sprd_max=q_max)
+    mean = xb.mean(-1, keepdims=True)
+    x = xb - mean
+    fac = np.ones((nv, npts))
+    inc = np.einsum("vpk,pmk->vpm", x, w)
+    if mode == 1:
+        inc = (1 - alpha) * inc + alpha * x
+    if mode == 2:
+        va = np.einsum("vpk,pmk,vpm->vp", x, pa, x)
+        vg = (x * x).sum(-1)
+        ok = (beta != 0) & (va > 0) & (vg > 0)
+        fac[ok] = alpha * np.sqrt(vg[ok] / (va[ok] * (ne - 1))) - alpha + 1
+        inc = inc * fac[..., None]
+    inc = inc + np.einsum("vpk,pk->vp", x, tm)[..., None]
+    want = mean + beta[..., None] * inc + (1 - beta)[..., None] * x
+    q = want[q_var]
+    qm = q.mean(-1, keepdims=True)
+    sp = np.sqrt(((q - qm) ** 2).sum(-1, keepdims=True) / (ne - 1)) / qm
+    want[q_var] = np.where(sp > q_max, qm + (q - qm) * q_max / sp, q)
+    _close(xa.cpu().numpy(), want)
+    if mode == 2:
+        _close(infl.cpu().numpy(), fac)
+
+
+@pytest.mark.parametrize("ne,nv,merged", [(2, 40, False), (31, 1, True), (33, 16, False), (64, 17, True), (127, 3, False)])
+def test_update_f64_edges(cuda, ne, nv, merged):
+    from letkf_gb300.core import update_f64
+
+    rng = np.random.default_rng(ne)
+    npts = 19
+    w = rng.standard_normal((npts, ne, ne)) / ne
+    tm = rng.standard_normal((npts, ne)) * 0.1
+    xb = rng.standard_normal((nv, npts, ne)) + 3.0
+    xa = update_f64(_t(xb, cuda), _t(w, cuda), None if merged else _t(tm, cuda)).cpu().numpy()
+    mean = xb.mean(-1, keepdims=True)
+    x = xb - mean
+    want = mean + np.einsum("vpk,pmk->vpm", x, w)
+    if not merged:
+        want = want + np.einsum("vpk,pk->vp", x, tm)[..., None]
+    _close(xa, want)
+
+
+@pytest.mark.parametrize("ne", [2, 31, 63, 64, 65, 96, 128, 129, 200])
+def test_obs_analysis_edges(cuda, ne):
+    import torch
+
+    from letkf_gb300.core import obs_analysis
+
+    rng = np.random.default_rng(ne)
+    n, alpha, q_max = 41, 0.25, 0.1
+    tr = rng.standard_normal((n, ne, ne)) / ne + np.eye(ne)
+    h = rng.standard_normal((n, ne))
+    y = rng.uniform(3.0, 6.0, n)
+    mode = (np.arange(n) % 3).astype(np.int32)
+    anal, mean = obs_analysis(_t(tr, cuda), _t(y, cuda), _t(h, cuda), alpha, _t(mode, cuda, torch.int32), q_max)
+    a = y[:, None] + (1 - alpha) * np.einsum("pk,pmk->pm", h, tr) + alpha * h
+    a[mode == 1] = (y[:, None] + h)[mode == 1]
+    m = np.where(mode == 1, y, a.mean(1))
+    sp = np.sqrt(((a - m[:, None]) ** 2).sum(1) / (ne - 1)) / m
+    cut = (mode == 2) & (sp > q_max)
+    a[cut] = (m[:, None] + (a - m[:, None]) * (q_max / sp)[:, None])[cut]
+    _close(anal.cpu().numpy(), a)
+    _close(mean.cpu().numpy(), m)
+
+
+@pytest.mark.parametrize("ne,npts,nterm", [(2, 1, 1), (15, 7, 2), (16, 9, 3), (17, 2500, 4), (33, 40, 5), (64, 1300, 6),
+                                           (96, 12, 7), (130, 20, 8)])
+def test_efso_edges(cuda, ne, npts, nterm):
+    import torch
+
+    from letkf_gb300.core import efso
+
+    rng = np.random.default_rng(ne + npts)
+    nobs, nv = 300, nterm + 2
+    cnt = rng.integers(0, 45, npts)
+    cnt[0] = 33
+    offs = np.concatenate([[0], np.cumsum(cnt)]).astype(np.int64)
+    idx = rng.integers(0, nobs, int(offs[-1])).astype(np.int32)
+    rd, rl = rng.uniform(0.5, 2.0, idx.size), rng.uniform(0.0, 1.0, idx.size)
+    hdxa, dep = rng.standard_normal((nobs, ne)), rng.standard_normal(nobs)
+    fcst, fcer = rng.standard_normal((nv, npts, ne)), rng.standard_normal((nv, npts))
+    term = list(range(nterm)) + [0, -1]
+    dj, sense = efso(ne, _t(offs, cuda, torch.int64), _t(idx, cuda, torch.int32), _t(rd, cuda), _t(rl, cuda),
+                     _t(hdxa, cuda), _t(fcst, cuda), _t(fcer, cuda), term, _t(dep, cuda))
+    want = np.zeros((nobs, nterm))
+    point = np.repeat(np.arange(npts), cnt)
+    for t in range(nterm):
+        w1 = sum(fcst[v] * fcer[v][:, None] for v in range(nv) if term[v] == t)
+        np.add.at(want[:, t], idx, (hdxa[idx] * w1[point]).sum(1) * rl / rd)
+    _close(dj.cpu().numpy(), want)
+    _close(sense.cpu().numpy(), want * dep[:, None])
