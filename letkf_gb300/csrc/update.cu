@@ -25,8 +25,7 @@
 // the quadratic form of RTPS goes over unordered pairs: x' Pa x = sum_d sum_i
 // x(i) D(d,i) x(i+d mod k), D(d,i) = Pa(i,i+d) + Pa(i+d,i), d = 0..k/2, formed
 // once per point for all variables, half the products of the full form and
-// every lane busy.  RTPS, 20,000 points, k = 50, 11 variables: 7.77 -> 2.89 ms
-// (FP64 pipe 78 % busy).
+// every lane busy.  RTPS, 20,000 points, k = 50, 11 variables: 7.77 -> 2.53 ms.
 #include "letkf_common.cuh"
 
 namespace letkf {
@@ -51,19 +50,36 @@ __host__ __device__ inline size_t upd_smem_doubles(int n, int nv, int mode) {
   return (size_t)n * (n | 1) + d + n + (size_t)vc * n + 4 * (size_t)vc + n;
 }
 
+// a[u] += sum_k x(v_u, k) W(k, m_u) for the first N of a thread's outputs (mm: offset of member m_u)
+template <int N, int U>
+__device__ __forceinline__ void upd_sums(int n, int sk, const double* xp, const double* W, const int (&vv)[U],
+                                         const int (&mm)[U], double (&a)[U]) {
+#pragma unroll(N == 1 ? 8 : 4)
+  for (int k = 0; k < n; k++)
+#pragma unroll
+    for (int u = 0; u < N; u++) a[u] = fma(xp[vv[u] * n + k], W[k * sk + mm[u]], a[u]);
+}
+
 // Points p0 .. p0+cnt-1 of arrays holding npts points; trans / transm / pao
-// are indexed from p0.
+// are indexed from p0.  MODE and BETA (r.beta given) are compiled in: an
+// operation that is only predicated off still takes its FP64 slot.
+template <int MODE, bool BETA>
 __global__ void __launch_bounds__(UPD_NT) update_f64_kernel(int n, int npts, int p0, int cnt, int nv,
                                                              const double* __restrict__ xb,
                                                              const double* __restrict__ trans,
                                                              const double* __restrict__ transm,
                                                              const double* __restrict__ pao, RelaxArgs r, double* xa) {
+  constexpr bool PLAIN = MODE == 0 && !BETA;
   extern __shared__ __align__(16) double su[];
   const int ld = n | 1, nh = n / 2, vcm = nv < UPD_VC ? nv : UPD_VC;
-  double* W = su;                          // [k][ld]
+  // W(k, m) at k sk + m sm: as in memory, or transposed where the row length
+  // would put the lanes' members on few banks
+  const bool tr = n % 16 == 0;
+  const int sk = tr ? ld : 1, sm = tr ? 1 : n;
+  double* W = su;
   double* D = W + (size_t)n * ld;          // [nh + 1][n] (RTPS)
-  double* prod = D + (r.mode == 2 ? (size_t)(nh + 1) * n : 0);  // [vcm][n] (RTPS)
-  double* tm = prod + (r.mode == 2 ? (size_t)vcm * n : 0);      // [n]
+  double* prod = D + (MODE == 2 ? (size_t)(nh + 1) * n : 0);  // [vcm][n] (RTPS)
+  double* tm = prod + (MODE == 2 ? (size_t)vcm * n : 0);      // [n]
   double* xp = tm + n;                     // [vcm][n]
   double* mean = xp + (size_t)vcm * n;     // [vcm] each
   double* fac = mean + vcm;
@@ -75,14 +91,19 @@ __global__ void __launch_bounds__(UPD_NT) update_f64_kernel(int n, int npts, int
     const int p = p0 + pl;
     __syncthreads();
     const double* Tp = trans + (size_t)pl * n * n;
+    if (tr) {
 #pragma unroll 4
-    for (int idx = tid; idx < n * n; idx += UPD_NT) {
-      const int m = idx / n, k = idx - m * n;
-      W[k * ld + m] = Tp[idx];
+      for (int idx = tid; idx < n * n; idx += UPD_NT) {
+        const int m = idx / n, k = idx - m * n;
+        W[k * ld + m] = Tp[idx];
+      }
+    } else {
+#pragma unroll 4
+      for (int idx = tid; idx < n * n; idx += UPD_NT) W[idx] = Tp[idx];
     }
     if (transm)
       for (int k = tid; k < n; k += UPD_NT) tm[k] = transm[(size_t)pl * n + k];
-    if (r.mode == 2) {
+    if (MODE == 2) {
       // first the element of each pair that starts it, then the other one onto it
       const double* Pp = pao + (size_t)pl * n * n;
 #pragma unroll 4
@@ -112,14 +133,14 @@ __global__ void __launch_bounds__(UPD_NT) update_f64_kernel(int n, int npts, int
         double s = xp[v * n];
         for (int m = 1; m < n; m++) s = s + xp[v * n + m];
         mean[v] = s / (double)n;
-        bet[v] = r.beta ? r.beta[(size_t)(v0 + v) * npts + p] : 1.0;
+        if (BETA) bet[v] = r.beta[(size_t)(v0 + v) * npts + p];
         fac[v] = 1.0;
       }
       __syncthreads();
       for (int t = tid; t < total; t += UPD_NT) xp[t] = xp[t] - mean[t / n];
       __syncthreads();
       const int nch = (total + 31) / 32;  // 32 outputs (variable, member) a chunk, chunks over the warps
-      if (r.mode == 2) {
+      if (MODE == 2) {
         for (int c = wid; c < nch; c += UPD_NT / 32) {
           const int t = min(32 * c + lane, total - 1);
           const int v = t / n, i = t - v * n;
@@ -137,14 +158,14 @@ __global__ void __launch_bounds__(UPD_NT) update_f64_kernel(int n, int npts, int
       }
       // sums over the members by eight lanes per variable (a full warp would
       // spend more FP64 slots on the reduction than on the sum)
-      if (transm || r.mode == 2) {
+      if (transm || MODE == 2) {
         for (int vb = 4 * wid; vb < vc; vb += UPD_NT / 8) {
           const int v = min(vb + (lane >> 3), vc - 1);
           const double* x = xp + v * n;
           double sx = 0.0, va = 0.0, vg = 0.0;
           if (transm)
             for (int k = lane & 7; k < n; k += 8) sx = fma(x[k], tm[k], sx);
-          if (r.mode == 2)
+          if (MODE == 2)
             for (int k = lane & 7; k < n; k += 8) {
               va = va + prod[v * n + k];
               vg = fma(x[k], x[k], vg);
@@ -152,16 +173,16 @@ __global__ void __launch_bounds__(UPD_NT) update_f64_kernel(int n, int npts, int
 #pragma unroll
           for (int o = 4; o > 0; o >>= 1) {
             if (transm) sx += __shfl_xor_sync(0xffffffffu, sx, o);
-            if (r.mode == 2) {
+            if (MODE == 2) {
               va += __shfl_xor_sync(0xffffffffu, va, o);
               vg += __shfl_xor_sync(0xffffffffu, vg, o);
             }
           }
           if ((lane & 7) == 0 && vb + (lane >> 3) < vc) {
             tx[v] = sx;
-            if (r.mode == 2) {  // beta == 0 skips weight_RTPS (factor 1)
+            if (MODE == 2) {  // beta == 0 skips weight_RTPS (factor 1)
               double f = 1.0;
-              if (bet[v] != 0.0 && vg > 0.0 && va > 0.0)
+              if ((!BETA || bet[v] != 0.0) && vg > 0.0 && va > 0.0)
                 f = r.alpha * sqrt(vg / (va * (double)(n - 1))) - r.alpha + 1.0;
               fac[v] = f;
               if (r.rtps_infl) r.rtps_infl[(size_t)(v0 + v) * npts + p] = f;
@@ -169,41 +190,49 @@ __global__ void __launch_bounds__(UPD_NT) update_f64_kernel(int n, int npts, int
           }
         }
       }
-      __syncthreads();
+      if (transm || MODE == 2) __syncthreads();
       const bool clip = r.q_sprd_max > 0.0 && r.q_var >= v0 && r.q_var < v0 + vc;
       constexpr int U = 4;
       for (int c0 = wid; c0 < nch; c0 += U * (UPD_NT / 32)) {
         const int nu = min(U, (nch - c0 + UPD_NT / 32 - 1) / (UPD_NT / 32));
         double a[U];
-        int vv[U], mm[U];
+        int vv[U], mm[U], off[U];
 #pragma unroll
         for (int u = 0; u < U; u++) {
           const int t = min(32 * (c0 + u * (UPD_NT / 32)) + lane, total - 1);
           vv[u] = t / n;
           mm[u] = t - vv[u] * n;
-          a[u] = 0.0;
+          // the plain update adds up from the mean, as the reference does
+          a[u] = PLAIN ? mean[vv[u]] : 0.0;
+          if (PLAIN && transm) a[u] = a[u] + tx[vv[u]];
+          off[u] = mm[u] * sm;
         }
-#pragma unroll 2
-        for (int k = 0; k < n; k++)
-#pragma unroll
-          for (int u = 0; u < U; u++)
-            if (u < nu) a[u] = fma(xp[vv[u] * n + k], W[k * ld + mm[u]], a[u]);
+        // one loop per count: a multiply-add that is only predicated off takes its FP64 slot
+        if (nu == 4)
+          upd_sums<4>(n, sk, xp, W, vv, off, a);
+        else if (nu == 3)
+          upd_sums<3>(n, sk, xp, W, vv, off, a);
+        else if (nu == 2)
+          upd_sums<2>(n, sk, xp, W, vv, off, a);
+        else
+          upd_sums<1>(n, sk, xp, W, vv, off, a);
 #pragma unroll
         for (int u = 0; u < U; u++) {
           if (u >= nu || 32 * (c0 + u * (UPD_NT / 32)) + lane >= total) continue;
           const int v = vv[u], m = mm[u];
-          const double b = bet[v], x = xp[v * n + m];
-          double inc;
-          if (b == 0.0) {
-            inc = x;
-          } else {
-            inc = a[u];
-            if (r.mode == 1) inc = (1.0 - r.alpha) * inc + r.alpha * x;
-            if (r.mode == 2) inc = fac[v] * inc;
+          const double x = xp[v * n + m];
+          double inc = a[u];
+          if (!PLAIN) {
+            if (MODE == 1) inc = (1.0 - r.alpha) * inc + r.alpha * x;
+            if (MODE == 2) inc = fac[v] * inc;
             if (transm) inc = inc + tx[v];
-            if (b != 1.0) inc = b * inc + (1.0 - b) * x;
+            if (BETA) {
+              const double b = bet[v];
+              inc = b == 0.0 ? x : b == 1.0 ? inc : b * inc + (1.0 - b) * x;
+            }
+            inc = mean[v] + inc;
           }
-          const double y = mean[v] + inc;
+          const double y = inc;
           if (clip && v0 + v == r.q_var)
             qv[m] = y;
           else
@@ -231,12 +260,129 @@ __global__ void __launch_bounds__(UPD_NT) update_f64_kernel(int n, int npts, int
   }
 }
 
-static int launch_update(int ne, int npts, int p0, int cnt, int nv, const double* xb, const double* trans,
-                         const double* transm, const double* pao, const RelaxArgs& r, double* xa,
-                         cudaStream_t stream) {
-  const size_t smem = sizeof(double) * upd_smem_doubles(ne, nv, r.mode);
-  const cudaError_t err =
-      cudaFuncSetAttribute(update_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+// The plain update of few variables: a warp per batch of rows (variable,
+// point), no barrier.  Each lane reads its member's row of trans straight from
+// global memory, 64 consecutive bytes at a time where rows are 16-byte aligned;
+// x stays in shared memory, no more of it than the batch needs, because the
+// rest of the SM's 256 KB is the L1 that holds the lines the lanes are in the
+// middle of (with room for 16 rows always: k = 100 0.72 ms instead of 0.27).
+// What bounds it is FP64 slots beside the k products of an output: a
+// member-order mean costs as many as the products when one lane does it alone,
+// so lanes take the rows of the batch.  One variable, 100,000 points of k = 32:
+// 0.57 -> 0.22 ms, 20,000 of k = 50: 0.22 -> 0.16, 4,000 of k = 128: 0.75 ->
+// 0.16 (before: a CTA per point).  The sums are those of the kernel above in
+// the same order, so the results are the same bits.
+constexpr int UPR_ROWS = 16;
+
+template <int NVT, bool VEC>
+__global__ void __launch_bounds__(UPD_NT, 8) update_rows_kernel(int n, int npts, int p0, int cnt, int pb,
+                                                                const double* __restrict__ xb,
+                                                                const double* __restrict__ trans,
+                                                                const double* __restrict__ transm, double* xa) {
+  // pb points of NVT rows each in a batch
+  extern __shared__ __align__(16) double su[];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, ld = n | 1;
+  double* xs = su + (size_t)wid * pb * NVT * (ld + 1);  // [point][variable][ld]
+  double* tx = xs + pb * NVT * ld;
+  const int nbatch = (cnt + pb - 1) / pb;
+  for (int b = blockIdx.x * (UPD_NT / 32) + wid; b < nbatch; b += gridDim.x * (UPD_NT / 32)) {
+    const int q0 = b * pb, nq = min(pb, cnt - q0), nr = nq * NVT;
+    __syncwarp();
+    for (int r = 0; r < nr; r++) {
+      const double* src = xb + ((size_t)(r % NVT) * npts + p0 + q0 + r / NVT) * n;
+      for (int m = lane; m < n; m += 32) xs[r * ld + m] = src[m];
+    }
+    __syncwarp();
+    double mean = 0.0;
+    if (lane < nr) {
+      const double* x = xs + lane * ld;
+      double s = x[0];
+      for (int m = 1; m < n; m++) s = s + x[m];
+      mean = s / (double)n;
+    }
+    for (int r = 0; r < nr; r++) {
+      const double mr = __shfl_sync(0xffffffffu, mean, r);
+      for (int m = lane; m < n; m += 32) xs[r * ld + m] = xs[r * ld + m] - mr;
+    }
+    __syncwarp();
+    if (transm) {
+      for (int rb = 0; rb < nr; rb += 4) {
+        const int r = min(rb + (lane >> 3), nr - 1);
+        const double* t = transm + (size_t)(q0 + r / NVT) * n;
+        double sx = 0.0;
+        for (int k = lane & 7; k < n; k += 8) sx = fma(xs[r * ld + k], t[k], sx);
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) sx += __shfl_xor_sync(0xffffffffu, sx, o);
+        if ((lane & 7) == 0 && rb + (lane >> 3) < nr) tx[r] = sx;
+      }
+      __syncwarp();
+    }
+    for (int q = 0; q < nq; q++) {
+      const double* x = xs + q * NVT * ld;
+      double mr[NVT];
+#pragma unroll
+      for (int v = 0; v < NVT; v++) mr[v] = __shfl_sync(0xffffffffu, mean, q * NVT + v);
+      for (int m = lane; m < n; m += 32) {
+        const double* w = trans + ((size_t)(q0 + q) * n + m) * n;
+        double a[NVT];
+#pragma unroll
+        for (int v = 0; v < NVT; v++) a[v] = transm ? mr[v] + tx[q * NVT + v] : mr[v];
+        int k = 0;
+        if (VEC) {
+          for (; k + 8 <= n; k += 8) {
+            double2 t[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) t[i] = *reinterpret_cast<const double2*>(w + k + 2 * i);
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+              for (int v = 0; v < NVT; v++) {
+                a[v] = fma(x[v * ld + k + 2 * i], t[i].x, a[v]);
+                a[v] = fma(x[v * ld + k + 2 * i + 1], t[i].y, a[v]);
+              }
+          }
+        }
+#pragma unroll 4
+        for (; k < n; k++) {
+          const double t = w[k];
+#pragma unroll
+          for (int v = 0; v < NVT; v++) a[v] = fma(x[v * ld + k], t, a[v]);
+        }
+#pragma unroll
+        for (int v = 0; v < NVT; v++) xa[((size_t)v * npts + p0 + q0 + q) * n + m] = a[v];
+      }
+    }
+  }
+}
+
+template <int NVT, bool VEC>
+static int launch_update_rows(int ne, int npts, int p0, int cnt, const double* xb, const double* trans,
+                              const double* transm, double* xa, cudaStream_t stream) {
+  static std::atomic<uint32_t> done{0};
+  const cudaError_t err = set_smem_once(update_rows_kernel<NVT, VEC>,
+                                        sizeof(double) * (UPD_NT / 32) * (size_t)(UPR_ROWS * (LETKF_MAX_NE + 1) + UPR_ROWS), done);
+  if (err != cudaSuccess) return cuda_status(err);
+  int dev = 0, nsm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  // full batches only where every SM then still has two rounds of warps
+  int pb = cnt / (nsm * 64);
+  pb = pb < 1 ? 1 : pb > UPR_ROWS / NVT ? UPR_ROWS / NVT : pb;
+  const size_t smem = sizeof(double) * (UPD_NT / 32) * (size_t)pb * NVT * ((ne | 1) + 1);
+  const int need = (cnt + pb * (UPD_NT / 32) - 1) / (pb * (UPD_NT / 32));
+  const int grid = need < nsm * 8 ? need : nsm * 8;
+  update_rows_kernel<NVT, VEC><<<grid, UPD_NT, smem, stream>>>(ne, npts, p0, cnt, pb, xb, trans, transm, xa);
+  note_launch();
+  return cuda_status(cudaGetLastError());
+}
+
+template <int MODE, bool BETA>
+static int launch_update_as(int ne, int npts, int p0, int cnt, int nv, const double* xb, const double* trans,
+                            const double* transm, const double* pao, const RelaxArgs& r, double* xa,
+                            cudaStream_t stream) {
+  const size_t smem = sizeof(double) * upd_smem_doubles(ne, nv, MODE);
+  auto kern = update_f64_kernel<MODE, BETA>;
+  const cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (err != cudaSuccess) return cuda_status(err);
   int dev = 0, nsm = 0;
   cudaGetDevice(&dev);
@@ -245,9 +391,21 @@ static int launch_update(int ne, int npts, int p0, int cnt, int nv, const double
   int per_sm = (int)((size_t)(220 * 1024) / (smem + 1024));
   per_sm = per_sm < 1 ? 1 : per_sm > 8 ? 8 : per_sm;
   const int grid = cnt < nsm * per_sm ? cnt : nsm * per_sm;
-  update_f64_kernel<<<grid, UPD_NT, smem, stream>>>(ne, npts, p0, cnt, nv, xb, trans, transm, pao, r, xa);
+  kern<<<grid, UPD_NT, smem, stream>>>(ne, npts, p0, cnt, nv, xb, trans, transm, pao, r, xa);
   note_launch();
   return cuda_status(cudaGetLastError());
+}
+
+static int launch_update(int ne, int npts, int p0, int cnt, int nv, const double* xb, const double* trans,
+                         const double* transm, const double* pao, const RelaxArgs& r, double* xa,
+                         cudaStream_t stream) {
+#define UPD_AS(MODE)                                                                                             \
+  return r.beta ? launch_update_as<MODE, true>(ne, npts, p0, cnt, nv, xb, trans, transm, pao, r, xa, stream) \
+                : launch_update_as<MODE, false>(ne, npts, p0, cnt, nv, xb, trans, transm, pao, r, xa, stream)
+  if (r.mode == 2) UPD_AS(2);
+  if (r.mode == 1) UPD_AS(1);
+  UPD_AS(0);
+#undef UPD_AS
 }
 
 int launch_update_f64_range(int ne, int npts_total, int p0, int cnt, int nv, const double* xb, const double* trans,
@@ -255,6 +413,26 @@ int launch_update_f64_range(int ne, int npts_total, int p0, int cnt, int nv, con
   if (ne < 2 || npts_total < 0 || p0 < 0 || cnt < 0 || p0 + cnt > npts_total || nv < 1) return LETKF_ERR_ARG;
   if (ne > LETKF_MAX_NE) return LETKF_ERR_CAPACITY;
   if (cnt == 0) return LETKF_OK;
+  const bool vec = ne % 2 == 0 && reinterpret_cast<uintptr_t>(trans) % 16 == 0;
+#define UPR_LAUNCH(NVT)                                                                                 \
+  return vec ? launch_update_rows<NVT, true>(ne, npts_total, p0, cnt, xb, trans, transm, xa, stream) \
+             : launch_update_rows<NVT, false>(ne, npts_total, p0, cnt, xb, trans, transm, xa, stream)
+  // A warp per batch of rows re-reads x for every member it holds, the CTA form
+  // fills the lanes over all variables: the lines where they cross, measured
+  // with n = 20 / 40 / 64 / 128 (rows against CTA, us): 4 variables 534 / 606 /
+  // 521 / 497 against 591 / 537 / 533 / 1183, 2 variables 279 / 325 / 302 / 274
+  // against 498 / 342 / 340 / 895, 6 variables
+  // (64, 128) 747 / 736 against 823 / 1503.
+  const int rows = ne <= 32 ? 4 : ne <= 55 ? 2 : 6;
+  if (nv <= rows) {
+    if (nv == 1) UPR_LAUNCH(1);
+    if (nv == 2) UPR_LAUNCH(2);
+    if (nv == 3) UPR_LAUNCH(3);
+    if (nv == 4) UPR_LAUNCH(4);
+    if (nv == 5) UPR_LAUNCH(5);
+    UPR_LAUNCH(6);
+  }
+#undef UPR_LAUNCH
   const RelaxArgs r = {0, 0.0, nullptr, -1, 0.0, nullptr};
   return launch_update(ne, npts_total, p0, cnt, nv, xb, trans, transm, nullptr, r, xa, stream);
 }

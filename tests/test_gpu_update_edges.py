@@ -64,12 +64,15 @@ def test_relaxed_update_edges(cuda, ne, nv, mode, q_var):
         _close(infl.cpu().numpy(), fac)
 
 
-@pytest.mark.parametrize("ne,nv,merged", [(2, 40, False), (31, 1, True), (33, 16, False), (64, 17, True), (127, 3, False)])
-def test_update_f64_edges(cuda, ne, nv, merged):
+@pytest.mark.parametrize("ne,nv,merged", [(2, 40, False), (31, 1, True), (33, 16, False), (64, 17, True), (127, 3, False),
+                                          (7, 4, True), (32, 4, False), (40, 2, True), (55, 2, False), (56, 6, True),
+                                          (64, 5, False), (128, 1, True), (101, 6, False)])
+@pytest.mark.parametrize("npts", [1, 19, 20_000])
+def test_update_f64_edges(cuda, ne, nv, merged, npts):
     from letkf_gb300.core import update_f64
 
     rng = np.random.default_rng(ne)
-    npts = 19
+    npts = min(npts, 3_000_000 // (ne * ne))
     w = rng.standard_normal((npts, ne, ne)) / ne
     tm = rng.standard_normal((npts, ne)) * 0.1
     xb = rng.standard_normal((nv, npts, ne)) + 3.0
