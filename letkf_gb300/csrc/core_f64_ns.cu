@@ -29,15 +29,17 @@
 // come straight from shared memory and one warp per sub-partition keeps it
 // busy; the FP32 phases of one CTA overlap the FP64 phases of the others on
 // the SM.  Measured: 8,640 regional points of k = 64 (mean list about 300)
-// 183 -> 28 ms; 32,256 SPEEDY-grid points of k = 40 (mean list 86) 233 -> 31
-// ms (FP64 pipe 50 % busy, FP32 24 %, 66 % and 20 % with every residual in
-// FP64: 34 ms); a 40-point ring of k = 20, one point per SM, 1.43 -> 0.1 ms.
+// 183 -> 26 ms (FP64 pipe 69 % busy); 32,256 SPEEDY-grid points of k = 40 (mean
+// list 86) 233 -> 23 ms (FP64 pipe 55 %, FP32 30 %); with every residual in
+// FP64 a tenth more; a 40-point ring of k = 20, one point per SM, 1.43 -> 0.1.
 //
 // A point is left to core_f64.cu (status LETKF_PENDING until its launch) where
 // mtx_eigen's truncation or the conditioning could matter (c <= 0, or
 // s / c >= 1e5 where s >= lambda_max), or where the iteration does not reach
 // its residual.
 #include <math.h>
+
+#include <type_traits>
 
 #include "letkf_common.cuh"
 
@@ -47,11 +49,15 @@ constexpr int FN_NT = 128;
 
 template <int NP>
 struct FnCfg {
-  static constexpr int TR = NP / 16, TC = NP / 8;         // FP32 product tile of a thread
+  // FP32 product tile of a thread: TR consecutive rows, TC columns; the lanes' fast index runs along the
+  // columns, so a warp reads and writes consecutive words of a row
+  static constexpr int TR = NP / 8, TC = NP / 16;
   static constexpr int CH = NP >= 32 ? 16 : 8;            // observations per staged chunk
   static constexpr int NB = NP / 8;                       // 8 x 8 blocks a side
   static constexpr int MAXL = (NB * (NB + 1) / 2 + 3) / 4;  // lower blocks of a warp
   static constexpr int MAXF = (NB * NB + 3) / 4;            // blocks of a warp, full matrix
+  // and the fewest for the ensembles this width serves (NB - 1 blocks a side; a warp may have none at 16)
+  static constexpr int MINL = NP == 16 ? 1 : NB * (NB - 1) / 2 / 4, MINF = NP == 16 ? 1 : (NB - 1) * (NB - 1) / 4;
   // CTAs an SM holds: three FP64 matrices each (96, 54, 24, 6 KB)
   static constexpr int MINB = NP == 64 ? 2 : NP == 48 ? 4 : NP == 32 ? 6 : 8;
   // doubles after the matrices: b, wbar, scratch, four partial b, two chunks' weights / departures / rloc, reductions
@@ -83,9 +89,26 @@ __device__ __forceinline__ void fn_ld(const float* p, float (&v)[N]) {
   }
 }
 
+// column of element b of a thread's tile, tx = threadIdx.x % 16
+template <int NP>
+__device__ __forceinline__ int fn_col(int tx, int b) {
+  constexpr int TC = FnCfg<NP>::TC;
+  return TC == 3 ? 16 * b + tx : TC * tx + b;
+}
+
+template <int NP>
+__device__ __forceinline__ void fn_ldc(const float* p, int tx, float (&v)[FnCfg<NP>::TC]) {
+  if constexpr (FnCfg<NP>::TC == 3) {
+#pragma unroll
+    for (int b = 0; b < 3; b++) v[b] = p[16 * b + tx];
+  } else {
+    fn_ld<FnCfg<NP>::TC>(p + FnCfg<NP>::TC * tx, v);
+  }
+}
+
 // acc = X^T Yb for this thread's tile (X symmetric, or its transpose is meant)
 template <int NP>
-__device__ __forceinline__ void fn_gemm(const float* X, const float* Yb, int i0, int j0,
+__device__ __forceinline__ void fn_gemm(const float* X, const float* Yb, int i0, int tx,
                                         float (&acc)[FnCfg<NP>::TR][FnCfg<NP>::TC]) {
   using C = FnCfg<NP>;
 #pragma unroll
@@ -96,7 +119,7 @@ __device__ __forceinline__ void fn_gemm(const float* X, const float* Yb, int i0,
   for (int k = 0; k < NP; k++) {
     float av[C::TR], bv[C::TC];
     fn_ld<C::TR>(X + k * NP + i0, av);
-    fn_ld<C::TC>(Yb + k * NP + j0, bv);
+    fn_ldc<NP>(Yb + k * NP, tx, bv);
 #pragma unroll
     for (int a = 0; a < C::TR; a++)
 #pragma unroll
@@ -114,25 +137,35 @@ __device__ __forceinline__ int2 fn_lower(int id) {
   return make_int2(bi, id);
 }
 
-// acc[b] += X^T Yb over k < n8 on this warp's lower blocks (8 x 8; a lane has
-// row lane / 4 and the two columns 2 (lane % 4) of each)
-template <int NP>
-__device__ __forceinline__ void fn_lower_product(const double* X, const double* Yb, int n8, int mine,
-                                                 const int (&xo)[FnCfg<NP>::MAXL], const int (&yo)[FnCfg<NP>::MAXL],
-                                                 double (&acc)[FnCfg<NP>::MAXL][2]) {
-  constexpr int MAXL = FnCfg<NP>::MAXL;
-#pragma unroll 2
+// acc[b] += X^T Yb over k < n8 on M 8 x 8 blocks (a lane has row lane / 4 and
+// the two columns 2 (lane % 4) of each)
+template <int NP, int M, int N>
+__device__ __forceinline__ void fn_product(const double* X, const double* Yb, int n8, const int (&xo)[N],
+                                           const int (&yo)[N], double (&acc)[N][2]) {
+#pragma unroll(M <= 8 ? 2 : 1)
   for (int k = 0; k < n8; k++) {
     const double* xk = X + k * NP;
     const double* yk = Yb + k * NP;
 #pragma unroll
-    for (int b = 0; b < MAXL; b++)
-      if (b < mine) {
-        const double a = xk[xo[b]];
-        const double2 y = *reinterpret_cast<const double2*>(yk + yo[b]);
-        acc[b][0] = fma(a, y.x, acc[b][0]);
-        acc[b][1] = fma(a, y.y, acc[b][1]);
-      }
+    for (int b = 0; b < M; b++) {
+      const double a = xk[xo[b]];
+      const double2 y = *reinterpret_cast<const double2*>(yk + yo[b]);
+      acc[b][0] = fma(a, y.x, acc[b][0]);
+      acc[b][1] = fma(a, y.y, acc[b][1]);
+    }
+  }
+}
+
+// f(std::integral_constant<int, m>) for this warp's block count, LO .. N: one
+// loop per count, because a multiply-add that is only predicated off still
+// takes its FP64 slot (k = 40 in the 48-wide kernel: 4 of 6 blocks are real)
+template <int N, int LO, typename F>
+__device__ __forceinline__ void fn_counted(int m, F&& f) {
+  if constexpr (N >= LO) {
+    if (m == N)
+      f(std::integral_constant<int, N>());
+    else
+      fn_counted<N - 1, LO>(m, f);
   }
 }
 
@@ -144,19 +177,19 @@ __device__ __forceinline__ void fn_lower_product(const double* X, const double* 
 template <int NP>
 __device__ bool fn_newton_schulz(float* Y, float* Z, float* T, float* TT, float* redf, float lo) {
   using C = FnCfg<NP>;
-  const int tid = threadIdx.x, i0 = (tid & 15) * C::TR, j0 = (tid >> 4) * C::TC;
+  const int tid = threadIdx.x, i0 = (tid >> 4) * C::TR, tx = tid & 15;
   float acc[C::TR][C::TC], yn[C::TR][C::TC];
   float prev = INFINITY;
   for (int it = 0; it < 24; it++) {
-    fn_gemm<NP>(Z, Y, i0, j0, acc);
+    fn_gemm<NP>(Z, Y, i0, tx, acc);
     float e2 = 0.f;
 #pragma unroll
     for (int a = 0; a < C::TR; a++)
 #pragma unroll
       for (int b = 0; b < C::TC; b++) {
-        T[(i0 + a) * NP + j0 + b] = acc[a][b];
-        TT[(j0 + b) * NP + i0 + a] = acc[a][b];
-        const float d = acc[a][b] - (i0 + a == j0 + b ? 1.f : 0.f);
+        T[(i0 + a) * NP + fn_col<NP>(tx, b)] = acc[a][b];
+        TT[fn_col<NP>(tx, b) * NP + i0 + a] = acc[a][b];
+        const float d = acc[a][b] - (i0 + a == fn_col<NP>(tx, b) ? 1.f : 0.f);
         e2 = fmaf(d, d, e2);
       }
     e2 = block_sum<float, FN_NT>(e2, redf);  // publishes T
@@ -164,23 +197,23 @@ __device__ bool fn_newton_schulz(float* Y, float* Z, float* T, float* TT, float*
     const float al = ns_scale(lo), sa = sqrtf(al);
     const float ka = 1.5f * sa, kb = 0.5f * al * sa;
     lo = f_ns(al * lo);
-    fn_gemm<NP>(Y, T, i0, j0, acc);
+    fn_gemm<NP>(Y, T, i0, tx, acc);
 #pragma unroll
     for (int a = 0; a < C::TR; a++)
 #pragma unroll
-      for (int b = 0; b < C::TC; b++) yn[a][b] = ka * Y[(i0 + a) * NP + j0 + b] - kb * acc[a][b];
-    fn_gemm<NP>(TT, Z, i0, j0, acc);
+      for (int b = 0; b < C::TC; b++) yn[a][b] = ka * Y[(i0 + a) * NP + fn_col<NP>(tx, b)] - kb * acc[a][b];
+    fn_gemm<NP>(TT, Z, i0, tx, acc);
 #pragma unroll
     for (int a = 0; a < C::TR; a++)
 #pragma unroll
-      for (int b = 0; b < C::TC; b++) acc[a][b] = ka * Z[(i0 + a) * NP + j0 + b] - kb * acc[a][b];
+      for (int b = 0; b < C::TC; b++) acc[a][b] = ka * Z[(i0 + a) * NP + fn_col<NP>(tx, b)] - kb * acc[a][b];
     __syncthreads();
 #pragma unroll
     for (int a = 0; a < C::TR; a++)
 #pragma unroll
       for (int b = 0; b < C::TC; b++) {
-        Y[(i0 + a) * NP + j0 + b] = yn[a][b];
-        Z[(i0 + a) * NP + j0 + b] = acc[a][b];
+        Y[(i0 + a) * NP + fn_col<NP>(tx, b)] = yn[a][b];
+        Z[(i0 + a) * NP + fn_col<NP>(tx, b)] = acc[a][b];
       }
     __syncthreads();
     // converged, or at the FP32 floor of this spectrum (Newton's method takes it from there)
@@ -196,52 +229,52 @@ __device__ bool fn_newton_schulz(float* Y, float* Z, float* T, float* TT, float*
 template <int NP>
 __device__ void fn_sign(float* Y, float* Y2, float* R, float* U, float lo) {
   using C = FnCfg<NP>;
-  const int tid = threadIdx.x, i0 = (tid & 15) * C::TR, j0 = (tid >> 4) * C::TC;
+  const int tid = threadIdx.x, i0 = (tid >> 4) * C::TR, tx = tid & 15;
   float acc[C::TR][C::TC], yn[C::TR][C::TC], rn[C::TR][C::TC];
   for (int it = 0; it < 20; it++) {
     const bool last = lo > 0.999f;
-    fn_gemm<NP>(Y, Y, i0, j0, acc);
+    fn_gemm<NP>(Y, Y, i0, tx, acc);
 #pragma unroll
     for (int a = 0; a < C::TR; a++)
 #pragma unroll
-      for (int b = 0; b < C::TC; b++) Y2[(i0 + a) * NP + j0 + b] = acc[a][b];
-    fn_gemm<NP>(R, Y, i0, j0, acc);
+      for (int b = 0; b < C::TC; b++) Y2[(i0 + a) * NP + fn_col<NP>(tx, b)] = acc[a][b];
+    fn_gemm<NP>(R, Y, i0, tx, acc);
 #pragma unroll
     for (int a = 0; a < C::TR; a++)
 #pragma unroll
-      for (int b = 0; b < C::TC; b++) U[(i0 + a) * NP + j0 + b] = acc[a][b];
+      for (int b = 0; b < C::TC; b++) U[(i0 + a) * NP + fn_col<NP>(tx, b)] = acc[a][b];
     __syncthreads();
     const float al = ns_scale(lo), sa = sqrtf(al);
     const float ka = 1.5f * sa, kb = 0.5f * al * sa;
     lo = f_ns(al * lo);
     if (!last) {
-      fn_gemm<NP>(Y, Y2, i0, j0, acc);
+      fn_gemm<NP>(Y, Y2, i0, tx, acc);
 #pragma unroll
       for (int a = 0; a < C::TR; a++)
 #pragma unroll
-        for (int b = 0; b < C::TC; b++) yn[a][b] = ka * Y[(i0 + a) * NP + j0 + b] - kb * acc[a][b];
+        for (int b = 0; b < C::TC; b++) yn[a][b] = ka * Y[(i0 + a) * NP + fn_col<NP>(tx, b)] - kb * acc[a][b];
     }
-    fn_gemm<NP>(Y, U, i0, j0, acc);  // Y R Y
+    fn_gemm<NP>(Y, U, i0, tx, acc);  // Y R Y
 #pragma unroll
     for (int a = 0; a < C::TR; a++)
 #pragma unroll
-      for (int b = 0; b < C::TC; b++) rn[a][b] = ka * R[(i0 + a) * NP + j0 + b] + kb * acc[a][b];
-    fn_gemm<NP>(Y2, R, i0, j0, acc);  // Y^2 R; R Y^2 is its transpose
+      for (int b = 0; b < C::TC; b++) rn[a][b] = ka * R[(i0 + a) * NP + fn_col<NP>(tx, b)] + kb * acc[a][b];
+    fn_gemm<NP>(Y2, R, i0, tx, acc);  // Y^2 R; R Y^2 is its transpose
     __syncthreads();
 #pragma unroll
     for (int a = 0; a < C::TR; a++)
 #pragma unroll
       for (int b = 0; b < C::TC; b++) {
-        U[(i0 + a) * NP + j0 + b] = acc[a][b];
-        if (!last) Y[(i0 + a) * NP + j0 + b] = yn[a][b];
+        U[(i0 + a) * NP + fn_col<NP>(tx, b)] = acc[a][b];
+        if (!last) Y[(i0 + a) * NP + fn_col<NP>(tx, b)] = yn[a][b];
       }
     __syncthreads();
 #pragma unroll
     for (int b = 0; b < C::TC; b++) {
       float m[C::TR];
-      fn_ld<C::TR>(U + (j0 + b) * NP + i0, m);
+      fn_ld<C::TR>(U + fn_col<NP>(tx, b) * NP + i0, m);
 #pragma unroll
-      for (int a = 0; a < C::TR; a++) R[(i0 + a) * NP + j0 + b] = rn[a][b] - kb * (acc[a][b] + m[a]);
+      for (int a = 0; a < C::TR; a++) R[(i0 + a) * NP + fn_col<NP>(tx, b)] = rn[a][b] - kb * (acc[a][b] + m[a]);
     }
     __syncthreads();
     if (last) return;
@@ -280,7 +313,7 @@ __global__ void __launch_bounds__(FN_NT, FnCfg<NP>::MINB) core_f64_ns_kernel(
     double* parm_infl, double* trans, double* transm, double* pao, int rdiag_wloc, double minfl, int* status,
     int* counter) {
   using C = FnCfg<NP>;
-  constexpr int Q = NP * NP, CH = C::CH, MAXL = C::MAXL, MAXF = C::MAXF;
+  constexpr int Q = NP * NP, CH = C::CH, MAXL = C::MAXL, MAXF = C::MAXF, MINL = C::MINL, MINF = C::MINF;
   extern __shared__ __align__(16) double sm[];
   double* A = sm;           // A; in the sign iteration Y, Y^2 (FP32)
   double* Z = sm + Q;       // FP32 Z, T, then FP64 Z; with P: the staged rows
@@ -380,7 +413,7 @@ __global__ void __launch_bounds__(FN_NT, FnCfg<NP>::MINB) core_f64_ns_kernel(
         p3 = p3 + w[2 * CH + tid];
       }
       __syncthreads();
-      fn_lower_product<NP>(Yw, y, nr, mine, xo, yo, acc);
+      fn_counted<MAXL, MINL>(mine, [&](auto m) { fn_product<NP, decltype(m)::value>(Yw, y, nr, xo, yo, acc); });
       for (int r = wid; r < nr; r += 4) {
         const double d = w[CH + r];
 #pragma unroll
@@ -458,14 +491,14 @@ __global__ void __launch_bounds__(FN_NT, FnCfg<NP>::MINB) core_f64_ns_kernel(
     }
     if (ok) {
       // Z exactly symmetric; A/s as pairs of floats in A's place (A is in T)
-      const int i0 = (tid & 15) * C::TR, j0 = (tid >> 4) * C::TC;
+      const int i0 = (tid >> 4) * C::TR, tx = tid & 15;
       float z[C::TR][C::TC];
 #pragma unroll
       for (int b = 0; b < C::TC; b++) {
         float m[C::TR];
-        fn_ld<C::TR>(Z32 + (j0 + b) * NP + i0, m);
+        fn_ld<C::TR>(Z32 + fn_col<NP>(tx, b) * NP + i0, m);
 #pragma unroll
-        for (int a = 0; a < C::TR; a++) z[a][b] = 0.5f * (Z32[(i0 + a) * NP + j0 + b] + m[a]);
+        for (int a = 0; a < C::TR; a++) z[a][b] = 0.5f * (Z32[(i0 + a) * NP + fn_col<NP>(tx, b)] + m[a]);
       }
       float2* A2 = reinterpret_cast<float2*>(A);
       for (int idx = tid; idx < Q; idx += FN_NT) {
@@ -477,7 +510,7 @@ __global__ void __launch_bounds__(FN_NT, FnCfg<NP>::MINB) core_f64_ns_kernel(
 #pragma unroll
       for (int a = 0; a < C::TR; a++)
 #pragma unroll
-        for (int b = 0; b < C::TC; b++) Z32[(i0 + a) * NP + j0 + b] = z[a][b];
+        for (int b = 0; b < C::TC; b++) Z32[(i0 + a) * NP + fn_col<NP>(tx, b)] = z[a][b];
       __syncthreads();
 
       // ---- 3. Newton's method anchored to A ----
@@ -506,18 +539,19 @@ __global__ void __launch_bounds__(FN_NT, FnCfg<NP>::MINB) core_f64_ns_kernel(
             ph[b][0] = ph[b][1] = off;
             pl[b][0] = pl[b][1] = 0.f;
           }
-          for (int k = 0; k < n8; k++) {
-            const float2* ak = A2 + k * NP;
-            const float* zk = Z32 + k * NP;
+          fn_counted<MAXF, MINF>(minef, [&](auto m) {
+            for (int k = 0; k < n8; k++) {
+              const float2* ak = A2 + k * NP;
+              const float* zk = Z32 + k * NP;
 #pragma unroll
-            for (int b = 0; b < MAXF; b++)
-              if (b < minef) {
+              for (int b = 0; b < decltype(m)::value; b++) {
                 const float2 a = ak[fx[b]];
                 const float2 y = *reinterpret_cast<const float2*>(zk + fy[b]);
                 fn_df_mac(ph[b][0], pl[b][0], a, y.x);
                 fn_df_mac(ph[b][1], pl[b][1], a, y.y);
               }
-          }
+            }
+          });
           float2* P2 = reinterpret_cast<float2*>(P);
 #pragma unroll
           for (int b = 0; b < MAXF; b++)
@@ -532,18 +566,19 @@ __global__ void __launch_bounds__(FN_NT, FnCfg<NP>::MINB) core_f64_ns_kernel(
             qh[b][0] = qh[b][1] = off;
             ql[b][0] = ql[b][1] = 0.f;
           }
-          for (int k = 0; k < n8; k++) {
-            const float* zk = Z32 + k * NP;
-            const float2* pk = P2 + k * NP;
+          fn_counted<MAXL, MINL>(mine, [&](auto m) {
+            for (int k = 0; k < n8; k++) {
+              const float* zk = Z32 + k * NP;
+              const float2* pk = P2 + k * NP;
 #pragma unroll
-            for (int b = 0; b < MAXL; b++)
-              if (b < mine) {
+              for (int b = 0; b < decltype(m)::value; b++) {
                 const float z = zk[xo[b]];
                 const float4 y = *reinterpret_cast<const float4*>(pk + yo[b]);
                 fn_df_mac(qh[b][0], ql[b][0], make_float2(y.x, y.y), z);
                 fn_df_mac(qh[b][1], ql[b][1], make_float2(y.z, y.w), z);
               }
-          }
+            }
+          });
 #pragma unroll
           for (int b = 0; b < MAXL; b++)
 #pragma unroll
@@ -555,26 +590,14 @@ __global__ void __launch_bounds__(FN_NT, FnCfg<NP>::MINB) core_f64_ns_kernel(
           double pf[MAXF][2];
 #pragma unroll
           for (int b = 0; b < MAXF; b++) pf[b][0] = pf[b][1] = 0.0;
-#pragma unroll 2
-          for (int k = 0; k < n8; k++) {
-            const double* ak = A + k * NP;
-            const double* zk = Z + k * NP;
-#pragma unroll
-            for (int b = 0; b < MAXF; b++)
-              if (b < minef) {
-                const double a = ak[fx[b]];
-                const double2 y = *reinterpret_cast<const double2*>(zk + fy[b]);
-                pf[b][0] = fma(a, y.x, pf[b][0]);
-                pf[b][1] = fma(a, y.y, pf[b][1]);
-              }
-          }
+          fn_counted<MAXF, MINF>(minef, [&](auto m) { fn_product<NP, decltype(m)::value>(A, Z, n8, fx, fy, pf); });
 #pragma unroll
           for (int b = 0; b < MAXF; b++)
             if (b < minef) *reinterpret_cast<double2*>(P + fx[b] * NP + fy[b]) = make_double2(pf[b][0], pf[b][1]);
           __syncthreads();
 #pragma unroll
           for (int b = 0; b < MAXL; b++) acc[b][0] = acc[b][1] = 0.0;
-          fn_lower_product<NP>(Z, P, n8, mine, xo, yo, acc);
+          fn_counted<MAXL, MINL>(mine, [&](auto m) { fn_product<NP, decltype(m)::value>(Z, P, n8, xo, yo, acc); });
 #pragma unroll
           for (int b = 0; b < MAXL; b++)
 #pragma unroll
@@ -623,17 +646,17 @@ __global__ void __launch_bounds__(FN_NT, FnCfg<NP>::MINB) core_f64_ns_kernel(
 #pragma unroll
           for (int a = 0; a < C::TR; a++)
 #pragma unroll
-            for (int b = 0; b < C::TC; b++) z[a][b] = Z32[(i0 + a) * NP + j0 + b];
+            for (int b = 0; b < C::TC; b++) z[a][b] = Z32[(i0 + a) * NP + fn_col<NP>(tx, b)];
           __syncthreads();
         }
 #pragma unroll
         for (int b = 0; b < C::TC; b++) {
           float m[C::TR];
-          fn_ld<C::TR>(R32 + (j0 + b) * NP + i0, m);
+          fn_ld<C::TR>(R32 + fn_col<NP>(tx, b) * NP + i0, m);
 #pragma unroll
           for (int a = 0; a < C::TR; a++) {
-            double* zz = Z + (i0 + a) * NP + j0 + b;
-            *zz = (it == 0 ? (double)z[a][b] : *zz) + (double)(0.25f * (R32[(i0 + a) * NP + j0 + b] + m[a]));
+            double* zz = Z + (i0 + a) * NP + fn_col<NP>(tx, b);
+            *zz = (it == 0 ? (double)z[a][b] : *zz) + (double)(0.25f * (R32[(i0 + a) * NP + fn_col<NP>(tx, b)] + m[a]));
           }
         }
         __syncthreads();
@@ -687,7 +710,7 @@ __global__ void __launch_bounds__(FN_NT, FnCfg<NP>::MINB) core_f64_ns_kernel(
       double* Pa = pao + (size_t)p * n * n;
 #pragma unroll
       for (int b = 0; b < MAXL; b++) acc[b][0] = acc[b][1] = 0.0;
-      fn_lower_product<NP>(Z, Z, n8, mine, xo, yo, acc);
+      fn_counted<MAXL, MINL>(mine, [&](auto m) { fn_product<NP, decltype(m)::value>(Z, Z, n8, xo, yo, acc); });
 #pragma unroll
       for (int b = 0; b < MAXL; b++)
         if (b < mine) {
