@@ -53,14 +53,62 @@ __global__ void lk_weights_kernel(int64_t n, const float* __restrict__ rdiag, co
   if (i < n) w[i] = wloc ? 1.0f / rdiag[i] : rloc[i] / rdiag[i];
 }
 
-// per point: p1, p3, b = Ywᵀ dep, trace, branch, A = G + cI, s, Y0, Z0
-__global__ void __launch_bounds__(LKP_NT) lk_prep_kernel(int ne, int kp, const int64_t* __restrict__ offs,
+// One of LK_PIECES pieces of a point's list: b = Ywᵀ dep (FP32 within a piece),
+// p1 = sum w dep^2, p3 = sum rloc.  A block per point walked the whole list one
+// row after the other: 24,000 rows of k = 512 took 6 ms for four points.
+constexpr int LK_PIECES = 32;
+
+__global__ void __launch_bounds__(LKP_NT) lk_sums_kernel(int ne, int kp, const int64_t* __restrict__ offs,
                                                           const float* __restrict__ rows,
                                                           const __nv_bfloat16* __restrict__ rows16,
                                                           const int* __restrict__ ridx,
                                                           const float* __restrict__ w,
                                                           const float* __restrict__ dep,
-                                                          const float* __restrict__ rloc, const double* infl_in,
+                                                          const float* __restrict__ rloc, float* pb, double* pp) {
+  __shared__ double red[LKP_NT / 32];
+  const int b = blockIdx.y, piece = blockIdx.x, tid = threadIdx.x;
+  const int64_t r0 = offs[b];
+  const int L = (int)(offs[b + 1] - r0), per = (L + LK_PIECES - 1) / LK_PIECES;
+  const int l0 = min(L, piece * per), l1 = min(L, l0 + per);
+  // list entry e: its row (packed, or observation ridx[e]) and departure
+  auto row_of = [&](int64_t e) -> size_t { return ridx ? (size_t)ridx[e] : (size_t)e; };
+  for (int m = tid; m < kp; m += LKP_NT) {
+    float acc = 0.f;
+    if (m < ne) {
+      if (rows16) {
+#pragma unroll 8
+        for (int l = l0; l < l1; l++) {
+          const size_t r = row_of(r0 + l);
+          acc = fmaf(w[r0 + l] * dep[r], __bfloat162float(rows16[r * ne + m]), acc);
+        }
+      } else {
+#pragma unroll 8
+        for (int l = l0; l < l1; l++) {
+          const size_t r = row_of(r0 + l);
+          acc = fmaf(w[r0 + l] * dep[r], rows[r * ne + m], acc);
+        }
+      }
+    }
+    pb[((size_t)b * LK_PIECES + piece) * kp + m] = acc;
+  }
+  double p1 = 0.0, p3 = 0.0;
+  for (int l = l0 + tid; l < l1; l += LKP_NT) {
+    const double d = dep[row_of(r0 + l)];
+    p1 += d * d * (double)w[r0 + l];
+    p3 += (double)rloc[r0 + l];
+  }
+  p1 = block_sum<double, LKP_NT>(p1, red);
+  p3 = block_sum<double, LKP_NT>(p3, red);
+  if (tid == 0) {
+    pp[2 * (b * LK_PIECES + piece)] = p1;
+    pp[2 * (b * LK_PIECES + piece) + 1] = p3;
+  }
+}
+
+// per point: p1, p3, b, trace, branch, A = G + cI, s, Y0, Z0
+__global__ void __launch_bounds__(LKP_NT) lk_prep_kernel(int ne, int kp, const int64_t* __restrict__ offs,
+                                                          const float* __restrict__ pb,
+                                                          const double* __restrict__ pp, const double* infl_in,
                                                           double minfl, float* G, float* Y, float* Z,
                                                           float* bvec, float* inv_s, LkPoint* pt, int* active) {
   __shared__ double red[LKP_NT / 32];
@@ -68,8 +116,7 @@ __global__ void __launch_bounds__(LKP_NT) lk_prep_kernel(int ne, int kp, const i
   __shared__ __align__(16) float yv[1024];
   __shared__ float redf[LKP_NT / 32];
   const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const int64_t r0 = offs[b];
-  const int L = (int)(offs[b + 1] - r0);
+  const int L = (int)(offs[b + 1] - offs[b]);
   const size_t mo = (size_t)b * kp * kp;
   float* A = G + mo;
   auto bsum = [&](double v) {
@@ -81,27 +128,15 @@ __global__ void __launch_bounds__(LKP_NT) lk_prep_kernel(int ne, int kp, const i
     for (int i = 0; i < LKP_NT / 32; i++) t += red[i];
     return t;
   };
-  // list entry e: its row (packed, or observation ridx[e]) and departure
-  auto row_of = [&](int64_t e) -> size_t { return ridx ? (size_t)ridx[e] : (size_t)e; };
-  auto dep_of = [&](int64_t e) -> float { return dep[row_of(e)]; };
   double p1 = 0.0, p3 = 0.0;
-  for (int l = tid; l < L; l += LKP_NT) {
-    const double d = dep_of(r0 + l);
-    p1 += d * d * (double)w[r0 + l];
-    p3 += (double)rloc[r0 + l];
+  for (int i = 0; i < LK_PIECES; i++) {
+    p1 += pp[2 * (b * LK_PIECES + i)];
+    p3 += pp[2 * (b * LK_PIECES + i) + 1];
   }
-  p1 = bsum(p1);
-  p3 = bsum(p3);
   for (int m = tid; m < kp; m += LKP_NT) {
-    float acc = 0.f;
-    if (m < ne) {
-      if (rows16)
-        for (int l = 0; l < L; l++)
-          acc = fmaf(w[r0 + l] * dep_of(r0 + l), __bfloat162float(rows16[row_of(r0 + l) * ne + m]), acc);
-      else
-        for (int l = 0; l < L; l++) acc = fmaf(w[r0 + l] * dep_of(r0 + l), rows[row_of(r0 + l) * ne + m], acc);
-    }
-    bvec[(size_t)b * kp + m] = acc;
+    double acc = 0.0;
+    for (int i = 0; i < LK_PIECES; i++) acc += (double)pb[((size_t)b * LK_PIECES + i) * kp + m];
+    bvec[(size_t)b * kp + m] = (float)acc;
   }
   double tr = 0.0;
   for (int m = tid; m < ne; m += LKP_NT) tr += (double)A[(size_t)m * kp + m];
@@ -503,12 +538,27 @@ static int launch_lk_update(int ne, int npts, int nv, const void* xb, const floa
   return cuda_status(cudaGetLastError());
 }
 
+// out += the other pieces of a split Gram
+__global__ void lk_join_kernel(int64_t n4, LkGemmArgs a) {
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n4; t += (int64_t)gridDim.x * blockDim.x) {
+    float4 v = reinterpret_cast<const float4*>(a.outs[0])[t];
+    for (int i = 1; i < a.nsplit; i++) {
+      const float4 u = reinterpret_cast<const float4*>(a.outs[i])[t];
+      v.x += u.x;
+      v.y += u.y;
+      v.z += u.z;
+      v.w += u.w;
+    }
+    reinterpret_cast<float4*>(a.outs[0])[t] = v;
+  }
+}
+
 template <int MODE>
 static int lk_gemm(const LkGemmArgs& a, int nb, cudaStream_t s) {
   static_assert(LK_SMEM <= 227 * 1024, "shared memory");
   cudaError_t e = cudaFuncSetAttribute(largek_gemm_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, LK_SMEM);
   if (e != cudaSuccess) return cuda_status(e);
-  dim3 grid(a.kp / LK_TILE, a.kp / LK_TILE, nb);
+  dim3 grid(a.kp / LK_TILE, a.kp / LK_TILE, nb * (MODE == LK_GRAM ? a.nsplit : 1));
   largek_gemm_kernel<MODE><<<grid, LK_NT, LK_SMEM, s>>>(a);
   note_launch();
   return cuda_status(cudaGetLastError());
@@ -569,11 +619,16 @@ static int largek_core(int ne, int npts, const int64_t* offs, const float* rows,
   const size_t mat = (size_t)kp * kp;
   // batch: six kp x kp FP32 matrices per point, at most 1.5 GB
   int B = (int)std::min<size_t>((size_t)npts, std::max<size_t>(1, (size_t)(1536u << 20) / (6 * mat * 4)));
+  int dev = 0, nsm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   int64_t nrows = 0;
   if (cudaMemcpyAsync(&nrows, offs + npts, sizeof(int64_t), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
       cudaStreamSynchronize(s) != cudaSuccess)
     return LETKF_ERR_CUDA;
   float *w = nullptr, *G = nullptr, *Y = nullptr, *Z = nullptr, *Yn = nullptr, *Zn = nullptr, *T = nullptr;
+  float* pb = nullptr;
+  double* pp = nullptr;
   float *bvec = nullptr, *e2 = nullptr, *inv_s = nullptr, *alphas = nullptr, *betas = nullptr;
   int *active = nullptr, *count = nullptr, *err = nullptr, *restart = nullptr;
   LkPoint* pt = nullptr;
@@ -587,6 +642,8 @@ static int largek_core(int ne, int npts, const int64_t* offs, const float* rows,
   A(&Zn, sizeof(float) * mat * B);
   A(&T, sizeof(float) * mat * B);
   A(&bvec, sizeof(float) * (size_t)kp * B);
+  A(&pb, sizeof(float) * (size_t)kp * B * LK_PIECES);
+  A(&pp, sizeof(double) * 2 * B * LK_PIECES);
   A(&e2, sizeof(float) * B);
   A(&inv_s, sizeof(float) * B);
   A(&alphas, sizeof(float) * B);
@@ -610,6 +667,13 @@ static int largek_core(int ne, int npts, const int64_t* offs, const float* rows,
     g.mstride = (int64_t)mat;
     g.err_flag = err;
     // 1. Gram
+    // long lists over few points: their K in pieces on more CTAs, the pieces in
+    // the matrices that the iteration does not use yet
+    const int64_t tiles = (int64_t)nb * (kp / LK_TILE) * (kp / LK_TILE);
+    const bool split = nrows / npts >= LK_SPLIT_L && tiles < 2 * nsm;
+    float* const parts[LK_SPLITS] = {G, Y, Z, Yn, Zn, T};
+    for (int i = 0; i < LK_SPLITS; i++) g.outs[i] = parts[i];
+    g.nsplit = split ? LK_SPLITS : 1;
     g.out = G;
     g.rows = rows;
     g.rows16 = rows16;
@@ -619,9 +683,16 @@ static int largek_core(int ne, int npts, const int64_t* offs, const float* rows,
     g.ne = ne;
     st = lk_gemm<LK_GRAM>(g, nb, s);
     if (st) break;
+    if (split) {
+      lk_join_kernel<<<1024, 256, 0, s>>>((int64_t)mat * nb / 4, g);
+      note_launch();
+    }
+    g.nsplit = 1;
     // 2. prep
-    lk_prep_kernel<<<nb, LKP_NT, 0, s>>>(ne, kp, offs + p0, rows, rows16, ridx, w, dep, rloc, parm_infl + p0, minfl,
-                                         G, Y, Z, bvec, inv_s, pt, active);
+    lk_sums_kernel<<<dim3(LK_PIECES, nb), LKP_NT, 0, s>>>(ne, kp, offs + p0, rows, rows16, ridx, w, dep, rloc, pb, pp);
+    lk_prep_kernel<<<nb, LKP_NT, 0, s>>>(ne, kp, offs + p0, pb, pp, parm_infl + p0, minfl, G, Y, Z, bvec, inv_s, pt,
+                                         active);
+    note_launch();
     note_launch();
     // 3. coupled Newton-Schulz
     g.rows = nullptr;
@@ -721,7 +792,7 @@ static int largek_core(int ne, int npts, const int64_t* offs, const float* rows,
     st = cuda_status(cudaStreamSynchronize(s));
     if (st == LETKF_OK && h_err) st = LETKF_ERR_TIMEOUT;
   }
-  void* fr[] = {w, G, Y, Z, Yn, Zn, T, bvec, e2, inv_s, alphas, betas, active, count, err, pt, restart};
+  void* fr[] = {w, G, Y, Z, Yn, Zn, T, bvec, e2, inv_s, alphas, betas, active, count, err, pt, restart, pb, pp};
   for (void* p : fr)
     if (p) cudaFreeAsync(p, s);
   // points whose mixed-precision transform did not certify: the FP64 pass

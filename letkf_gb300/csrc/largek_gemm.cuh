@@ -36,6 +36,12 @@ constexpr int LK_STAGE = 4 * LK_OPER;    // A_hi, A_lo, B_hi, B_lo
 constexpr int LK_SMEM = 2 * LK_STAGE + 64;
 constexpr uint32_t LK_TMEM_COLS = 128;
 constexpr uint32_t LK_WAIT = 1u << 22;
+// The Gram's K is split over LK_SPLITS CTAs where the tiles alone are less than
+// two waves and the mean list is LK_SPLIT_L long: four points of k = 512 with
+// 24,000 rows are 64 tiles of 1,500 stages, 6.4 ms; split 1.2.  Shorter
+// lists keep one accumulator (and their bits).
+constexpr int LK_SPLITS = 6;
+constexpr int LK_SPLIT_L = 4096;
 
 enum { LK_GRAM = 0, LK_T = 1, LK_AXPBY = 2 };
 
@@ -58,6 +64,8 @@ struct LkGemmArgs {
   const float* wts;       // [nrows] weight of each row (rloc / rdiag)
   const int64_t* offs;    // [batch + 1] rows of point b: offs[b] .. offs[b+1]-1
   int ne;
+  int nsplit;             // pieces of K, each a CTA's with its own output
+  float* outs[LK_SPLITS];
   int* err_flag;
 };
 
@@ -85,7 +93,8 @@ __global__ void __launch_bounds__(LK_NT, 3) largek_gemm_kernel(LkGemmArgs a) {
   uint64_t* mbar = reinterpret_cast<uint64_t*>(sm + 2 * LK_STAGE);
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(sm + 2 * LK_STAGE + 16);
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const int b = blockIdx.z;
+  const int nsp = MODE == LK_GRAM ? a.nsplit : 1;
+  const int b = blockIdx.z / nsp, sp = blockIdx.z - b * nsp;
   const int m0 = blockIdx.y * LK_TILE, n0 = blockIdx.x * LK_TILE;
   const int kp = a.kp;
   const size_t mo = (size_t)b * a.mstride;
@@ -101,12 +110,18 @@ __global__ void __launch_bounds__(LK_NT, 3) largek_gemm_kernel(LkGemmArgs a) {
     return;
   }
   int nk;
+  int kfirst = 0;  // first stage of this CTA's piece of K
   int64_t r0 = 0;
   int L = 0;
   if (MODE == LK_GRAM) {
     r0 = a.offs[b];
     L = (int)(a.offs[b + 1] - r0);
     nk = (L + LK_KC - 1) / LK_KC;
+    if (nsp > 1) {
+      const int per = (nk + nsp - 1) / nsp;
+      kfirst = min(nk, sp * per);
+      nk = min(nk, kfirst + per) - kfirst;
+    }
   } else {
     nk = kp / LK_KC;
   }
@@ -134,7 +149,7 @@ __global__ void __launch_bounds__(LK_NT, 3) largek_gemm_kernel(LkGemmArgs a) {
   // so their latency overlaps the staging, the barrier and the MMA issue
   float va[8], vb[8];
   auto load_stage = [&](int c, float (&xa)[8], float (&xb)[8]) {
-    const int k0 = c * LK_KC + h * 8;
+    const int k0 = (MODE == LK_GRAM ? kfirst + c : c) * LK_KC + h * 8;
     if (MODE == LK_GRAM) {
       // A(m, l) = w_l y_l[m], B(n, l) = y_l[n]; rows beyond L or members beyond ne are 0
 #pragma unroll
@@ -246,7 +261,7 @@ __global__ void __launch_bounds__(LK_NT, 3) largek_gemm_kernel(LkGemmArgs a) {
 #pragma unroll
         for (int j = 0; j < 16; j++) v[j] = 0.f;
       }
-      float* dst = a.out + orow + c0;
+      float* dst = (MODE == LK_GRAM && nsp > 1 ? a.outs[sp] : a.out) + orow + c0;
       if (MODE == LK_AXPBY) {
         const float al = a.alpha_b ? a.alpha_b[b] : a.alpha;
         const float be = a.beta_b ? a.beta_b[b] : a.beta;
