@@ -105,16 +105,21 @@ __global__ void __launch_bounds__(LKP_NT) lk_sums_kernel(int ne, int kp, const i
   }
 }
 
-// per point: p1, p3, b, trace, branch, A = G + cI, s, Y0, Z0
-__global__ void __launch_bounds__(LKP_NT) lk_prep_kernel(int ne, int kp, const int64_t* __restrict__ offs,
+// per point: p1, p3, b, trace, branch, A = G + cI, s, Y0, Z0.  Eight reads of A
+// (Gershgorin's goes with the power iteration's first) and the writes of Y and
+// Z bound it; 16 warps a point keep the loads in flight.  k = 512, 256 points:
+// 1157 -> 536 us.
+constexpr int LKQ_NT = 512;
+
+__global__ void __launch_bounds__(LKQ_NT, 2) lk_prep_kernel(int ne, int kp, const int64_t* __restrict__ offs,
                                                           const float* __restrict__ pb,
                                                           const double* __restrict__ pp, const double* infl_in,
                                                           double minfl, float* G, float* Y, float* Z,
                                                           float* bvec, float* inv_s, LkPoint* pt, int* active) {
-  __shared__ double red[LKP_NT / 32];
+  __shared__ double red[LKQ_NT / 32];
   __shared__ __align__(16) float xv[1024];
   __shared__ __align__(16) float yv[1024];
-  __shared__ float redf[LKP_NT / 32];
+  __shared__ float redf[LKQ_NT / 32];
   const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int L = (int)(offs[b + 1] - offs[b]);
   const size_t mo = (size_t)b * kp * kp;
@@ -125,7 +130,7 @@ __global__ void __launch_bounds__(LKP_NT) lk_prep_kernel(int ne, int kp, const i
     if (lane == 0) red[wid] = v;
     __syncthreads();
     double t = 0.0;
-    for (int i = 0; i < LKP_NT / 32; i++) t += red[i];
+    for (int i = 0; i < LKQ_NT / 32; i++) t += red[i];
     return t;
   };
   double p1 = 0.0, p3 = 0.0;
@@ -133,13 +138,13 @@ __global__ void __launch_bounds__(LKP_NT) lk_prep_kernel(int ne, int kp, const i
     p1 += pp[2 * (b * LK_PIECES + i)];
     p3 += pp[2 * (b * LK_PIECES + i) + 1];
   }
-  for (int m = tid; m < kp; m += LKP_NT) {
+  for (int m = tid; m < kp; m += LKQ_NT) {
     double acc = 0.0;
     for (int i = 0; i < LK_PIECES; i++) acc += (double)pb[((size_t)b * LK_PIECES + i) * kp + m];
     bvec[(size_t)b * kp + m] = (float)acc;
   }
   double tr = 0.0;
-  for (int m = tid; m < ne; m += LKP_NT) tr += (double)A[(size_t)m * kp + m];
+  for (int m = tid; m < ne; m += LKQ_NT) tr += (double)A[(size_t)m * kp + m];
   tr = bsum(tr);
   double infl = infl_in[b];
   int kind = 0;
@@ -170,43 +175,34 @@ __global__ void __launch_bounds__(LKP_NT) lk_prep_kernel(int ne, int kp, const i
   }
   if (kind != 0) return;
   const float cf = (float)c;
-  for (int m = tid; m < kp; m += LKP_NT) A[(size_t)m * kp + m] = (m < ne ? A[(size_t)m * kp + m] : 0.f) + cf;
+  for (int m = tid; m < kp; m += LKQ_NT) A[(size_t)m * kp + m] = (m < ne ? A[(size_t)m * kp + m] : 0.f) + cf;
   __syncthreads();
   // Gershgorin bound and power iteration (s >= lambda_max / 2 keeps Newton-Schulz convergent);
   // one warp per row, the lanes over 16-byte column groups (coalesced row reads)
   const int kp4 = kp / 4;
   float gmax = 0.f;
-  for (int m = wid; m < kp; m += LKP_NT / 32) {
-    const float4* row4 = reinterpret_cast<const float4*>(A + (size_t)m * kp);
-    float g = 0.f;
-    for (int j4 = lane; j4 < kp4; j4 += 32) {
-      const float4 x = row4[j4];
-      g += (fabsf(x.x) + fabsf(x.y)) + (fabsf(x.z) + fabsf(x.w));
-    }
-    gmax = fmaxf(gmax, warp_sum(g));
-  }
-  for (int m = tid; m < kp; m += LKP_NT) xv[m] = A[(size_t)m * kp + m] * (1.f + 0.25f * __sinf(1.7f * m));
+  for (int m = tid; m < kp; m += LKQ_NT) xv[m] = A[(size_t)m * kp + m] * (1.f + 0.25f * __sinf(1.7f * m));
   __syncthreads();
-  if (lane == 0) redf[wid] = gmax;
-  __syncthreads();
-  gmax = 0.f;
-  for (int i = 0; i < LKP_NT / 32; i++) gmax = fmaxf(gmax, redf[i]);
   float lam = 0.f;
   const float4* xv4 = reinterpret_cast<const float4*>(xv);
   for (int it = 0; it < 8; it++) {
-    for (int m = wid; m < kp; m += LKP_NT / 32) {
+    for (int m = wid; m < kp; m += LKQ_NT / 32) {
       const float4* row4 = reinterpret_cast<const float4*>(A + (size_t)m * kp);
-      float acc = 0.f;
+      float acc = 0.f, g = 0.f;
+#pragma unroll 4
       for (int j4 = lane; j4 < kp4; j4 += 32) {
         const float4 x = row4[j4], v = xv4[j4];
         acc = fmaf(x.x, v.x, fmaf(x.y, v.y, fmaf(x.z, v.z, fmaf(x.w, v.w, acc))));
+        g += (fabsf(x.x) + fabsf(x.y)) + (fabsf(x.z) + fabsf(x.w));
       }
       acc = warp_sum(acc);
+      if (it == 0) gmax = fmaxf(gmax, warp_sum(g));
       if (lane == 0) yv[m] = acc;
     }
+    if (it == 0 && lane == 0) redf[wid] = gmax;
     __syncthreads();
     double nrm2 = 0.0, x2 = 0.0;
-    for (int m = tid; m < kp; m += LKP_NT) {
+    for (int m = tid; m < kp; m += LKQ_NT) {
       nrm2 += (double)yv[m] * yv[m];
       x2 += (double)xv[m] * xv[m];
     }
@@ -214,9 +210,10 @@ __global__ void __launch_bounds__(LKP_NT) lk_prep_kernel(int ne, int kp, const i
     x2 = bsum(x2);
     lam = (float)sqrt(nrm2 / fmax(x2, 1e-300));
     const float inv = (float)(1.0 / sqrt(fmax(nrm2, 1e-300)));
-    for (int m = tid; m < kp; m += LKP_NT) xv[m] = yv[m] * inv;
+    for (int m = tid; m < kp; m += LKQ_NT) xv[m] = yv[m] * inv;
     __syncthreads();
   }
+  for (int i = 0; i < LKQ_NT / 32; i++) gmax = fmaxf(gmax, redf[i]);
   const float s = lam > 0.f ? 1.05f * lam : gmax;
   const float is = 1.f / s;
   if (tid == 0) {
@@ -226,12 +223,16 @@ __global__ void __launch_bounds__(LKP_NT) lk_prep_kernel(int ne, int kp, const i
     pt[b].steps = 0;
     inv_s[b] = is;
   }
-  float* Yb = Y + mo;
-  float* Zb = Z + mo;
-  for (int64_t idx = tid; idx < (int64_t)kp * kp; idx += LKP_NT) {
-    const int i = (int)(idx / kp), j = (int)(idx - (int64_t)i * kp);
-    Yb[idx] = A[idx] * is;
-    Zb[idx] = i == j ? 1.f : 0.f;
+  for (int m = wid; m < kp; m += LKQ_NT / 32) {
+    const size_t at = mo + (size_t)m * kp;
+#pragma unroll 4
+    for (int j4 = lane; j4 < kp4; j4 += 32) {
+      const float4 x = reinterpret_cast<const float4*>(G + at)[j4];
+      const int dg = m - 4 * j4;  // the diagonal's place in the group
+      reinterpret_cast<float4*>(Y + at)[j4] = make_float4(x.x * is, x.y * is, x.z * is, x.w * is);
+      reinterpret_cast<float4*>(Z + at)[j4] =
+          make_float4(dg == 0 ? 1.f : 0.f, dg == 1 ? 1.f : 0.f, dg == 2 ? 1.f : 0.f, dg == 3 ? 1.f : 0.f);
+    }
   }
 }
 
@@ -370,105 +371,120 @@ __global__ void __launch_bounds__(LKP_NT) lk_certify_kernel(int ne, int kp, cons
   }
 }
 
-// Z <- (Zn + Znᵀ) / 2 for active points
-__global__ void lk_symmetrize_kernel(int kp, const float* __restrict__ Zn, float* Z, const int* __restrict__ active) {
-  const int b = blockIdx.y;
-  if (!active[b]) return;
+// Z <- (Zn + Znᵀ) / 2 for active points: a CTA has a 32 x 32 tile on or below
+// the diagonal and its mirror tile, turned in shared memory
+__global__ void __launch_bounds__(LKP_NT) lk_symmetrize_kernel(int kp, const float* __restrict__ Zn, float* Z,
+                                                               const int* __restrict__ active) {
+  __shared__ float t[32][33], u[32][33];
+  const int b = blockIdx.z;
+  if (!active[b] || blockIdx.x > blockIdx.y) return;
   const size_t mo = (size_t)b * kp * kp;
-  for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < (int64_t)kp * kp;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    const int i = (int)(idx / kp), j = (int)(idx - (int64_t)i * kp);
-    Z[mo + idx] = 0.5f * (Zn[mo + idx] + Zn[mo + (size_t)j * kp + i]);
+  const int i0 = blockIdx.y * 32, j0 = blockIdx.x * 32, c = threadIdx.x & 31;
+  for (int r = threadIdx.x >> 5; r < 32; r += LKP_NT / 32) {
+    t[r][c] = Zn[mo + (size_t)(i0 + r) * kp + j0 + c];
+    u[r][c] = Zn[mo + (size_t)(j0 + r) * kp + i0 + c];
+  }
+  __syncthreads();
+  for (int r = threadIdx.x >> 5; r < 32; r += LKP_NT / 32) {
+    Z[mo + (size_t)(i0 + r) * kp + j0 + c] = 0.5f * (t[r][c] + u[c][r]);
+    Z[mo + (size_t)(j0 + r) * kp + i0 + c] = 0.5f * (u[r][c] + t[c][r]);
   }
 }
 
-// W, wbar, inflation, status for the points of a batch
-__global__ void __launch_bounds__(LKP_NT) lk_finalize_kernel(int ne, int kp, const float* __restrict__ Z,
-                                                              const float* __restrict__ bvec,
+// y = Z x for the points that have a transform, LKF_NT rows a CTA.  Z is
+// symmetric to the bit, so its rows are read as columns (whole lines).
+constexpr int LKF_NT = 128;
+
+__global__ void __launch_bounds__(LKF_NT) lk_matvec_kernel(int ne, int kp, const float* __restrict__ Z,
+                                                            const float* __restrict__ x,
+                                                            const LkPoint* __restrict__ pt, float* y) {
+  __shared__ float v[LETKF_LARGEK_MAX_NE];
+  const int b = blockIdx.y, m = blockIdx.x * LKF_NT + threadIdx.x;
+  if (pt[b].kind != 0) return;
+  for (int j = threadIdx.x; j < ne; j += LKF_NT) v[j] = x[(size_t)b * kp + j];
+  __syncthreads();
+  if (m >= ne) return;
+  const float* Zb = Z + (size_t)b * kp * kp;
+  float acc = 0.f;
+#pragma unroll 16
+  for (int j = 0; j < ne; j++) acc = fmaf(Zb[(size_t)j * kp + m], v[j], acc);
+  y[(size_t)b * kp + m] = acc;
+}
+
+// W, wbar = h / s (h = Z Z b), inflation, status for the points of a batch,
+// LKF_NT rows a CTA
+__global__ void __launch_bounds__(LKF_NT) lk_finalize_kernel(int ne, int kp, const float* __restrict__ Z,
+                                                              const float* __restrict__ hvec,
                                                               const LkPoint* __restrict__ pt, double* infl,
                                                               float* trans, float* transm, int* status) {
-  __shared__ float g[1024];
-  const int b = blockIdx.x, tid = threadIdx.x;
+  const int b = blockIdx.y, tid = threadIdx.x;
+  const int m0 = blockIdx.x * LKF_NT, m1 = min(ne, m0 + LKF_NT);
   const LkPoint q = pt[b];
   float* tr = trans + (size_t)b * ne * ne;
-  if (q.kind != 0) {
-    const float d = q.kind == 1 ? (float)sqrt(q.infl) : 1.f;
-    for (int idx = tid; idx < ne * ne; idx += LKP_NT) tr[idx] = (idx / ne == idx % ne) ? d : 0.f;
-    if (transm)
-      for (int m = tid; m < ne; m += LKP_NT) transm[(size_t)b * ne + m] = 0.f;
-    if (tid == 0) status[b] = q.kind == 1 ? LETKF_OK : (q.kind == 2 ? LETKF_ERR_CAPACITY : LETKF_ERR_EIG);
-    return;
-  }
-  const float* Zb = Z + (size_t)b * kp * kp;
-  const float* bv = bvec + (size_t)b * kp;
-  for (int m = tid; m < ne; m += LKP_NT) {
-    float acc = 0.f;
-    for (int j = 0; j < ne; j++) acc = fmaf(Zb[(size_t)m * kp + j], bv[j], acc);
-    g[m] = acc;
-  }
-  __syncthreads();
-  const float inv_s = (float)(1.0 / q.s);
-  if (transm)
-    for (int m = tid; m < ne; m += LKP_NT) {
-      float acc = 0.f;
-      for (int j = 0; j < ne; j++) acc = fmaf(Zb[(size_t)m * kp + j], g[j], acc);
-      transm[(size_t)b * ne + m] = acc * inv_s;
-    }
+  const float d = q.kind == 1 ? (float)sqrt(q.infl) : 1.f;
   const float coef = (float)sqrt((double)(ne - 1) / q.s);
+  const float* Zb = Z + (size_t)b * kp * kp;
   // trans(k, m) = W[k][m] at column-major index m * ne + k (W symmetric)
-  for (int idx = tid; idx < ne * ne; idx += LKP_NT) {
-    const int m = idx / ne, k = idx - m * ne;
-    tr[idx] = coef * Zb[(size_t)k * kp + m];
-  }
-  if (tid == 0) {
-    infl[b] = infl_update(ne, q.infl, q.p1, q.trace, q.p3);
-    status[b] = LETKF_OK;
+#pragma unroll 4
+  for (int m = m0; m < m1; m++)
+    for (int k = tid; k < ne; k += LKF_NT)
+      tr[(size_t)m * ne + k] = q.kind != 0 ? (k == m ? d : 0.f) : coef * Zb[(size_t)m * kp + k];
+  if (transm && m0 + tid < m1)
+    transm[(size_t)b * ne + m0 + tid] = q.kind != 0 ? 0.f : hvec[(size_t)b * kp + m0 + tid] * (float)(1.0 / q.s);
+  if (blockIdx.x == 0 && tid == 0) {
+    if (q.kind == 0) infl[b] = infl_update(ne, q.infl, q.p1, q.trace, q.p3);
+    status[b] = q.kind <= 1 ? LETKF_OK : (q.kind == 2 ? LETKF_ERR_CAPACITY : LETKF_ERR_EIG);
   }
 }
 
 // xa(p,m,v) = mean + sum_k xb'(k) (trans(k,m) + transm(k)) for any ne: the
-// product in FP32 from 32-row tiles of trans staged through shared memory,
-// the mean and the mean increment in FP64 (as the fused sweeps)
-constexpr int LKU_KT = 32;
+// product in FP32, the mean and the mean increment in FP64 (as the fused
+// sweeps).  What it cannot do without is one read of trans; a warp has 32 of
+// its columns and stages 32 x 32 tiles of them (whole lines, the next tile's
+// loads in flight during a tile's products) in its own shared memory, so that
+// no barrier of the CTA lies between the loads.  A point is one CTA's: xa may
+// be xb.  k = 512, 256 points, 6 variables: 505 -> 113 us.
+constexpr int LKU_MAX_NT = 512;
+constexpr int LKU_LD = 33;  // padded row of a tile (conflict-free both ways)
 
-// floats before the FP64 array of lk_update_kernel's shared memory (8-byte aligned)
-__host__ __device__ constexpr int lku_base_floats(int nv, int ne) {
-  return (nv * ne + LKU_KT * (ne + 1) + 1) & ~1;
-}
+// threads of the CTA of a point
+static int lku_threads(int ne) { return std::min(LKU_MAX_NT, std::max(128, (ne + 31) / 32 * 32)); }
+// floats of a variable's perturbations, 16-byte rows
+__host__ __device__ constexpr int lku_xld(int ne) { return (ne + 3) & ~3; }
 
 // BF == false: xb, xa [nv][npts][ne] FP32 members.  BF == true: members
 // stored as an FP32 mean xmean [nv][npts] plus BF16 perturbations xb
 // [nv][npts][ne]; the analysis likewise (amean = mean + xb' transm in FP64,
 // xa = xb' trans rounded to BF16)
 template <bool BF>
-__global__ void __launch_bounds__(LKP_NT) lk_update_kernel(int ne, int npts, int nv, const void* __restrict__ xb_,
+__global__ void __launch_bounds__(LKU_MAX_NT, 2) lk_update_kernel(int ne, int npts, int nv, const void* __restrict__ xb_,
                                                             const float* __restrict__ xmean,
                                                             const float* __restrict__ trans,
                                                             const float* __restrict__ transm, void* xa_,
                                                             float* amean) {
   extern __shared__ __align__(16) float su[];
-  const int ld = ne + 1;                   // padded row of the staged tile (conflict-free columns)
-  float* xs = su;                          // [nv][ne] perturbations
-  float* tt = xs + nv * ne;                // [LKU_KT][ld] trans(k0 + kk, m)
-  double* base = reinterpret_cast<double*>(su + lku_base_floats(nv, ne));  // [nv] mean + increment
+  __shared__ double base[8];               // mean + increment
+  const int xld = lku_xld(ne), nt = blockDim.x;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  float* xs = su;                          // [nv][xld] perturbations
+  float* tt = xs + nv * xld + wid * 32 * LKU_LD;  // [32][LKU_LD] trans(k0 + kk, m0 + i)
   for (int p = blockIdx.x; p < npts; p += gridDim.x) {
     __syncthreads();
-    for (int t = tid; t < nv * ne; t += LKP_NT) {
+    for (int t = tid; t < nv * ne; t += nt) {
       const int v = t / ne, m = t - v * ne;
       const size_t at = ((size_t)v * npts + p) * ne + m;
-      xs[t] = BF ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(xb_)[at])
-                 : reinterpret_cast<const float*>(xb_)[at];
+      xs[v * xld + m] = BF ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(xb_)[at])
+                           : reinterpret_cast<const float*>(xb_)[at];
     }
     __syncthreads();
-    for (int v = wid; v < nv; v += LKP_NT / 32) {
+    for (int v = wid; v < nv; v += nt / 32) {
       double sx = 0.0;
-      for (int m = lane; m < ne; m += 32) sx += (double)xs[v * ne + m];
+      for (int m = lane; m < ne; m += 32) sx += (double)xs[v * xld + m];
       const double mean = warp_sum(sx) / (double)ne;  // of the members (BF: of the stored perturbations)
       double dl = 0.0;
       for (int m = lane; m < ne; m += 32) {
-        const float x = (float)((double)xs[v * ne + m] - mean);
-        xs[v * ne + m] = x;
+        const float x = (float)((double)xs[v * xld + m] - mean);
+        xs[v * xld + m] = x;
         if (transm) dl += (double)x * (double)transm[(size_t)p * ne + m];
       }
       dl = warp_sum(dl);
@@ -481,44 +497,57 @@ __global__ void __launch_bounds__(LKP_NT) lk_update_kernel(int ne, int npts, int
         }
       }
     }
-    float acc[8][2];
-#pragma unroll
-    for (int v = 0; v < 8; v++) acc[v][0] = acc[v][1] = 0.f;
+    __syncthreads();
     const float* tp = trans + (size_t)p * ne * ne;
-    for (int k0 = 0; k0 < ne; k0 += LKU_KT) {
-      const int kn = min(LKU_KT, ne - k0);
-      __syncthreads();
-      // column m of trans is contiguous in k: each thread copies whole runs
-      for (int t = tid; t < kn * ne; t += LKP_NT) {
-        const int m = t / kn, kk = t - m * kn;
-        tt[kk * ld + m] = tp[(size_t)m * ne + k0 + kk];
-      }
-      __syncthreads();
+    for (int m0 = wid * 32; m0 < ne; m0 += nt) {
+      const int mn = min(32, ne - m0);
+      float acc[8], next[32];
 #pragma unroll
-      for (int h = 0; h < 2; h++) {
-        const int m = tid + h * LKP_NT;
-        if (m >= ne) continue;
-        for (int kk = 0; kk < kn; kk++) {
-          const float w = tt[kk * ld + m];
+      for (int v = 0; v < 8; v++) acc[v] = 0.f;
+      // column m of trans is contiguous in k
+      auto load_tile = [&](int k0) {
+#pragma unroll
+        for (int i = 0; i < 32; i++)
+          next[i] = i < mn && k0 + lane < ne ? tp[(size_t)(m0 + i) * ne + k0 + lane] : 0.f;
+      };
+      load_tile(0);
+      for (int k0 = 0; k0 < ne; k0 += 32) {
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 32; i++) tt[lane * LKU_LD + i] = next[i];
+        __syncwarp();
+        if (k0 + 32 < ne) load_tile(k0 + 32);
+        const int kn = min(32, ne - k0);
+        int kk = 0;
+        for (; kk + 4 <= kn; kk += 4) {
+          float w[4];
+#pragma unroll
+          for (int j = 0; j < 4; j++) w[j] = tt[(kk + j) * LKU_LD + lane];
 #pragma unroll
           for (int v = 0; v < 8; v++)
-            if (v < nv) acc[v][h] = fmaf(xs[v * ne + k0 + kk], w, acc[v][h]);
+            if (v < nv) {
+              const float4 x = *reinterpret_cast<const float4*>(xs + v * xld + k0 + kk);
+              acc[v] = fmaf(x.w, w[3], fmaf(x.z, w[2], fmaf(x.y, w[1], fmaf(x.x, w[0], acc[v]))));
+            }
+        }
+        for (; kk < kn; kk++) {
+          const float w = tt[kk * LKU_LD + lane];
+#pragma unroll
+          for (int v = 0; v < 8; v++)
+            if (v < nv) acc[v] = fmaf(xs[v * xld + k0 + kk], w, acc[v]);
         }
       }
-    }
+      if (lane < mn) {
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
-      const int m = tid + h * LKP_NT;
-      if (m >= ne) continue;
-#pragma unroll
-      for (int v = 0; v < 8; v++)
-        if (v < nv) {
-          const size_t at = ((size_t)v * npts + p) * ne + m;
-          if (BF)
-            reinterpret_cast<__nv_bfloat16*>(xa_)[at] = __float2bfloat16_rn(acc[v][h]);
-          else
-            reinterpret_cast<float*>(xa_)[at] = (float)(base[v] + (double)acc[v][h]);
-        }
+        for (int v = 0; v < 8; v++)
+          if (v < nv) {
+            const size_t at = ((size_t)v * npts + p) * ne + m0 + lane;
+            if (BF)
+              reinterpret_cast<__nv_bfloat16*>(xa_)[at] = __float2bfloat16_rn(acc[v]);
+            else
+              reinterpret_cast<float*>(xa_)[at] = (float)(base[v] + (double)acc[v]);
+          }
+      }
     }
   }
 }
@@ -526,14 +555,15 @@ __global__ void __launch_bounds__(LKP_NT) lk_update_kernel(int ne, int npts, int
 template <bool BF>
 static int launch_lk_update(int ne, int npts, int nv, const void* xb, const float* xmean, const float* trans,
                             const float* transm, void* xa, float* amean, cudaStream_t stream) {
-  const size_t smem = sizeof(float) * (size_t)lku_base_floats(nv, ne) + sizeof(double) * 8;
+  const int nt = lku_threads(ne);
+  const size_t smem = sizeof(float) * ((size_t)nv * lku_xld(ne) + (size_t)nt * LKU_LD);
   cudaError_t e = cudaFuncSetAttribute(lk_update_kernel<BF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return cuda_status(e);
   int dev = 0, nsm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   const int grid = npts < nsm * 4 ? npts : nsm * 4;
-  lk_update_kernel<BF><<<grid, LKP_NT, smem, stream>>>(ne, npts, nv, xb, xmean, trans, transm, xa, amean);
+  lk_update_kernel<BF><<<grid, nt, smem, stream>>>(ne, npts, nv, xb, xmean, trans, transm, xa, amean);
   note_launch();
   return cuda_status(cudaGetLastError());
 }
@@ -558,7 +588,8 @@ static int lk_gemm(const LkGemmArgs& a, int nb, cudaStream_t s) {
   static_assert(LK_SMEM <= 227 * 1024, "shared memory");
   cudaError_t e = cudaFuncSetAttribute(largek_gemm_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, LK_SMEM);
   if (e != cudaSuccess) return cuda_status(e);
-  dim3 grid(a.kp / LK_TILE, a.kp / LK_TILE, nb * (MODE == LK_GRAM ? a.nsplit : 1));
+  const int nt = a.kp / LK_TILE;
+  const dim3 grid(nt, nt, nb * (MODE == LK_GRAM ? a.nsplit : 1));
   largek_gemm_kernel<MODE><<<grid, LK_NT, LK_SMEM, s>>>(a);
   note_launch();
   return cuda_status(cudaGetLastError());
@@ -690,7 +721,7 @@ static int largek_core(int ne, int npts, const int64_t* offs, const float* rows,
     g.nsplit = 1;
     // 2. prep
     lk_sums_kernel<<<dim3(LK_PIECES, nb), LKP_NT, 0, s>>>(ne, kp, offs + p0, rows, rows16, ridx, w, dep, rloc, pb, pp);
-    lk_prep_kernel<<<nb, LKP_NT, 0, s>>>(ne, kp, offs + p0, pb, pp, parm_infl + p0, minfl, G, Y, Z, bvec, inv_s, pt,
+    lk_prep_kernel<<<nb, LKQ_NT, 0, s>>>(ne, kp, offs + p0, pb, pp, parm_infl + p0, minfl, G, Y, Z, bvec, inv_s, pt,
                                          active);
     note_launch();
     note_launch();
@@ -772,8 +803,8 @@ static int largek_core(int ne, int npts, const int64_t* offs, const float* rows,
       g.out = Zn;
       st = lk_gemm<LK_AXPBY>(g, nb, s);
       if (st) break;
-      dim3 sg(64, nb);
-      lk_symmetrize_kernel<<<sg, 256, 0, s>>>(kp, Zn, Z, active);
+      dim3 sg(kp / 32, kp / 32, nb);
+      lk_symmetrize_kernel<<<sg, LKP_NT, 0, s>>>(kp, Zn, Z, active);
       note_launch();
     }
     // certificate of every transform against the exact A
@@ -782,8 +813,14 @@ static int largek_core(int ne, int npts, const int64_t* offs, const float* rows,
       note_launch();
     }
     // 5. transform, mean weights, inflation
-    lk_finalize_kernel<<<nb, LKP_NT, 0, s>>>(ne, kp, Z, bvec, pt, parm_infl + p0, trans + (size_t)p0 * ne * ne,
+    const dim3 fg((ne + LKF_NT - 1) / LKF_NT, nb);
+    float *gv = pb, *hv = pb + (size_t)kp * nb;  // the list sums are done with
+    lk_matvec_kernel<<<fg, LKF_NT, 0, s>>>(ne, kp, Z, bvec, pt, gv);
+    lk_matvec_kernel<<<fg, LKF_NT, 0, s>>>(ne, kp, Z, gv, pt, hv);
+    lk_finalize_kernel<<<fg, LKF_NT, 0, s>>>(ne, kp, Z, hv, pt, parm_infl + p0, trans + (size_t)p0 * ne * ne,
                                              transm ? transm + (size_t)p0 * ne : nullptr, status + p0);
+    note_launch();
+    note_launch();
     note_launch();
   }
   int h_err = 0;

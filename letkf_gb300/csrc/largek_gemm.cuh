@@ -5,10 +5,21 @@
 // memory and enter the tensor core as three-term TF32 splits
 // (x = hi + lo, hi = x with the low 13 mantissa bits cleared):
 //   acc = A_hi B_hi + A_hi B_lo + A_lo B_hi        (about 1e-6 relative)
-// staged K-major (SWIZZLE_NONE core matrices of 8 rows x 16 bytes) in two
-// 32 KB stages (K = 16) so the staging of stage c+1 overlaps the MMAs of
-// stage c; 64 KB per CTA lets three CTAs share an SM (384 TMEM columns), so
-// one CTA's MMAs also overlap another's global loads.
+// The tile is computed transposed, outᵀ = Yᵀ Xᵀ: the tensor core's A is Yᵀ,
+// whose rows the lanes read as whole lines of Y, and is staged in tensor memory
+// (a thread has one of its rows; 32 columns a K = 16 stage); its B is X, K-major
+// in shared memory (SWIZZLE_NONE core matrices of 8 rows x 16 bytes, 20 KB a
+// stage).  What bounded the kernel was shared-memory bandwidth: with both
+// operands there a stage wrote 32 KB and its six MMAs read 48 KB (data pipe 94 %
+// busy, tensor pipe 27 %), now 16 and 24, and a row per lane of X took a tag
+// lookup a lane.  Two stages share a barrier, two such pairs are in flight, and
+// two CTAs share an SM (256 TMEM columns each), so that one's MMAs overlap the
+// other's global loads.  The tile leaves through shared memory, a row per warp
+// request (a row per lane took 32 wavefronts a store).  k = 512, 256 points, one
+// product: 580 -> 327 us (tensor memory and tile alone 425); the products and
+// their order are the same, and so are the bits.  The Gram (lists of 464 rows a
+// point, BF16): 900 -> 470 us, its list entries a pair ahead of the rows and
+// nothing waiting on a row before its use.
 //
 // Modes:
 //   LK_GRAM   out = Ywᵀ Y over the point's local rows (K = its L, Yw = w_l y_l):
@@ -31,10 +42,18 @@ namespace letkf {
 constexpr int LK_NT = 256;
 constexpr int LK_TILE = 128;
 constexpr int LK_KC = 16;                // K per stage
-constexpr int LK_OPER = 8192;            // one 128 x 16 TF32 operand
-constexpr int LK_STAGE = 4 * LK_OPER;    // A_hi, A_lo, B_hi, B_lo
-constexpr int LK_SMEM = 2 * LK_STAGE + 64;
-constexpr uint32_t LK_TMEM_COLS = 128;
+// B's core matrices lie 32 bytes apart, so that a quarter warp's 16-byte stores
+// (two rows of four) fall into different banks
+constexpr int LK_LBO = 160, LK_SBO = 4 * LK_LBO;
+constexpr int LK_OPER = 16 * LK_SBO;     // one 128 x 16 TF32 operand
+constexpr int LK_STAGE = 2 * LK_OPER;    // B_hi, B_lo
+constexpr int LK_RING = 4;               // stages: two pairs
+constexpr int LK_OUT_LD = LK_TILE + 4;   // floats of a row of the output tile (conflict-free 16-byte columns)
+constexpr int LK_BUF = LK_RING * LK_STAGE;
+constexpr int LK_SMEM = LK_BUF + 64;
+static_assert(LK_BUF >= LK_TILE * LK_OUT_LD * 4, "the tile takes the stages' place");
+constexpr uint32_t LK_TMEM_COLS = 256;   // accumulator, then A's stages
+constexpr uint32_t LK_TMEM_A = 128;
 constexpr uint32_t LK_WAIT = 1u << 22;
 // The Gram's K is split over LK_SPLITS CTAs where the tiles alone are less than
 // two waves and the mean list is LK_SPLIT_L long: four points of k = 512 with
@@ -82,16 +101,16 @@ __device__ __forceinline__ void lk_store(unsigned char* hi_base, unsigned char* 
                                          const float (&v)[4]) {
   float4 h, l;
   lk_split4(v, h, l);
-  const uint32_t off = tc::kmajor_off(r, kk, LK_KC);
+  const uint32_t off = (uint32_t)((r >> 3) * LK_SBO + (kk >> 2) * LK_LBO + (r & 7) * 16);
   *reinterpret_cast<float4*>(hi_base + off) = h;
   *reinterpret_cast<float4*>(lo_base + off) = l;
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(LK_NT, 3) largek_gemm_kernel(LkGemmArgs a) {
+__global__ void __launch_bounds__(LK_NT, 2) largek_gemm_kernel(LkGemmArgs a) {
   extern __shared__ __align__(1024) unsigned char sm[];
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(sm + 2 * LK_STAGE);
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(sm + 2 * LK_STAGE + 16);
+  uint64_t* mbar = reinterpret_cast<uint64_t*>(sm + LK_BUF);
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(sm + LK_BUF + 16);
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int nsp = MODE == LK_GRAM ? a.nsplit : 1;
   const int b = blockIdx.z / nsp, sp = blockIdx.z - b * nsp;
@@ -144,75 +163,125 @@ __global__ void __launch_bounds__(LK_NT, 3) largek_gemm_kernel(LkGemmArgs a) {
   int tmo = 0;
   const int r = tid & 127, h = tid >> 7;  // staging: row r, K half h (8 values)
 
-  // stage values of this thread: rows r of A and B, K half h (8 values each);
-  // the next stage's loads are issued before this stage is split and stored,
-  // so their latency overlaps the staging, the barrier and the MMA issue
-  float va[8], vb[8];
-  auto load_stage = [&](int c, float (&xa)[8], float (&xb)[8]) {
-    const int k0 = (MODE == LK_GRAM ? kfirst + c : c) * LK_KC + h * 8;
+  // stage values of this thread, both stages of a pair; the next pair's loads
+  // are issued before this pair is split and stored.  A: row r, K half h.  B:
+  // in the Gram the same of the weighted rows; else four columns of rows tid / 4
+  // and 64 + tid / 4 (a quarter of the sectors' lines that a row per lane
+  // touches)
+  float va[2][8], vb[2][8];
+  // Gram: a lane has an entry of a pair's list rows, loaded a pair ahead of
+  // the rows themselves; the weight is applied, and what lies beyond L or ne cleared, where
+  // a value is used, so that nothing waits on its load before (those load a
+  // valid address: any row serves)
+  size_t er = 0;
+  float ew = 0.f, nw = 0.f;
+  const bool in_a = n0 + r < a.ne, in_b = m0 + r < a.ne;
+  const int ca_ = in_a ? n0 + r : 0, cb_ = in_b ? m0 + r : 0;
+  auto load_list = [&](int c) {
+    const int l = min((kfirst + c) * LK_KC + lane, L - 1);
+    er = a.ridx ? (size_t)a.ridx[r0 + l] : (size_t)(r0 + l);
+    ew = a.wts[r0 + l];
+  };
+  auto load_stage = [&](int c, int q, float (&xa)[8], float (&xb)[8]) {
     if (MODE == LK_GRAM) {
-      // A(m, l) = w_l y_l[m], B(n, l) = y_l[n]; rows beyond L or members beyond ne are 0
+      // A(n, l) = y_l[n], B(m, l) = w_l y_l[m]
+      size_t at[8];
 #pragma unroll
-      for (int j = 0; j < 8; j++) {
-        const int l = k0 + j;
-        float ya = 0.f, yb = 0.f;
-        if (l < L) {
-          const size_t ri = a.ridx ? (size_t)a.ridx[r0 + l] : (size_t)(r0 + l);
-          const float w = a.wts[r0 + l];
-          if (a.rows16) {
-            const __nv_bfloat16* row = a.rows16 + ri * a.ne;
-            if (m0 + r < a.ne) ya = w * __bfloat162float(row[m0 + r]);
-            if (n0 + r < a.ne) yb = __bfloat162float(row[n0 + r]);
-          } else {
-            const float* row = a.rows + ri * a.ne;
-            if (m0 + r < a.ne) ya = w * row[m0 + r];
-            if (n0 + r < a.ne) yb = row[n0 + r];
-          }
-        }
-        xa[j] = ya;
-        xb[j] = yb;
+      for (int j = 0; j < 8; j++) at[j] = (size_t)__shfl_sync(0xffffffffu, er, 16 * q + 8 * h + j) * a.ne;
+      if (a.rows16) {
+        const unsigned short* y16 = reinterpret_cast<const unsigned short*>(a.rows16);
+#pragma unroll
+        for (int j = 0; j < 8; j++) xa[j] = __uint_as_float((uint32_t)y16[at[j] + ca_]);
+#pragma unroll
+        for (int j = 0; j < 8; j++) xb[j] = __uint_as_float((uint32_t)y16[at[j] + cb_]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; j++) xa[j] = a.rows[at[j] + ca_];
+#pragma unroll
+        for (int j = 0; j < 8; j++) xb[j] = a.rows[at[j] + cb_];
       }
     } else {
-      const float4 x0 = *reinterpret_cast<const float4*>(a.X + mo + (size_t)(m0 + r) * kp + k0);
-      const float4 x1 = *reinterpret_cast<const float4*>(a.X + mo + (size_t)(m0 + r) * kp + k0 + 4);
-      xa[0] = x0.x;
-      xa[1] = x0.y;
-      xa[2] = x0.z;
-      xa[3] = x0.w;
-      xa[4] = x1.x;
-      xa[5] = x1.y;
-      xa[6] = x1.z;
-      xa[7] = x1.w;
 #pragma unroll
-      for (int j = 0; j < 8; j++) xb[j] = a.Y[mo + (size_t)(k0 + j) * kp + n0 + r];
+      for (int j = 0; j < 8; j++) xa[j] = a.Y[mo + (size_t)(c * LK_KC + h * 8 + j) * kp + n0 + r];
+#pragma unroll
+      for (int i = 0; i < 2; i++) {
+        const float4 x = *reinterpret_cast<const float4*>(a.X + mo + (size_t)(m0 + 64 * i + (tid >> 2)) * kp +
+                                                          c * LK_KC + 4 * (tid & 3));
+        xb[4 * i] = x.x;
+        xb[4 * i + 1] = x.y;
+        xb[4 * i + 2] = x.z;
+        xb[4 * i + 3] = x.w;
+      }
     }
   };
-  if (nk > 0) load_stage(0, va, vb);
-
-  for (int c = 0; c < nk; c++) {
-    const int buf = c & 1;
-    float ca[8], cb[8];
+  if (MODE == LK_GRAM && nk > 0) load_list(0);
 #pragma unroll
-    for (int j = 0; j < 8; j++) {
-      ca[j] = va[j];
-      cb[j] = vb[j];
+  for (int q = 0; q < 2; q++)
+    if (q < nk) load_stage(q, q, va[q], vb[q]);
+  if (MODE == LK_GRAM && nk > 0) {
+    nw = ew;
+    load_list(2);
+  }
+
+  const uint32_t alane = (uint32_t)(32 * (wid & 3)) << 16;  // a warp's TMEM lanes
+  for (int c = 0; c < nk; c += 2) {
+    const int buf = (c >> 1) & 1, ns = min(2, nk - c);
+    float ca[2][8], cb[2][8];
+#pragma unroll
+    for (int q = 0; q < 2; q++)
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        ca[q][j] = va[q][j];
+        cb[q][j] = vb[q][j];
+      }
+    const float cw = nw;
+#pragma unroll
+    for (int q = 0; q < 2; q++)
+      if (c + 2 + q < nk) load_stage(c + 2 + q, q, va[q], vb[q]);
+    if (MODE == LK_GRAM) {
+      nw = ew;
+      load_list(c + 4);
     }
-    if (c + 1 < nk) load_stage(c + 1, va, vb);
     if ((outst >> buf) & 1u) {
       if (!tc::mbar_wait(&mbar[buf], (par >> buf) & 1u, LK_WAIT)) tmo = 1;
       par ^= 1u << buf;
       outst &= ~(1u << buf);
     }
     tc::fence_after_sync();
-    unsigned char* st = sm + buf * LK_STAGE;
 #pragma unroll
-    for (int g = 0; g < 2; g++) {
-      const int kk = h * 8 + g * 4;
-      const float qa[4] = {ca[4 * g], ca[4 * g + 1], ca[4 * g + 2], ca[4 * g + 3]};
-      const float qb[4] = {cb[4 * g], cb[4 * g + 1], cb[4 * g + 2], cb[4 * g + 3]};
-      lk_store(st, st + LK_OPER, r, kk, qa);
-      lk_store(st + 2 * LK_OPER, st + 3 * LK_OPER, r, kk, qb);
+    for (int q = 0; q < 2; q++) {
+      if (q >= ns) break;
+      const int slot = 2 * buf + q;
+      unsigned char* st = sm + slot * LK_STAGE;
+      if (MODE == LK_GRAM) {
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+          const float w = __shfl_sync(0xffffffffu, cw, 16 * q + 8 * h + j);
+          const bool in_l = (kfirst + c + q) * LK_KC + 8 * h + j < L;
+          if (a.rows16) {
+            ca[q][j] = __uint_as_float(__float_as_uint(ca[q][j]) << 16);
+            cb[q][j] = __uint_as_float(__float_as_uint(cb[q][j]) << 16);
+          }
+          ca[q][j] = in_l && in_a ? ca[q][j] : 0.f;
+          cb[q][j] = in_l && in_b ? __fmul_rn(w, cb[q][j]) : 0.f;
+        }
+      }
+      float hi[8], lo[8];
+#pragma unroll
+      for (int j = 0; j < 8; j++) tc::split_tf32(ca[q][j], hi[j], lo[j]);
+      const uint32_t at = tacc + alane + LK_TMEM_A + 32 * slot + 8 * h;
+      tc::tmem_st8(at, hi);
+      tc::tmem_st8(at + 16, lo);
+#pragma unroll
+      for (int g = 0; g < 2; g++) {
+        const float qb[4] = {cb[q][4 * g], cb[q][4 * g + 1], cb[q][4 * g + 2], cb[q][4 * g + 3]};
+        if (MODE == LK_GRAM)
+          lk_store(st, st + LK_OPER, r, h * 8 + g * 4, qb);
+        else
+          lk_store(st, st + LK_OPER, 64 * g + (tid >> 2), 4 * (tid & 3), qb);
+      }
     }
+    tc::tmem_wait_st();
     tc::fence_smem_async();
     tc::fence_before_sync();
     if (__syncthreads_or(tmo)) {  // a bounded wait gave up: issue nothing more
@@ -221,15 +290,20 @@ __global__ void __launch_bounds__(LK_NT, 3) largek_gemm_kernel(LkGemmArgs a) {
     }
     if (tid == 0) {
       tc::fence_after_sync();
-      const uint32_t s0 = sbase + buf * LK_STAGE;
 #pragma unroll
-      for (int pass = 0; pass < 3; pass++) {
-        const uint32_t sa = s0 + (pass == 2 ? LK_OPER : 0);
-        const uint32_t sb = s0 + 2 * LK_OPER + (pass == 1 ? LK_OPER : 0);
+      for (int q = 0; q < 2; q++) {
+        if (q >= ns) break;
+        const int slot = 2 * buf + q;
+        const uint32_t s0 = sbase + slot * LK_STAGE, a0 = tacc + LK_TMEM_A + 32 * slot;
 #pragma unroll
-        for (int s = 0; s < LK_KC / 8; s++)
-          tc::mma_tf32(tacc, tc::smem_desc(sa + s * 256, 128, LK_KC * 32), tc::smem_desc(sb + s * 256, 128, LK_KC * 32),
-                       idesc, (c == 0 && pass == 0 && s == 0) ? 0u : 1u);
+        for (int pass = 0; pass < 3; pass++) {
+          const uint32_t sa = a0 + (pass == 1 ? 16 : 0);
+          const uint32_t sb = s0 + (pass == 2 ? LK_OPER : 0);
+#pragma unroll
+          for (int s = 0; s < LK_KC / 8; s++)
+            tc::mma_tf32_ts(tacc, sa + 8 * s, tc::smem_desc(sb + s * 2 * LK_LBO, LK_LBO, LK_SBO), idesc,
+                            (c == 0 && q == 0 && pass == 0 && s == 0) ? 0u : 1u);
+        }
       }
       tc::mma_commit(&mbar[buf]);
     }
@@ -246,51 +320,52 @@ __global__ void __launch_bounds__(LK_NT, 3) largek_gemm_kernel(LkGemmArgs a) {
   if (bad) {
     if (tid == 0 && a.err_flag) atomicExch(a.err_flag, 1);
   } else {
-    // epilogue: warp w reads TMEM lanes 32 (w % 4) .. +31 (rows), columns 64 (w / 4) .. +63
-    const int row = 32 * (wid & 3) + lane;
-    const int cb = 64 * (wid >> 2);
-    const uint32_t taddr = tacc + ((uint32_t)(32 * (wid & 3)) << 16) + (uint32_t)cb;
-    float e2 = 0.f;
-    const size_t orow = mo + (size_t)(m0 + row) * kp + n0 + cb;
+    // epilogue: warp w reads TMEM lanes 32 (w % 4) .. +31 (the tile's columns),
+    // TMEM columns 64 (w / 4) .. +63 (its rows); then a row per warp request
+    float* tile = reinterpret_cast<float*>(sm);
+    {
+      const int tcol = 32 * (wid & 3) + lane, rb = 64 * (wid >> 2);
+      const uint32_t taddr = tacc + alane + (uint32_t)rb;
 #pragma unroll 1
-    for (int c0 = 0; c0 < 64; c0 += 16) {
-      float v[16];
-      if (nk > 0) {
-        tc::tmem_ld16(taddr + c0, v);
-      } else {
-#pragma unroll
-        for (int j = 0; j < 16; j++) v[j] = 0.f;
-      }
-      float* dst = (MODE == LK_GRAM && nsp > 1 ? a.outs[sp] : a.out) + orow + c0;
-      if (MODE == LK_AXPBY) {
-        const float al = a.alpha_b ? a.alpha_b[b] : a.alpha;
-        const float be = a.beta_b ? a.beta_b[b] : a.beta;
-        if (a.D) {
-          const float* dd = a.D + orow + c0;
-#pragma unroll
-          for (int j = 0; j < 16; j += 4) {
-            const float4 d4 = *reinterpret_cast<const float4*>(dd + j);
-            *reinterpret_cast<float4*>(dst + j) =
-                make_float4(al * v[j] + be * d4.x, al * v[j + 1] + be * d4.y, al * v[j + 2] + be * d4.z,
-                            al * v[j + 3] + be * d4.w);
-          }
+      for (int c0 = 0; c0 < 64; c0 += 16) {
+        float v[16];
+        if (nk > 0) {
+          tc::tmem_ld16(taddr + c0, v);
         } else {
 #pragma unroll
-          for (int j = 0; j < 16; j += 4)
-            *reinterpret_cast<float4*>(dst + j) = make_float4(al * v[j], al * v[j + 1], al * v[j + 2], al * v[j + 3]);
-        }
-      } else {
-        if (MODE == LK_T) {
-#pragma unroll
-          for (int j = 0; j < 16; j++) {
-            const float dl = v[j] - ((m0 + row == n0 + cb + c0 + j) ? 1.f : 0.f);
-            e2 = fmaf(dl, dl, e2);
-          }
+          for (int j = 0; j < 16; j++) v[j] = 0.f;
         }
 #pragma unroll
-        for (int j = 0; j < 16; j += 4)
-          *reinterpret_cast<float4*>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+        for (int j = 0; j < 16; j++) tile[(rb + c0 + j) * LK_OUT_LD + tcol] = v[j];
       }
+    }
+    __syncthreads();
+    const float al = MODE == LK_AXPBY ? (a.alpha_b ? a.alpha_b[b] : a.alpha) : 1.f;
+    const float be = MODE == LK_AXPBY ? (a.beta_b ? a.beta_b[b] : a.beta) : 0.f;
+    float* out = MODE == LK_GRAM && nsp > 1 ? a.outs[sp] : a.out;
+    float e2 = 0.f;
+#pragma unroll 4
+    for (int row = wid; row < LK_TILE; row += LK_NT / 32) {
+      const int col = 4 * lane;
+      const size_t at = mo + (size_t)(m0 + row) * kp + n0 + col;
+      float4 v = *reinterpret_cast<const float4*>(tile + row * LK_OUT_LD + col);
+      if (MODE == LK_AXPBY) {
+        if (a.D) {
+          const float4 d = *reinterpret_cast<const float4*>(a.D + at);
+          // one rounding for the product by alpha, as the compiler had it: bits matter to the iteration's fixed point
+          v = make_float4(fmaf(be, d.x, __fmul_rn(al, v.x)), fmaf(be, d.y, __fmul_rn(al, v.y)),
+                          fmaf(be, d.z, __fmul_rn(al, v.z)), fmaf(be, d.w, __fmul_rn(al, v.w)));
+        } else {
+          v = make_float4(al * v.x, al * v.y, al * v.z, al * v.w);
+        }
+      }
+      if (MODE == LK_T) {
+        const int dg = m0 + row - n0 - col;  // the diagonal's place in v
+        const float d0 = v.x - (dg == 0 ? 1.f : 0.f), d1 = v.y - (dg == 1 ? 1.f : 0.f);
+        const float d2 = v.z - (dg == 2 ? 1.f : 0.f), d3 = v.w - (dg == 3 ? 1.f : 0.f);
+        e2 = fmaf(d0, d0, fmaf(d1, d1, fmaf(d2, d2, fmaf(d3, d3, e2))));
+      }
+      *reinterpret_cast<float4*>(out + at) = v;
     }
     if (MODE == LK_T) {
       e2 = warp_sum(e2);
