@@ -67,6 +67,7 @@ struct TcLayout {
   static constexpr int PCAP = TC_CH + TC_CPT * TC_NT;  // pending-list entries
   static constexpr int PIDX = RED + 256;         // int[PCAP]
   static constexpr int PW = PIDX + 4 * PCAP;
+  static_assert(PIDX % 16 == 0 && PCAP % 4 == 0 && TC_CH % 8 == 0, "16-byte loads of the pending list");
   static constexpr int PD = PW + 4 * PCAP;
   static constexpr int PR = PD + 4 * PCAP;
   static constexpr int ROWIB = PR + 4 * PCAP;
@@ -87,10 +88,11 @@ __device__ __forceinline__ float col_dot64(const float* M, const float* x, int c
   float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
 #pragma unroll 4
   for (int j = 0; j < 64; j += 4) {
-    a0 = fmaf(M[j * 64 + c], x[j], a0);
-    a1 = fmaf(M[(j + 1) * 64 + c], x[j + 1], a1);
-    a2 = fmaf(M[(j + 2) * 64 + c], x[j + 2], a2);
-    a3 = fmaf(M[(j + 3) * 64 + c], x[j + 3], a3);
+    const float4 xj = *reinterpret_cast<const float4*>(x + j);
+    a0 = fmaf(M[j * 64 + c], xj.x, a0);
+    a1 = fmaf(M[(j + 1) * 64 + c], xj.y, a1);
+    a2 = fmaf(M[(j + 2) * 64 + c], xj.z, a2);
+    a3 = fmaf(M[(j + 3) * 64 + c], xj.w, a3);
   }
   return (a0 + a1) + (a2 + a3);
 }
@@ -255,19 +257,30 @@ __global__ void __launch_bounds__(TC_NT, 4) sweep_tc_kernel(SweepArgs a) {
       tc::fence_after_sync();
       unsigned char* stg = sm + L::STG + buf * L::STG_SIZE;
       constexpr int KH = TC_CH / 2;  // observations per thread: member m, half hh
-      float yv[KH], wv[KH];
+      float yv[KH], wv[KH], dv[KH];
+      // four entries of the pending list per shared-memory load; what lies
+      // beyond nr is old and not used
+#pragma unroll
+      for (int g = 0; g < KH / 4; g++) {
+        const int kb = hh * KH + 4 * g;
+        const int4 i4 = *reinterpret_cast<const int4*>(ss.pidx + kb);
+        const float4 w4 = *reinterpret_cast<const float4*>(ss.pw + kb);
+        const float4 d4 = *reinterpret_cast<const float4*>(ss.pd + kb);
+        const int ix[4] = {i4.x, i4.y, i4.z, i4.w};
+        const float wx[4] = {w4.x, w4.y, w4.z, w4.w}, dx[4] = {d4.x, d4.y, d4.z, d4.w};
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          float y = 0.f;
+          if (kb + j < nr && m < n) y = a.ens_obs[(size_t)ix[j] * n + m];
+          yv[4 * g + j] = y;
+          wv[4 * g + j] = kb + j < nr ? wx[j] : 0.f;
+          dv[4 * g + j] = kb + j < nr ? dx[j] : 0.f;
+        }
+      }
 #pragma unroll
       for (int kk = 0; kk < KH; kk++) {
-        const int k = hh * KH + kk;
-        float y = 0.f, w = 0.f, dd = 0.f;
-        if (k < nr) {
-          w = ss.pw[k];
-          dd = ss.pd[k];
-          if (m < n) y = a.ens_obs[(size_t)ss.pidx[k] * n + m];
-        }
-        yv[kk] = y;
-        wv[kk] = y * w;
-        bpart = fmaf(wv[kk], dd, bpart);
+        wv[kk] = yv[kk] * wv[kk];
+        bpart = fmaf(wv[kk], dv[kk], bpart);
       }
 #pragma unroll
       for (int g = 0; g < KH / 4; g++) {
@@ -797,16 +810,21 @@ __global__ void __launch_bounds__(TC_NT, 4) sweep_tc_kernel(SweepArgs a) {
           float* Af = reinterpret_cast<float*>(sm + L::YF);  // A / s
           float* Pf = reinterpret_cast<float*>(sm + L::ZF);  // A Z, then Q; the probe vectors
           if (r >= 64) {
+            // lanes start at different column groups, and the upper four groups
+            // store their halves in the other order: the eight rows of a quarter
+            // warp's store lie in distinct banks (all in one otherwise)
             float* dst = Zf + (r - 64) * 64;
   #pragma unroll 1
-            for (int c0 = 0; c0 < 64; c0 += 8) {
+            for (int i = 0; i < 8; i++) {
+              const int c0 = 8 * ((i + r) & 7), sw = (c0 >> 5) << 2;
               const uint32_t off = tc::kmajor_off_bf16(r, c0, 64);
               float sh[8], sl[8];
               unpack8(*reinterpret_cast<const uint4*>(sm + L::S_HI + off), sh);
               unpack8(*reinterpret_cast<const uint4*>(sm + L::S_LO + off), sl);
-              *reinterpret_cast<float4*>(dst + c0) = make_float4(sh[0] + sl[0], sh[1] + sl[1], sh[2] + sl[2], sh[3] + sl[3]);
-              *reinterpret_cast<float4*>(dst + c0 + 4) =
-                  make_float4(sh[4] + sl[4], sh[5] + sl[5], sh[6] + sl[6], sh[7] + sl[7]);
+              const float4 z0 = make_float4(sh[0] + sl[0], sh[1] + sl[1], sh[2] + sl[2], sh[3] + sl[3]);
+              const float4 z1 = make_float4(sh[4] + sl[4], sh[5] + sl[5], sh[6] + sl[6], sh[7] + sl[7]);
+              *reinterpret_cast<float4*>(dst + c0 + sw) = sw ? z1 : z0;
+              *reinterpret_cast<float4*>(dst + c0 + 4 - sw) = sw ? z0 : z1;
             }
           }
           __syncthreads();
@@ -816,7 +834,7 @@ __global__ void __launch_bounds__(TC_NT, 4) sweep_tc_kernel(SweepArgs a) {
               float v[16];
               tc::tmem_ld16(D1 + lane_off + c0, v);
   #pragma unroll
-              for (int j = 0; j < 16; j++) Af[r * 64 + c0 + j] = v[j] * inv_s;
+              for (int j = 0; j < 16; j++) Af[(c0 + j) * 64 + r] = v[j] * inv_s;  // symmetric to the bit
             }
           }
           tc::fence_before_sync();
@@ -946,8 +964,19 @@ __global__ void __launch_bounds__(TC_NT, 4) sweep_tc_kernel(SweepArgs a) {
       const int mm = tid & 63, vg = tid >> 6;
       if (mm < n) {
         float acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 2
-        for (int k = 0; k < n; k++) {
+        int k = 0;
+        for (; k + 4 <= n; k += 4) {
+          float w[4];
+#pragma unroll
+          for (int i = 0; i < 4; i++) w[i] = Wm[(k + i) * 64 + mm];
+#pragma unroll
+          for (int j = 0; j < 4; j++)
+            if (vg + 2 * j < nv) {
+              const float4 x = *reinterpret_cast<const float4*>(xs + (vg + 2 * j) * 64 + k);
+              acc[j] = fmaf(x.w, w[3], fmaf(x.z, w[2], fmaf(x.y, w[1], fmaf(x.x, w[0], acc[j]))));
+            }
+        }
+        for (; k < n; k++) {
           const float w = Wm[k * 64 + mm];
 #pragma unroll
           for (int j = 0; j < 4; j++)

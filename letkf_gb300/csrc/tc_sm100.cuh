@@ -223,14 +223,16 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) {
 
 // 8 values -> hi and lo bf16 packs (16 bytes each)
 __device__ __forceinline__ void split8(const float* v, uint4& hi, uint4& lo) {
-  float h[8], l[8];
+  // a pair at a time: one conversion gives both high halves and their pack
+  uint32_t h[4], l[4];
 #pragma unroll
-  for (int j = 0; j < 8; j++) {
-    h[j] = __bfloat162float(__float2bfloat16_rn(v[j]));
-    l[j] = v[j] - h[j];
+  for (int j = 0; j < 4; j++) {
+    h[j] = pack_bf16x2(v[2 * j], v[2 * j + 1]);
+    l[j] = pack_bf16x2(v[2 * j] - __uint_as_float(h[j] << 16),
+                       v[2 * j + 1] - __uint_as_float(h[j] & 0xFFFF0000u));
   }
-  hi = make_uint4(pack_bf16x2(h[0], h[1]), pack_bf16x2(h[2], h[3]), pack_bf16x2(h[4], h[5]), pack_bf16x2(h[6], h[7]));
-  lo = make_uint4(pack_bf16x2(l[0], l[1]), pack_bf16x2(l[2], l[3]), pack_bf16x2(l[4], l[5]), pack_bf16x2(l[6], l[7]));
+  hi = make_uint4(h[0], h[1], h[2], h[3]);
+  lo = make_uint4(l[0], l[1], l[2], l[3]);
 }
 
 // 4 values -> tf32 hi (low 13 mantissa bits cleared) and the FP32 remainder
