@@ -6,7 +6,7 @@
 // ambiguous band |ndist - cutoff| < 1e-3 cutoff is re-tested with the
 // reference's FP64 formula.  Accepted observations are compacted, in the
 // reference order, into a pending list (index, weight rloc/err^2, departure,
-// rloc); `flush(nr)` consumes the first nr entries whenever CH are pending and
+// rloc); `flush(nr, o)` consumes entries o .. o+nr-1 whenever CH are pending and
 // once more for the remainder.  Returns the number of accepted observations.
 // With probe >= 0 the accepted entries are also written, in emitted order, to
 // the selection probe of SweepArgs (slot `probe`).
@@ -95,12 +95,13 @@ struct SwCache {
 
 // Compaction of one batch of CPT*NT evaluated candidates: accepted ones go to
 // the pending list (and the probe) in candidate order, survivors to the
-// column cache; flush(CH) consumes the pending list in stages of CH.
+// column cache; flush(CH, off) consumes the pending list in stages of CH.
 template <int NT, int CH, int CPT, typename Flush>
 __device__ __forceinline__ void sw_compact(const SweepArgs& a, const SearchSmem& s, int probe, const SwCand (&cg)[CPT],
                                            int& pend, int& L, const SwCache& cache, int& nsurv, Flush& flush) {
   const bool BUILD = cache.ent != nullptr;  // uniform
   constexpr int NW = NT / 32;
+  static_assert(CH <= NT, "one pass moves the tail");
   constexpr int SV = CPT * NW + 1;  // survivors' counts follow the accepted ones
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const unsigned below = (1u << lane) - 1u;
@@ -163,35 +164,21 @@ __device__ __forceinline__ void sw_compact(const SweepArgs& a, const SearchSmem&
   L += s.wcnt[CPT * NW];
   if (BUILD) nsurv += s.wcnt[SV + CPT * NW];
   __syncthreads();
-  while (pend >= CH) {
-    flush(CH);
-    __syncthreads();
-    // move the tail (fewer than CPT*NT entries) to the front
-    const int rest = pend - CH;
-    int i0[CPT];
-    float w0[CPT], d0[CPT], r0[CPT];
-#pragma unroll
-    for (int g = 0; g < CPT; g++) {
-      const int t = g * NT + tid;
-      if (t < rest) {
-        i0[g] = s.pidx[CH + t];
-        w0[g] = s.pw[CH + t];
-        d0[g] = s.pd[CH + t];
-        r0[g] = s.pr[CH + t];
-      }
+  // stages straight from the list: flush(CH, off) has a barrier after its reads,
+  // and the tail moves once, after the last stage (it is shorter than CH, so
+  // what it reads and writes do not overlap).  Moving it after every stage took
+  // three barriers a stage more.
+  int off = 0;
+  for (; pend - off >= CH; off += CH) flush(CH, off);
+  if (off > 0) {
+    const int t = tid;
+    pend -= off;
+    if (t < pend) {
+      s.pidx[t] = s.pidx[off + t];
+      s.pw[t] = s.pw[off + t];
+      s.pd[t] = s.pd[off + t];
+      s.pr[t] = s.pr[off + t];
     }
-    __syncthreads();
-#pragma unroll
-    for (int g = 0; g < CPT; g++) {
-      const int t = g * NT + tid;
-      if (t < rest) {
-        s.pidx[t] = i0[g];
-        s.pw[t] = w0[g];
-        s.pd[t] = d0[g];
-        s.pr[t] = r0[g];
-      }
-    }
-    pend = rest;
     __syncthreads();
   }
 }
@@ -297,7 +284,7 @@ __device__ int sweep_search(const SweepArgs& a, double ri, double rj, double log
     }
   }
   if (pend > 0) {
-    flush(pend);
+    flush(pend, 0);
     __syncthreads();
   }
   if (probe >= 0 && threadIdx.x == 0) a.probe_count[probe] = L;
@@ -349,7 +336,7 @@ __device__ int sweep_search_cached(const SweepArgs& a, const int4* __restrict__ 
     e1 = f1;
   }
   if (pend > 0) {
-    flush(pend);
+    flush(pend, 0);
     __syncthreads();
   }
   if (probe >= 0 && threadIdx.x == 0) a.probe_count[probe] = L;
@@ -377,7 +364,7 @@ __device__ int sweep_list(const SweepArgs& a, int q, const SearchSmem& s, Flush&
       s.pd[t] = q4.z;
     }
     __syncthreads();
-    flush(nr);
+    flush(nr, 0);
     __syncthreads();
   }
   return (int)(o1 - o0);

@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(TC_NT, 4) sweep_tc_kernel(SweepArgs a) {
     float bpart = 0.f, p1 = 0.f, p3 = 0.f;
     int chunk = 0;
     bool first = true;
-    auto flush = [&](int nr) {
+    auto flush = [&](int nr, int o) {  // entries o .. o + nr - 1 of the pending list
       const int buf = chunk & 1;
       if ((outst >> buf) & 1u) {
         wait_bar(buf);
@@ -262,10 +262,10 @@ __global__ void __launch_bounds__(TC_NT, 4) sweep_tc_kernel(SweepArgs a) {
       // beyond nr is old and not used
 #pragma unroll
       for (int g = 0; g < KH / 4; g++) {
-        const int kb = hh * KH + 4 * g;
-        const int4 i4 = *reinterpret_cast<const int4*>(ss.pidx + kb);
-        const float4 w4 = *reinterpret_cast<const float4*>(ss.pw + kb);
-        const float4 d4 = *reinterpret_cast<const float4*>(ss.pd + kb);
+        const int kb = hh * KH + 4 * g;  // of the stage
+        const int4 i4 = *reinterpret_cast<const int4*>(ss.pidx + o + kb);
+        const float4 w4 = *reinterpret_cast<const float4*>(ss.pw + o + kb);
+        const float4 d4 = *reinterpret_cast<const float4*>(ss.pd + o + kb);
         const int ix[4] = {i4.x, i4.y, i4.z, i4.w};
         const float wx[4] = {w4.x, w4.y, w4.z, w4.w}, dx[4] = {d4.x, d4.y, d4.z, d4.w};
 #pragma unroll
@@ -294,9 +294,9 @@ __global__ void __launch_bounds__(TC_NT, 4) sweep_tc_kernel(SweepArgs a) {
         *reinterpret_cast<float4*>(stg + L::STG_BL + off) = l;
       }
       for (int k = tid; k < nr; k += TC_NT) {
-        const float dd = ss.pd[k];
-        p1 = fmaf(dd * dd, ss.pw[k], p1);
-        p3 += ss.pr[k];
+        const float dd = ss.pd[o + k];
+        p1 = fmaf(dd * dd, ss.pw[o + k], p1);
+        p3 += ss.pr[o + k];
       }
       tc::fence_smem_async();
       tc::fence_before_sync();
@@ -450,44 +450,38 @@ __global__ void __launch_bounds__(TC_NT, 4) sweep_tc_kernel(SweepArgs a) {
         }
         tc::fence_before_sync();
         // scaling s: power iteration guarded by the Gershgorin bound (s >= lambda_max / 2)
-        float gsum = 0.f;
+        // and ||A||_F from the same reads of the columns
+        float gsum = 0.f, f2 = 0.f;
         if (tid < 64) {
-          float g0 = 0.f, g1 = 0.f, g2 = 0.f, g3 = 0.f;
+          float g0 = 0.f, g1 = 0.f, g2 = 0.f, g3 = 0.f, q0 = 0.f, q1 = 0.f, q2 = 0.f, q3 = 0.f;
 #pragma unroll 4
           for (int j = 0; j < 64; j += 4) {
-            g0 += fabsf(Gt[gsw(j, tid)]);
-            g1 += fabsf(Gt[gsw(j + 1, tid)]);
-            g2 += fabsf(Gt[gsw(j + 2, tid)]);
-            g3 += fabsf(Gt[gsw(j + 3, tid)]);
+            const float x0 = Gt[gsw(j, tid)], x1 = Gt[gsw(j + 1, tid)];
+            const float x2 = Gt[gsw(j + 2, tid)], x3 = Gt[gsw(j + 3, tid)];
+            g0 += fabsf(x0);
+            g1 += fabsf(x1);
+            g2 += fabsf(x2);
+            g3 += fabsf(x3);
+            q0 = fmaf(x0, x0, q0);
+            q1 = fmaf(x1, x1, q1);
+            q2 = fmaf(x2, x2, q2);
+            q3 = fmaf(x3, x3, q3);
           }
           gsum = (g0 + g1) + (g2 + g3);
+          f2 = (q0 + q1) + (q2 + q3);
           vx[tid] = Gt[gsw(tid, tid)] * (1.f + 0.25f * __sinf(1.7f * tid));
         }
         gsum = warp_max(gsum);
-        __syncthreads();
-        if (lane == 0) red[wid] = gsum;
+        f2 = warp_sum(f2);
+        if (lane == 0) {
+          red[wid] = gsum;
+          red[4 + wid] = f2;
+        }
         __syncthreads();
         const float gmax = fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3]));
-        __syncthreads();
-        float lam = 0.f, fro = 0.f;
-        if (a.tc_scale_bound) {
-          // s = min(||A||_F, Gershgorin) >= lambda_max: every eigenvalue of A/s is <= 1
-          float f2 = 0.f;
-          if (tid < 64) {
-            float q0 = 0.f, q1 = 0.f, q2 = 0.f, q3 = 0.f;
-#pragma unroll 4
-            for (int j = 0; j < 64; j += 4) {
-              const float x0 = Gt[gsw(j, tid)], x1 = Gt[gsw(j + 1, tid)];
-              const float x2 = Gt[gsw(j + 2, tid)], x3 = Gt[gsw(j + 3, tid)];
-              q0 = fmaf(x0, x0, q0);
-              q1 = fmaf(x1, x1, q1);
-              q2 = fmaf(x2, x2, q2);
-              q3 = fmaf(x3, x3, q3);
-            }
-            f2 = (q0 + q1) + (q2 + q3);
-          }
-          fro = sqrtf(block_sum<float, TC_NT>(f2, red));
-        }
+        // with tc_scale_bound s = min(||A||_F, Gershgorin) >= lambda_max: every eigenvalue of A/s is <= 1
+        const float fro = sqrtf(red[4] + red[5]);
+        float lam = 0.f;
         for (int it = 0; it < (a.tc_scale_bound ? 0 : 8); it++) {
           float part = 0.f, xx = 0.f;
           if (tid < 64) {
@@ -868,7 +862,10 @@ __global__ void __launch_bounds__(TC_NT, 4) sweep_tc_kernel(SweepArgs a) {
           }
           if (polish)
             it += ns_polish<TC_NP>(Af, Zf, Pf, red, tc_max > 0 ? TC_POLISH_MAX : a.max_ns_iter, a.polish_tol, &ok);
-          for (int idx = tid; idx < 64 * 64; idx += TC_NT) Wm[idx] = coef * Zf[idx];
+          for (int idx = tid; idx < 64 * 64 / 4; idx += TC_NT) {
+            const float4 z = reinterpret_cast<const float4*>(Zf)[idx];
+            reinterpret_cast<float4*>(Wm)[idx] = make_float4(coef * z.x, coef * z.y, coef * z.z, coef * z.w);
+          }
           __syncthreads();
         }
         }  // ok: Newton-Schulz attempted

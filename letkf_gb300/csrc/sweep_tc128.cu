@@ -61,6 +61,7 @@ struct T8Layout {
   static constexpr int PCAP = T8_CH + T8_NT;          // pending-list entries
   static constexpr int PIDX = RED + 256;              // int[PCAP]
   static constexpr int PW = PIDX + 4 * PCAP;
+  static_assert(PIDX % 16 == 0 && PCAP % 4 == 0 && T8_CH % 8 == 0, "16-byte loads of the pending list");
   static constexpr int PD = PW + 4 * PCAP;
   static constexpr int PR = PD + 4 * PCAP;
   static constexpr int ROWIB = PR + 4 * PCAP;
@@ -84,10 +85,11 @@ __device__ __forceinline__ float col_dot128(const float* M, const float* x, int 
   float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
 #pragma unroll 4
   for (int j = 0; j < 128; j += 4) {
-    a0 = fmaf(M[j * 128 + c], x[j], a0);
-    a1 = fmaf(M[(j + 1) * 128 + c], x[j + 1], a1);
-    a2 = fmaf(M[(j + 2) * 128 + c], x[j + 2], a2);
-    a3 = fmaf(M[(j + 3) * 128 + c], x[j + 3], a3);
+    const float4 xj = *reinterpret_cast<const float4*>(x + j);
+    a0 = fmaf(M[j * 128 + c], xj.x, a0);
+    a1 = fmaf(M[(j + 1) * 128 + c], xj.y, a1);
+    a2 = fmaf(M[(j + 2) * 128 + c], xj.z, a2);
+    a3 = fmaf(M[(j + 3) * 128 + c], xj.w, a3);
   }
   return (a0 + a1) + (a2 + a3);
 }
@@ -205,7 +207,7 @@ __global__ void __launch_bounds__(T8_NT, 1) sweep_tc128_kernel(SweepArgs a) {
     float bpart = 0.f, p1 = 0.f, p3 = 0.f;
     int chunk = 0;
     bool first = true;
-    auto flush = [&](int nr) {
+    auto flush = [&](int nr, int o) {  // entries o .. o + nr - 1 of the pending list
       const int buf = chunk & 1;
       if ((outst >> buf) & 1u) {
         wait_bar(buf);
@@ -214,19 +216,30 @@ __global__ void __launch_bounds__(T8_NT, 1) sweep_tc128_kernel(SweepArgs a) {
       tc::fence_after_sync();
       unsigned char* stg = sm + L::STG + buf * L::STG_SIZE;
       constexpr int KH = T8_CH / 2;  // observations per thread: member m, half hh
-      float yv[KH], wv[KH];
+      float yv[KH], wv[KH], dv[KH];
+      // four entries of the pending list per shared-memory load; what lies
+      // beyond nr is old and not used
+#pragma unroll
+      for (int g = 0; g < KH / 4; g++) {
+        const int kb = hh * KH + 4 * g;  // of the stage  // of the stage
+        const int4 i4 = *reinterpret_cast<const int4*>(ss.pidx + o + kb);
+        const float4 w4 = *reinterpret_cast<const float4*>(ss.pw + o + kb);
+        const float4 d4 = *reinterpret_cast<const float4*>(ss.pd + o + kb);
+        const int ix[4] = {i4.x, i4.y, i4.z, i4.w};
+        const float wx[4] = {w4.x, w4.y, w4.z, w4.w}, dx[4] = {d4.x, d4.y, d4.z, d4.w};
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          float y = 0.f;
+          if (kb + j < nr && m < n) y = a.ens_obs[(size_t)ix[j] * n + m];
+          yv[4 * g + j] = y;
+          wv[4 * g + j] = kb + j < nr ? wx[j] : 0.f;
+          dv[4 * g + j] = kb + j < nr ? dx[j] : 0.f;
+        }
+      }
 #pragma unroll
       for (int kk = 0; kk < KH; kk++) {
-        const int k = hh * KH + kk;
-        float y = 0.f, w = 0.f, dd = 0.f;
-        if (k < nr) {
-          w = ss.pw[k];
-          dd = ss.pd[k];
-          if (m < n) y = a.ens_obs[(size_t)ss.pidx[k] * n + m];
-        }
-        yv[kk] = y;
-        wv[kk] = y * w;
-        bpart = fmaf(wv[kk], dd, bpart);
+        wv[kk] = yv[kk] * wv[kk];
+        bpart = fmaf(wv[kk], dv[kk], bpart);
       }
 #pragma unroll
       for (int g = 0; g < KH / 4; g++) {
@@ -240,9 +253,9 @@ __global__ void __launch_bounds__(T8_NT, 1) sweep_tc128_kernel(SweepArgs a) {
         *reinterpret_cast<float4*>(stg + L::STG_BL + off) = l;
       }
       for (int k = tid; k < nr; k += T8_NT) {
-        const float dd = ss.pd[k];
-        p1 = fmaf(dd * dd, ss.pw[k], p1);
-        p3 += ss.pr[k];
+        const float dd = ss.pd[o + k];
+        p1 = fmaf(dd * dd, ss.pw[o + k], p1);
+        p3 += ss.pr[o + k];
       }
       tc::fence_smem_async();
       tc::fence_before_sync();
@@ -510,26 +523,25 @@ __global__ void __launch_bounds__(T8_NT, 1) sweep_tc128_kernel(SweepArgs a) {
           float* Zf = reinterpret_cast<float*>(sm + L::ZF);
           float* Af = reinterpret_cast<float*>(sm + L::AF);
           float* Pf = reinterpret_cast<float*>(sm + L::PF);
-#pragma unroll
-          for (int c0 = 0; c0 < 64; c0 += 8) {
-            const int c = cbase + c0;
+          // (column groups and halves in another order per row: distinct banks, as there)
+#pragma unroll 2
+          for (int i = 0; i < 8; i++) {
+            const int c0 = 8 * ((i + r) & 7), c = cbase + c0, sw = (c0 >> 5) << 2;
             const uint32_t off = tc::kmajor_off_bf16(r, c, 128);
             float sh[8], sl[8];
             unpack8(*reinterpret_cast<const uint4*>(sm + L::Z_HI + off), sh);
             unpack8(*reinterpret_cast<const uint4*>(sm + L::Z_LO + off), sl);
-            *reinterpret_cast<float4*>(Zf + r * 128 + c) =
-                make_float4(sh[0] + sl[0], sh[1] + sl[1], sh[2] + sl[2], sh[3] + sl[3]);
-            *reinterpret_cast<float4*>(Zf + r * 128 + c + 4) =
-                make_float4(sh[4] + sl[4], sh[5] + sl[5], sh[6] + sl[6], sh[7] + sl[7]);
+            const float4 z0 = make_float4(sh[0] + sl[0], sh[1] + sl[1], sh[2] + sl[2], sh[3] + sl[3]);
+            const float4 z1 = make_float4(sh[4] + sl[4], sh[5] + sl[5], sh[6] + sl[6], sh[7] + sl[7]);
+            *reinterpret_cast<float4*>(Zf + r * 128 + c + sw) = sw ? z1 : z0;
+            *reinterpret_cast<float4*>(Zf + r * 128 + c + 4 - sw) = sw ? z0 : z1;
           }
 #pragma unroll
           for (int c0 = 0; c0 < 64; c0 += 16) {
             float v[16];
             tc::tmem_ld16(DA + lane_off + cbase + c0, v);
 #pragma unroll
-            for (int j = 0; j < 16; j += 4)
-              *reinterpret_cast<float4*>(Af + r * 128 + cbase + c0 + j) =
-                  make_float4(v[j] * inv_s, v[j + 1] * inv_s, v[j + 2] * inv_s, v[j + 3] * inv_s);
+            for (int j = 0; j < 16; j++) Af[(cbase + c0 + j) * 128 + r] = v[j] * inv_s;  // symmetric to the bit
           }
           tc::fence_before_sync();
           __syncthreads();
@@ -555,7 +567,10 @@ __global__ void __launch_bounds__(T8_NT, 1) sweep_tc128_kernel(SweepArgs a) {
           }
           if (polish)
             it += ns_polish<T8_NP>(Af, Zf, Pf, red, tc_max > 0 ? T8_POLISH_MAX : a.max_ns_iter, a.polish_tol, &ok);
-          for (int idx = tid; idx < 128 * 128; idx += T8_NT) Wm[idx] = coef * Zf[idx];
+          for (int idx = tid; idx < 128 * 128 / 4; idx += T8_NT) {
+            const float4 z = reinterpret_cast<const float4*>(Zf)[idx];
+            reinterpret_cast<float4*>(Wm)[idx] = make_float4(coef * z.x, coef * z.y, coef * z.z, coef * z.w);
+          }
           __syncthreads();
         }
         if (tmo) break;
@@ -637,8 +652,19 @@ __global__ void __launch_bounds__(T8_NT, 1) sweep_tc128_kernel(SweepArgs a) {
       const int mm = tid & 127, vgp = tid >> 7;
       if (mm < n) {
         float acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 2
-        for (int k = 0; k < n; k++) {
+        int k = 0;
+        for (; k + 4 <= n; k += 4) {
+          float w[4];
+#pragma unroll
+          for (int i = 0; i < 4; i++) w[i] = Wm[(k + i) * 128 + mm];
+#pragma unroll
+          for (int j = 0; j < 4; j++)
+            if (vgp + 2 * j < nv) {
+              const float4 x = *reinterpret_cast<const float4*>(xs + (vgp + 2 * j) * 128 + k);
+              acc[j] = fmaf(x.w, w[3], fmaf(x.z, w[2], fmaf(x.y, w[1], fmaf(x.x, w[0], acc[j]))));
+            }
+        }
+        for (; k < n; k++) {
           const float w = Wm[k * 128 + mm];
 #pragma unroll
           for (int j = 0; j < 4; j++)
