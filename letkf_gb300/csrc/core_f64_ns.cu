@@ -30,7 +30,8 @@
 // busy; the FP32 phases of one CTA overlap the FP64 phases of the others on
 // the SM.  Measured: 8,640 regional points of k = 64 (mean list about 300)
 // 183 -> 26 ms (FP64 pipe 69 % busy); 32,256 SPEEDY-grid points of k = 40 (mean
-// list 86) 233 -> 23 ms (FP64 pipe 55 %, FP32 30 %); with every residual in
+// list 86) 233 -> 21 ms (FP32 products over the 40 members, not the 48 of the
+// tiles: 2 ms of it); with every residual in
 // FP64 a tenth more; a 40-point ring of k = 20, one point per SM, 1.43 -> 0.1.
 //
 // A point is left to core_f64.cu (status LETKF_PENDING until its launch) where
@@ -106,9 +107,11 @@ __device__ __forceinline__ void fn_ldc(const float* p, int tx, float (&v)[FnCfg<
   }
 }
 
-// acc = X^T Yb for this thread's tile (X symmetric, or its transpose is meant)
+// acc = X^T Yb for this thread's tile (X symmetric, or its transpose is meant),
+// over k < n8: the padding's rows and columns of both are zero off its diagonal,
+// so that it leaves the ensemble's part alone, and its own values are not used
 template <int NP>
-__device__ __forceinline__ void fn_gemm(const float* X, const float* Yb, int i0, int tx,
+__device__ __forceinline__ void fn_gemm(const float* X, const float* Yb, int n8, int i0, int tx,
                                         float (&acc)[FnCfg<NP>::TR][FnCfg<NP>::TC]) {
   using C = FnCfg<NP>;
 #pragma unroll
@@ -116,7 +119,7 @@ __device__ __forceinline__ void fn_gemm(const float* X, const float* Yb, int i0,
 #pragma unroll
     for (int b = 0; b < C::TC; b++) acc[a][b] = 0.f;
 #pragma unroll 4
-  for (int k = 0; k < NP; k++) {
+  for (int k = 0; k < n8; k++) {
     float av[C::TR], bv[C::TC];
     fn_ld<C::TR>(X + k * NP + i0, av);
     fn_ldc<NP>(Yb + k * NP, tx, bv);
@@ -175,13 +178,13 @@ __device__ __forceinline__ void fn_counted(int m, F&& f) {
 // do not commute with A grow (measured: residual 1e-2 instead of 1e-6 at
 // lambda_max / c = 100), so T is also kept transposed, in TT.
 template <int NP>
-__device__ bool fn_newton_schulz(float* Y, float* Z, float* T, float* TT, float* redf, float lo) {
+__device__ bool fn_newton_schulz(float* Y, float* Z, float* T, float* TT, float* redf, int n8, float lo) {
   using C = FnCfg<NP>;
   const int tid = threadIdx.x, i0 = (tid >> 4) * C::TR, tx = tid & 15;
   float acc[C::TR][C::TC], yn[C::TR][C::TC];
   float prev = INFINITY;
   for (int it = 0; it < 24; it++) {
-    fn_gemm<NP>(Z, Y, i0, tx, acc);
+    fn_gemm<NP>(Z, Y, n8, i0, tx, acc);
     float e2 = 0.f;
 #pragma unroll
     for (int a = 0; a < C::TR; a++)
@@ -190,19 +193,19 @@ __device__ bool fn_newton_schulz(float* Y, float* Z, float* T, float* TT, float*
         T[(i0 + a) * NP + fn_col<NP>(tx, b)] = acc[a][b];
         TT[fn_col<NP>(tx, b) * NP + i0 + a] = acc[a][b];
         const float d = acc[a][b] - (i0 + a == fn_col<NP>(tx, b) ? 1.f : 0.f);
-        e2 = fmaf(d, d, e2);
+        if (i0 + a < n8 && fn_col<NP>(tx, b) < n8) e2 = fmaf(d, d, e2);
       }
     e2 = block_sum<float, FN_NT>(e2, redf);  // publishes T
     if (!isfinite(e2)) return false;
     const float al = ns_scale(lo), sa = sqrtf(al);
     const float ka = 1.5f * sa, kb = 0.5f * al * sa;
     lo = f_ns(al * lo);
-    fn_gemm<NP>(Y, T, i0, tx, acc);
+    fn_gemm<NP>(Y, T, n8, i0, tx, acc);
 #pragma unroll
     for (int a = 0; a < C::TR; a++)
 #pragma unroll
       for (int b = 0; b < C::TC; b++) yn[a][b] = ka * Y[(i0 + a) * NP + fn_col<NP>(tx, b)] - kb * acc[a][b];
-    fn_gemm<NP>(TT, Z, i0, tx, acc);
+    fn_gemm<NP>(TT, Z, n8, i0, tx, acc);
 #pragma unroll
     for (int a = 0; a < C::TR; a++)
 #pragma unroll
@@ -227,18 +230,18 @@ __device__ bool fn_newton_schulz(float* Y, float* Z, float* T, float* TT, float*
 // Y tends to I and R to 2 D with Y0 D + D Y0 = R0.  Scaled steps as in the
 // Newton-Schulz iteration (the eigenvalue map of Y^2 is the same).
 template <int NP>
-__device__ void fn_sign(float* Y, float* Y2, float* R, float* U, float lo) {
+__device__ void fn_sign(float* Y, float* Y2, float* R, float* U, int n8, float lo) {
   using C = FnCfg<NP>;
   const int tid = threadIdx.x, i0 = (tid >> 4) * C::TR, tx = tid & 15;
   float acc[C::TR][C::TC], yn[C::TR][C::TC], rn[C::TR][C::TC];
   for (int it = 0; it < 20; it++) {
     const bool last = lo > 0.999f;
-    fn_gemm<NP>(Y, Y, i0, tx, acc);
+    fn_gemm<NP>(Y, Y, n8, i0, tx, acc);
 #pragma unroll
     for (int a = 0; a < C::TR; a++)
 #pragma unroll
       for (int b = 0; b < C::TC; b++) Y2[(i0 + a) * NP + fn_col<NP>(tx, b)] = acc[a][b];
-    fn_gemm<NP>(R, Y, i0, tx, acc);
+    fn_gemm<NP>(R, Y, n8, i0, tx, acc);
 #pragma unroll
     for (int a = 0; a < C::TR; a++)
 #pragma unroll
@@ -248,18 +251,18 @@ __device__ void fn_sign(float* Y, float* Y2, float* R, float* U, float lo) {
     const float ka = 1.5f * sa, kb = 0.5f * al * sa;
     lo = f_ns(al * lo);
     if (!last) {
-      fn_gemm<NP>(Y, Y2, i0, tx, acc);
+      fn_gemm<NP>(Y, Y2, n8, i0, tx, acc);
 #pragma unroll
       for (int a = 0; a < C::TR; a++)
 #pragma unroll
         for (int b = 0; b < C::TC; b++) yn[a][b] = ka * Y[(i0 + a) * NP + fn_col<NP>(tx, b)] - kb * acc[a][b];
     }
-    fn_gemm<NP>(Y, U, i0, tx, acc);  // Y R Y
+    fn_gemm<NP>(Y, U, n8, i0, tx, acc);  // Y R Y
 #pragma unroll
     for (int a = 0; a < C::TR; a++)
 #pragma unroll
       for (int b = 0; b < C::TC; b++) rn[a][b] = ka * R[(i0 + a) * NP + fn_col<NP>(tx, b)] + kb * acc[a][b];
-    fn_gemm<NP>(Y2, R, i0, tx, acc);  // Y^2 R; R Y^2 is its transpose
+    fn_gemm<NP>(Y2, R, n8, i0, tx, acc);  // Y^2 R; R Y^2 is its transpose
     __syncthreads();
 #pragma unroll
     for (int a = 0; a < C::TR; a++)
@@ -487,7 +490,7 @@ __global__ void __launch_bounds__(FN_NT, FnCfg<NP>::MINB) core_f64_ns_kernel(
       const float isf = 1.f / sfac;
       for (int idx = tid; idx < Q; idx += FN_NT) Y32[idx] *= isf;
       __syncthreads();
-      ok = fn_newton_schulz<NP>(Y32, Z32, T32, Y32 + Q, redf, lo);
+      ok = fn_newton_schulz<NP>(Y32, Z32, T32, Y32 + Q, redf, n8, lo);
     }
     if (ok) {
       // Z exactly symmetric; A/s as pairs of floats in A's place (A is in T)
@@ -640,7 +643,7 @@ __global__ void __launch_bounds__(FN_NT, FnCfg<NP>::MINB) core_f64_ns_kernel(
             }
           }
         __syncthreads();
-        fn_sign<NP>(M32, M32 + Q, R32, R32 + Q, lo);
+        fn_sign<NP>(M32, M32 + Q, R32, R32 + Q, n8, lo);
         // Z <- Z + D, D symmetrised; after the first correction Z is FP64
         if (it == 0) {
 #pragma unroll
