@@ -72,7 +72,8 @@ __global__ void __launch_bounds__(LKP_NT) lk_sums_kernel(int ne, int kp, const i
   const int l0 = min(L, piece * per), l1 = min(L, l0 + per);
   // list entry e: its row (packed, or observation ridx[e]) and departure
   auto row_of = [&](int64_t e) -> size_t { return ridx ? (size_t)ridx[e] : (size_t)e; };
-  for (int m = tid; m < kp; m += LKP_NT) {
+  const int m = blockIdx.z * LKP_NT + tid;
+  if (m < kp) {
     float acc = 0.f;
     if (m < ne) {
       if (rows16) {
@@ -91,6 +92,7 @@ __global__ void __launch_bounds__(LKP_NT) lk_sums_kernel(int ne, int kp, const i
     }
     pb[((size_t)b * LK_PIECES + piece) * kp + m] = acc;
   }
+  if (blockIdx.z > 0) return;
   double p1 = 0.0, p3 = 0.0;
   for (int l = l0 + tid; l < l1; l += LKP_NT) {
     const double d = dep[row_of(r0 + l)];
@@ -720,7 +722,7 @@ static int largek_core(int ne, int npts, const int64_t* offs, const float* rows,
     }
     g.nsplit = 1;
     // 2. prep
-    lk_sums_kernel<<<dim3(LK_PIECES, nb), LKP_NT, 0, s>>>(ne, kp, offs + p0, rows, rows16, ridx, w, dep, rloc, pb, pp);
+    lk_sums_kernel<<<dim3(LK_PIECES, nb, (kp + LKP_NT - 1) / LKP_NT), LKP_NT, 0, s>>>(ne, kp, offs + p0, rows, rows16, ridx, w, dep, rloc, pb, pp);
     lk_prep_kernel<<<nb, LKQ_NT, 0, s>>>(ne, kp, offs + p0, pb, pp, parm_infl + p0, minfl, G, Y, Z, bvec, inv_s, pt,
                                          active);
     note_launch();

@@ -82,8 +82,8 @@ __global__ void l64_weight_kernel(L64Lists q) {
   q.ed[q.o[b] + l] = sw * (double)q.dep[q.ridx ? (size_t)q.ridx[e] : (size_t)e];
 }
 
-// one piece of a list: b = B^T (sqrt(w) dep) and the largest |B| of each
-// member, p1 = sum w dep^2 and p3 = sum rloc
+// one piece of a list, L64_NT members a CTA: b = B^T (sqrt(w) dep) and the
+// largest |B| of each member; p1 = sum w dep^2 and p3 = sum rloc
 __global__ void __launch_bounds__(L64_NT) l64_stats_kernel(L64Lists q, int np, double* pb, unsigned long long* pm,
                                                            double* pp) {
   __shared__ double red[L64_NT / 32];
@@ -91,7 +91,8 @@ __global__ void __launch_bounds__(L64_NT) l64_stats_kernel(L64Lists q, int np, d
   const int L = q.L[b], per = (L + L64_SPLIT - 1) / L64_SPLIT, l0 = s * per, l1 = min(L, l0 + per);
   const int64_t r0 = q.r0[b], o = q.o[b];
   const size_t at = ((size_t)b * L64_SPLIT + s) * np;
-  for (int m = tid; m < np; m += L64_NT) {
+  const int m = blockIdx.z * L64_NT + tid;
+  if (m < np) {
     double acc = 0.0;
     unsigned long long mx = 0;
     if (m < q.ne) {
@@ -106,6 +107,7 @@ __global__ void __launch_bounds__(L64_NT) l64_stats_kernel(L64Lists q, int np, d
     pb[at + m] = acc;
     pm[at + m] = mx;
   }
+  if (blockIdx.z > 0) return;
   double p1 = 0.0, p3 = 0.0;
   for (int l = l0 + tid; l < l1; l += L64_NT) {
     p1 += q.ed[o + l] * q.ed[o + l];
@@ -545,7 +547,7 @@ int largek_fp64_pass(int ne, int npts, const int64_t* offs, const float* rows, c
     cudaMemcpyAsync(Ls, hL.data(), sizeof(int) * nb, cudaMemcpyHostToDevice, s);
     // 1. Gram and the sums of the lists
     l64_weight_kernel<<<dim3((gl + 255) / 256, nb), 256, 0, s>>>(q);
-    l64_stats_kernel<<<dim3(L64_SPLIT, nb), L64_NT, 0, s>>>(q, np, pb, pm, pp);
+    l64_stats_kernel<<<dim3(L64_SPLIT, nb, (np + L64_NT - 1) / L64_NT), L64_NT, 0, s>>>(q, np, pb, pm, pp);
     l64_stats_sum_kernel<<<dim3((np + L64_NT - 1) / L64_NT, nb), L64_NT, 0, s>>>(np, pb, pm, pp, bvec, sl, pt);
     note_launch();
     note_launch();
