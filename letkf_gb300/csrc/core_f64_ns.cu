@@ -30,8 +30,8 @@
 // busy; the FP32 phases of one CTA overlap the FP64 phases of the others on
 // the SM.  Measured: 8,640 regional points of k = 64 (mean list about 300)
 // 183 -> 26 ms (FP64 pipe 69 % busy); 32,256 SPEEDY-grid points of k = 40 (mean
-// list 86) 233 -> 21 ms (FP32 products over the 40 members, not the 48 of the
-// tiles: 2 ms of it); with every residual in
+// list 86) 233 -> 21 ms (23 with FP32 products over the 48 columns of the tiles,
+// not the 40 members; FP64 pipe 59 %, FP32 28 %); with every residual in
 // FP64 a tenth more; a 40-point ring of k = 20, one point per SM, 1.43 -> 0.1.
 //
 // A point is left to core_f64.cu (status LETKF_PENDING until its launch) where
