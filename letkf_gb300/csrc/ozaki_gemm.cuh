@@ -8,9 +8,14 @@
 // accumulator: over K <= 512 its value is an integer of at most 8 * 512 * 64^2
 // = 2^24, so the tensor core's FP32 sum is exact whatever its order, and the
 // eight accumulators are joined in integers and rounded to FP64 once per 512
-// products.  What is dropped is below 2^-55 of the rows' largest elements for
-// each factor: a product as good as an FP64 one whose terms were rounded at
-// that size (K. Ozaki's error-free splitting, Ozaki, Ogita, Oishi, Rump 2012).
+// products; pieces of 512 are added up in FP64, and the tile is written (and
+// mirrored, and transposed) once, when its last piece is in.  Of one product
+// x y the rounding of the operands loses at most 2^-56 of each row's scale and
+// the pairs with i + j <= 6 at most 2^-53 of the two scales' product (7 pairs of
+// 2^12 2^-68 and a hundredth of that), a scale being at most twice the row's
+// largest element: as good as FP64 for elements near their row's largest, and
+// to the same absolute size for smaller ones (K. Ozaki's error-free splitting,
+// Ozaki, Ogita, Oishi, Rump 2012).
 //
 // Bound: BF16 mma.sync (598 TFLOP/s measured here), 36 of them for one FP64
 // multiply-add: 16 TFLOP/s where the FP64 pipe has 1.2 and DGEMM reached 0.92.
@@ -31,9 +36,10 @@ constexpr int OZ_KEXACT = 512;    // K up to which the FP32 sums are exact
 constexpr int OZ_NT = 256;
 constexpr int OZ_STAGES = 3;
 constexpr int OZ_OPER = OZ_D * OZ_TILE * OZ_KC * 2;  // bytes of one operand's stage
-constexpr int OZ_SMEM = OZ_STAGES * 2 * OZ_OPER;
 constexpr int OZ_OUT_LD = OZ_TILE + 1;
-static_assert(OZ_SMEM >= OZ_TILE * OZ_OUT_LD * 8, "the output tile reuses the stages");
+constexpr int OZ_RING = OZ_STAGES * 2 * OZ_OPER;
+constexpr int OZ_OUT = OZ_TILE * OZ_OUT_LD * 8;
+static_assert(OZ_RING >= OZ_OUT && OZ_RING + OZ_OUT <= 227 * 1024, "shared memory");
 
 // exponent e with |x| < 2^e for the largest magnitude whose bits are mx, as a
 // scale 2^e (NaN where a value is not finite)
@@ -63,7 +69,7 @@ struct OzGemm {
   const double* sa;      // [batch][n] row scales
   const double* sb;
   double* out;           // [batch or split][n][n] row-major
-  double* outT;          // its transpose, or NULL
+  double* outT;          // its transpose, or NULL (nsplit 1)
   int64_t obatch;        // elements between the outputs of two points
   int lower;             // only tiles on and below the diagonal
   int mirror;            // and their transposes (a symmetric product)
@@ -91,6 +97,9 @@ __device__ __forceinline__ void oz_ldm4(uint32_t addr, uint32_t (&r)[4]) {
 // bytes, chunks XORed so that eight rows of one chunk lie on all banks
 __device__ __forceinline__ uint32_t oz_off(int r, int c) { return (uint32_t)(r * 64 + ((c ^ ((r >> 1) & 3)) << 4)); }
 
+// MANY: more than one piece of K; the output tile, the sum of the pieces, then
+// lies after the stages and not in their place
+template <bool MANY>
 __global__ void __launch_bounds__(OZ_NT, 1) oz_gemm_kernel(OzGemm g) {
   extern __shared__ __align__(128) unsigned char osm[];
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -118,6 +127,7 @@ __global__ void __launch_bounds__(OZ_NT, 1) oz_gemm_kernel(OzGemm g) {
   // K is walked in exact pieces; piece p belongs to split p % nsplit
   const int K = g.kend ? min(g.K, (g.kend[b] + OZ_KC - 1) / OZ_KC * OZ_KC) : g.K;
   const int npiece = (K + OZ_KEXACT - 1) / OZ_KEXACT;
+  if (g.accumulate && split >= npiece) return;
 
   auto load = [&](int k0, int stage) {
     // 2 operands x 8 digits x 64 rows x 4 chunks of 16 bytes
@@ -140,7 +150,9 @@ __global__ void __launch_bounds__(OZ_NT, 1) oz_gemm_kernel(OzGemm g) {
   const double* sa = g.sa + (size_t)b * g.n + m0;
   const double* sb = g.sb + (size_t)b * g.n + n0;
   double* out = g.out + (size_t)b * g.obatch + (size_t)split * g.osplit;
-  bool first = true;
+  double* tile = reinterpret_cast<double*>(osm + (MANY ? OZ_RING : 0));  // an element is one thread's until the last piece is in
+  if (split >= npiece)
+    for (int t = tid; t < OZ_TILE * OZ_OUT_LD; t += OZ_NT) tile[t] = 0.0;
 
   for (int piece = split; piece < npiece; piece += g.nsplit) {
     const int kb = piece * OZ_KEXACT, nst = min(OZ_KEXACT, K - kb) / OZ_KC;
@@ -150,7 +162,7 @@ __global__ void __launch_bounds__(OZ_NT, 1) oz_gemm_kernel(OzGemm g) {
       for (int t = 0; t < 4; t++)
 #pragma unroll
         for (int e = 0; e < 4; e++) acc[q][t][e] = 0.f;
-    __syncthreads();  // the stages (and the output tile in them) are free
+    __syncthreads();  // the stages are free
     for (int s = 0; s < OZ_STAGES - 1; s++) {
       if (s < nst) load(kb + s * OZ_KC, s);
       asm volatile("cp.async.commit_group;" ::: "memory");
@@ -186,9 +198,10 @@ __global__ void __launch_bounds__(OZ_NT, 1) oz_gemm_kernel(OzGemm g) {
       }
     }
     // join the accumulators: sum_q acc_q 2^(7 q), two exact integers and one rounding
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();
-    double* tile = reinterpret_cast<double*>(osm);
+    if (!MANY) {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncthreads();
+    }
 #pragma unroll
     for (int t = 0; t < 4; t++)
 #pragma unroll
@@ -201,41 +214,44 @@ __global__ void __launch_bounds__(OZ_NT, 1) oz_gemm_kernel(OzGemm g) {
         }
         const double v = fma((double)hi, 268435456.0, (double)lo);  // 2^28
         const int r = row + (e >> 1) * 8, c = col + 8 * t + (e & 1);
-        tile[r * OZ_OUT_LD + c] = v * sa[r] * sb[c] * 4.336808689942018e-19;  // 2^-61
+        double* sum = tile + r * OZ_OUT_LD + c;
+        const double w = v * sa[r] * sb[c] * 4.336808689942018e-19;  // 2^-61
+        *sum = !MANY || piece == split ? w : *sum + w;
       }
-    __syncthreads();
-    const bool add = g.accumulate || !first;
-    first = false;
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  for (int t = tid; t < OZ_TILE * OZ_TILE; t += OZ_NT) {
+    const int r = t / OZ_TILE, c = t % OZ_TILE;
+    const double v = g.mirror && ti == tj && r < c ? tile[c * OZ_OUT_LD + r] : tile[r * OZ_OUT_LD + c];
+    double* o = out + (size_t)(m0 + r) * g.n + n0 + c;
+    *o = g.accumulate ? *o + v : v;
+  }
+  if ((g.mirror && ti != tj) || g.outT) {
+    double* oT = g.outT ? g.outT + (size_t)b * g.obatch : out;
     for (int t = tid; t < OZ_TILE * OZ_TILE; t += OZ_NT) {
-      const int r = t / OZ_TILE, c = t % OZ_TILE;
-      const double v = tile[r * OZ_OUT_LD + c];
-      double* o = out + (size_t)(m0 + r) * g.n + n0 + c;
-      if (add)
-        *o += v;
-      else if (!g.mirror || ti != tj)
-        *o = v;
-      else
-        *o = r >= c ? v : tile[c * OZ_OUT_LD + r];
-    }
-    if ((g.mirror && ti != tj) || g.outT) {
-      double* oT = g.outT ? g.outT + (size_t)b * g.obatch : out;
-      for (int t = tid; t < OZ_TILE * OZ_TILE; t += OZ_NT) {
-        const int c = t / OZ_TILE, r = t % OZ_TILE;
-        oT[(size_t)(n0 + c) * g.n + m0 + r] = tile[r * OZ_OUT_LD + c];
-      }
+      const int c = t / OZ_TILE, r = t % OZ_TILE;
+      double* o = oT + (size_t)(n0 + c) * g.n + m0 + r;
+      *o = g.accumulate ? *o + tile[r * OZ_OUT_LD + c] : tile[r * OZ_OUT_LD + c];
     }
   }
 }
 
-inline int oz_gemm(const OzGemm& g, int nb, cudaStream_t s) {
+template <bool MANY>
+int oz_launch(const OzGemm& g, int nb, cudaStream_t s) {
+  constexpr int bytes = OZ_RING + (MANY ? OZ_OUT : 0);
   static std::atomic<uint32_t> done{0};
-  const cudaError_t e = set_smem_once(oz_gemm_kernel, OZ_SMEM, done);
+  const cudaError_t e = set_smem_once(oz_gemm_kernel<MANY>, bytes, done);
   if (e != cudaSuccess) return cuda_status(e);
   const int nt = g.n / OZ_TILE;
   dim3 grid(g.lower ? nt * (nt + 1) / 2 : nt * nt, 1, nb * g.nsplit);
-  oz_gemm_kernel<<<grid, OZ_NT, OZ_SMEM, s>>>(g);
+  oz_gemm_kernel<MANY><<<grid, OZ_NT, bytes, s>>>(g);
   note_launch();
   return cuda_status(cudaGetLastError());
+}
+
+inline int oz_gemm(const OzGemm& g, int nb, cudaStream_t s) {
+  return g.K > OZ_KEXACT ? oz_launch<true>(g, nb, s) : oz_launch<false>(g, nb, s);
 }
 
 }  // namespace letkf

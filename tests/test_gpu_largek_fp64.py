@@ -119,3 +119,18 @@ def test_values_that_are_not_finite_stay_reported(cuda):
     st = out["status"].cpu().numpy()
     assert st[0] == 0 and st[1] != 0 and st[2] != 0
     assert np.isfinite(out["trans"][0].cpu().numpy()).all()
+
+
+@pytest.mark.parametrize("ne", [513, 576, 640, 1000, 1024])
+@pytest.mark.parametrize("alone", [True, False])
+def test_ensembles_of_more_than_one_piece(cuda, ne, alone):
+    """k x k products whose K is more than the 512 that one exact sum holds:
+    every tile, its mirror and its transpose are the sum of all pieces."""
+    Ls, err = ([700], [3e-4]) if alone else ([513, 200, 1100, 31], [1e-3, 1.0, 1e-3, 2e-5])
+    ref, out, pinf = _run(cuda, ne, Ls, np.array(err), ne)
+    hard = [0] if alone else [0, 2, 3]
+    assert (ref["kappa"][hard] > 1.0e5).all() and (ref["kappa"][hard] < 3.0e6).all()
+    assert (out["status"] == 0).all()
+    _check(ref, out, pinf, hard)
+    if not alone:
+        assert np.abs(out["trans"][1] - ref["trans"][1]).max() <= 1e-4 * np.abs(ref["trans"][1]).max()
