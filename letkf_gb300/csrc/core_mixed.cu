@@ -24,8 +24,8 @@ namespace letkf {
 // tile is what balances loads and multiply-adds); operands are loaded one step
 // ahead; up to k = 32 one warp takes a point by itself and never meets a
 // barrier; padding is to 16, 32, 48, 64, 96 or 128; the first step has Z = I
-// (one product instead of three) and the last needs no new Y; points are taken
-// from a counter.  100,000 points of k = 32 with 21 local observations: 5.49
+// (one product instead of three) and the last needs no new Y; a CTA's points
+// are handed out by the hardware.  100,000 points of k = 32 with 21 local observations: 5.49
 // -> 2.19 ms (FMA pipe 54 % busy); 4,001 points of k = 50 with 133 on average:
 // 1.77 -> 0.86 ms (48 %).  Every sum keeps the order that the eigensolver form
 // (and this one before) adds in, so transforms and inflation are unchanged to
@@ -35,11 +35,11 @@ template <int NP>
 struct MnCfg;
 template <>
 struct MnCfg<16> {
-  static constexpr int TX = 8, TY = 4, CH = 16, MINB = 8;
+  static constexpr int TX = 8, TY = 4, CH = 16, MINB = 16;
 };
 template <>
 struct MnCfg<32> {
-  static constexpr int TX = 8, TY = 4, CH = 32, MINB = 4;
+  static constexpr int TX = 8, TY = 4, CH = 32, MINB = 8;
 };
 template <>
 struct MnCfg<48> {
@@ -62,7 +62,11 @@ template <int NP>
 struct Mn {
   using C = MnCfg<NP>;
   static constexpr int TP = C::TX * C::TY;               // threads of a point
-  static constexpr int PPC = TP == 32 ? 4 : 1;           // points of a CTA
+  // points of a CTA: lists differ from point to point, and the CTA's shared memory is held until its last one is
+  // done; with one point 15 warps fit an SM where two leave 16 (100,000 points of k = 20, lists 0..150: four 2.36 ms,
+  // two 2.26, one 2.30).  Points taken from a counter in device memory take 2.22 there, but an allocation a call: 20,000
+  // points of k = 16 300 us against 165, 4,000 of k = 50 797 against 680 (calls in a row, that wait for nothing: 979, 993)
+  static constexpr int PPC = TP == 32 ? 2 : 1;
   // product tile of a thread: TR consecutive rows, TC columns in groups of G (4 where TC allows it) that lie
   // G TX apart, so that the lanes of a quarter warp read and write 128 consecutive bytes
   static constexpr int TR = NP / C::TY, TC = NP / C::TX, G = TC % 4 == 0 ? 4 : 2;
@@ -314,7 +318,7 @@ template <int NP>
 __global__ void __launch_bounds__(Mn<NP>::TP* Mn<NP>::PPC, MnCfg<NP>::MINB) core_mixed_ns_kernel(
     int n, int npts, const int64_t* __restrict__ offs, const float* __restrict__ rows,
     const float* __restrict__ rdiag, const float* __restrict__ rloc, const float* __restrict__ dep,
-    double* parm_infl, float* trans, float* transm, int rdiag_wloc, double minfl, int* status, int* counter) {
+    double* parm_infl, float* trans, float* transm, int rdiag_wloc, double minfl, int* status) {
   using M = Mn<NP>;
   using C = MnCfg<NP>;
   constexpr int TR = M::TR, TC = M::TC, TP = M::TP, CH = C::CH, Q = NP * NP;
@@ -329,12 +333,7 @@ __global__ void __launch_bounds__(Mn<NP>::TP* Mn<NP>::PPC, MnCfg<NP>::MINB) core
   float* wts = g + NP;        // weight, departure, rloc of a chunk, twice
   float* red = wts + 6 * CH;  // 32
   const int i0 = (tp / C::TX) * TR, tx = tp % C::TX;
-  // points beyond the first grid's worth are taken from a counter (lists and
-  // iteration counts differ from point to point)
-  int* next = reinterpret_cast<int*>(red + 31);
-  for (int p = blockIdx.x * M::PPC + slot; p < npts; p = *next) {
-    mn_sync<NP>();  // every thread has read *next
-    if (tp == 0) *next = counter ? (int)(gridDim.x * M::PPC) + atomicAdd(counter, 1) : npts;
+  for (int p = blockIdx.x * M::PPC + slot; p < npts; p += gridDim.x * M::PPC) {
     const int64_t r0 = offs[p];
     const int L = (int)(offs[p + 1] - r0);
     double infl = parm_infl[p];
@@ -569,21 +568,10 @@ static int launch_ns(int ne, int npts, const int64_t* offs, const float* rows, c
   auto kern = core_mixed_ns_kernel<NP>;
   const cudaError_t err = set_smem_once(kern, M::BYTES, done);
   if (err != cudaSuccess) return cuda_status(err);
-  int dev = 0, nsm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  const int fit = (int)((size_t)(227 * 1024) / (M::BYTES + 1024));
-  const int per_sm = fit < MnCfg<NP>::MINB ? (fit < 1 ? 1 : fit) : MnCfg<NP>::MINB;
-  const int need = (npts + M::PPC - 1) / M::PPC, grid = need < nsm * per_sm ? need : nsm * per_sm;
-  int* counter = nullptr;
-  if (need > grid) {
-    if (cudaMallocAsync((void**)&counter, sizeof(int), stream) != cudaSuccess) return LETKF_ERR_CUDA;
-    cudaMemsetAsync(counter, 0, sizeof(int), stream);
-  }
+  const int grid = (npts + M::PPC - 1) / M::PPC;
   kern<<<grid, M::TP * M::PPC, M::BYTES, stream>>>(ne, npts, offs, rows, rdiag, rloc, dep, parm_infl, trans, transm,
-                                                   rdiag_wloc, minfl, status, counter);
+                                                   rdiag_wloc, minfl, status);
   note_launch();
-  if (counter) cudaFreeAsync(counter, stream);
   return cuda_status(cudaGetLastError());
 }
 
