@@ -455,7 +455,7 @@ int largek_fp64_pass(int ne, int npts, const int64_t* offs, const float* rows, c
   double *sw = nullptr, *ed = nullptr, *pb = nullptr, *pp = nullptr, *vec = nullptr, *part = nullptr, *pinf = nullptr;
   unsigned long long* pm = nullptr;
   int64_t* r0 = nullptr;
-  int *Ls = nullptr, *counts = nullptr, *which = nullptr, *skip = nullptr, *kend = nullptr;
+  int *Ls = nullptr, *counts = nullptr, *which = nullptr, *skip = nullptr;
   L64Point* pt = nullptr;
   std::vector<void*> held;
   bool okm = true;
@@ -480,7 +480,6 @@ int largek_fp64_pass(int ne, int npts, const int64_t* offs, const float* rows, c
   alloc(&counts, sizeof(int) * 2);
   alloc(&which, sizeof(int) * R);
   alloc(&skip, sizeof(int) * R);
-  alloc(&kend, sizeof(int) * R);
   alloc(&pt, sizeof(L64Point) * R);
   rc = okm ? LETKF_OK : LETKF_ERR_CUDA;
   const size_t vs = (size_t)np * R;
@@ -526,11 +525,12 @@ int largek_fp64_pass(int ne, int npts, const int64_t* offs, const float* rows, c
     h.skip = skip;
     return oz_gemm(h, nb, s);
   };
+  // sources of the group's copies: written again only after the group's last synchronisation
+  std::vector<int64_t> hr(2 * R, 0);
+  std::vector<int> hL(R, 0);
   for (size_t g0 = 0; g0 < todo.size() && rc == LETKF_OK; g0 += R) {
     const int nb = (int)std::min<size_t>(R, todo.size() - g0);
     const dim3 rg(np / (L64_NT / 32), nb);
-    std::vector<int64_t> hr(2 * R, 0);
-    std::vector<int> hL(nb), hk(nb);
     int64_t o = 0;
     int gl = 0;
     for (int j = 0; j < nb; j++) {
@@ -554,8 +554,6 @@ int largek_fp64_pass(int ne, int npts, const int64_t* offs, const float* rows, c
     note_launch();
     cudaMemsetAsync(Gp, 0, sizeof(double) * mat * nb * nsplit, s);
     for (int k0 = 0; k0 < gl && rc == LETKF_OK; k0 += kc) {
-      for (int j = 0; j < nb; j++) hk[j] = std::max(0, std::min(kc, hL[j] - k0));
-      cudaMemcpyAsync(kend, hk.data(), sizeof(int) * nb, cudaMemcpyHostToDevice, s);
       l64_list_digits_kernel<<<dim3((std::min(kc, gl - k0) + 63) / 64, nt, nb), L64_NT, tile_bytes, s>>>(q, np, k0, kc,
                                                                                                        sl, dl);
       note_launch();
@@ -569,7 +567,8 @@ int largek_fp64_pass(int ne, int npts, const int64_t* offs, const float* rows, c
       h.nsplit = nsplit;
       h.lower = 1;
       h.accumulate = 1;
-      h.kend = kend;
+      h.len = Ls;
+      h.k0 = k0;
       rc = oz_gemm(h, nb, s);
     }
     if (rc != LETKF_OK) break;
@@ -631,7 +630,6 @@ int largek_fp64_pass(int ne, int npts, const int64_t* offs, const float* rows, c
     l64_matvec_kernel<<<rg, L64_NT, 0, s>>>(np, Z, bvec, gvec);
     l64_finalize_kernel<<<rg, L64_NT, 0, s>>>(ne, np, part, Z, gvec, pt, which, parm_infl, trans, transm, status);
     for (int i = 0; i < 6; i++) note_launch();
-    // the host arrays of the group's copies live until they are done
     rc = cuda_status(cudaStreamSynchronize(s));
   }
   for (void* p : held) cudaFreeAsync(p, s);

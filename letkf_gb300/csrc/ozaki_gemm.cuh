@@ -77,7 +77,8 @@ struct OzGemm {
   int nsplit;            // K split over this many CTAs, each with its own output
   int64_t osplit;        // elements between their outputs
   const int* skip;       // [batch] or NULL: 1 leaves the point's output alone
-  const int* kend;       // [batch] or NULL: K of the point, the digits past it up to a multiple of 64 are zero
+  const int* len;        // [batch] or NULL: K of the point is len - k0, the digits past it up to a multiple of 64 are zero
+  int k0;
 };
 
 __device__ __forceinline__ void oz_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
@@ -125,7 +126,7 @@ __global__ void __launch_bounds__(OZ_NT, 1) oz_gemm_kernel(OzGemm g) {
   const uint16_t* Bb = g.B + (size_t)b * OZ_D * plane + (size_t)n0 * g.K;
   const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(osm);
   // K is walked in exact pieces; piece p belongs to split p % nsplit
-  const int K = g.kend ? min(g.K, (g.kend[b] + OZ_KC - 1) / OZ_KC * OZ_KC) : g.K;
+  const int K = g.len ? max(0, min(g.K, (g.len[b] - g.k0 + OZ_KC - 1) / OZ_KC * OZ_KC)) : g.K;
   const int npiece = (K + OZ_KEXACT - 1) / OZ_KEXACT;
   if (g.accumulate && split >= npiece) return;
 

@@ -134,3 +134,34 @@ def test_ensembles_of_more_than_one_piece(cuda, ne, alone):
     _check(ref, out, pinf, hard)
     if not alone:
         assert np.abs(out["trans"][1] - ref["trans"][1]).max() <= 1e-4 * np.abs(ref["trans"][1]).max()
+
+
+def test_lists_of_several_digit_chunks_in_a_full_group(cuda):
+    """A group of 32 points holds 1,536 list entries' digits at a time at this
+    ensemble; lists around one and two chunks, one point in a second group."""
+    import torch
+
+    from letkf_gb300.core import core_batch_largek_indexed
+
+    ne, nobs = 513, 3300
+    rng = np.random.default_rng(17)
+    Ls = [1535, 1536, 1537, 600, 3071, 3072, 3073, 3200] + [int(x) for x in rng.integers(600, 1700, 25)]
+    offs = np.concatenate([[0], np.cumsum(Ls)]).astype(np.int64)
+    n = int(offs[-1])
+    basis = rng.standard_normal((24, ne)) * (0.6 ** np.arange(24))[:, None]
+    rows = (rng.standard_normal((nobs, 24)) @ basis).astype(np.float32)
+    rows -= rows.mean(1, keepdims=True)
+    idx = np.concatenate([np.sort(rng.choice(nobs, L, replace=False)) for L in Ls]).astype(np.int32)
+    rd = (rng.uniform(0.5, 2.0, n) * 1e-3).astype(np.float32)
+    rl = rng.uniform(0.05, 1.0, n).astype(np.float32)
+    d = rng.standard_normal(nobs).astype(np.float32)
+    infl = rng.uniform(0.95, 1.2, len(Ls))
+    f = lambda a: a.astype(np.float64)
+    ref = O.letkf_core_batch(ne, offs, f(rows)[idx], f(rd), f(rl), f(d)[idx], infl, want_transm=True)
+    ref["kappa"] = np.zeros(len(Ls))
+    t = lambda a, dt=torch.float32: torch.as_tensor(np.ascontiguousarray(a), dtype=dt, device=cuda)
+    pinf = t(infl, torch.float64)
+    out = core_batch_largek_indexed(ne, t(offs, torch.int64), t(idx, torch.int32), t(rows), t(d), t(rd), t(rl), pinf,
+                                    want_transm=True)
+    torch.cuda.synchronize()
+    _check(ref, {k: v.cpu().numpy() for k, v in out.items()}, pinf.cpu().numpy(), list(range(len(Ls))))
