@@ -11,12 +11,13 @@
 // beta + (1 - beta) I, xa = mean + xb' T; beta == 0 leaves mean + xb'; optional
 // clipping of the relative spread of one variable (Q_SPRD_MAX).
 //
-// One CTA per point, one kernel for both entry points (mode 0 with beta = 1 is
-// the plain update bit for bit).  The factors that do not depend on k stay out
-// of the sum: t(m) = sum_k x(k) W(k,m) and sum_k x(k) transm(k) once, then xa =
-// mean + beta (fac t + tx) + (1 - beta) x(m): one multiply-add per element of W
-// and variable where forming each weight first took five FP64 operations, and
-// increments added up before they meet the mean.
+// One CTA per point, one kernel for both entry points (mode 0 where beta is 1,
+// no array or an element of it, is the plain update bit for bit).  The factors
+// that do not depend on k stay out of the sum: t(m) = sum_k x(k) W(k,m) and
+// sum_k x(k) transm(k) once, then xa = mean + beta (fac t + tx) + (1 - beta)
+// x(m): one multiply-add per element of W and variable where forming each weight
+// first took five FP64 operations, and increments added up before they meet the
+// mean.
 //
 // Bound: the FP64 pipe (1.2 TFLOP/s; a warp instruction takes 16 cycles of an
 // SM), so lanes are kept full: outputs (variable, member) are flattened over
@@ -86,6 +87,7 @@ __global__ void __launch_bounds__(UPD_NT) update_f64_kernel(int n, int npts, int
   double* bet = fac + vcm;
   double* tx = bet + vcm;
   double* qv = tx + vcm;                   // [n]
+  __shared__ int one[UPD_VC];              // mode 0 with a beta array: beta is 1
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   for (int pl = blockIdx.x; pl < cnt; pl += gridDim.x) {
     const int p = p0 + pl;
@@ -135,6 +137,10 @@ __global__ void __launch_bounds__(UPD_NT) update_f64_kernel(int n, int npts, int
         mean[v] = s / (double)n;
         if (BETA) bet[v] = r.beta[(size_t)(v0 + v) * npts + p];
         fac[v] = 1.0;
+        if (MODE == 0 && BETA) {
+          one[v] = bet[v] == 1.0;
+          fac[v] = one[v] ? mean[v] : 0.0;  // what the sum of an output starts from
+        }
       }
       __syncthreads();
       for (int t = tid; t < total; t += UPD_NT) xp[t] = xp[t] - mean[t / n];
@@ -180,6 +186,7 @@ __global__ void __launch_bounds__(UPD_NT) update_f64_kernel(int n, int npts, int
           }
           if ((lane & 7) == 0 && vb + (lane >> 3) < vc) {
             tx[v] = sx;
+            if (MODE == 0 && BETA && one[v]) fac[v] = mean[v] + sx;
             if (MODE == 2) {  // beta == 0 skips weight_RTPS (factor 1)
               double f = 1.0;
               if ((!BETA || bet[v] != 0.0) && vg > 0.0 && va > 0.0)
@@ -202,8 +209,8 @@ __global__ void __launch_bounds__(UPD_NT) update_f64_kernel(int n, int npts, int
           const int t = min(32 * (c0 + u * (UPD_NT / 32)) + lane, total - 1);
           vv[u] = t / n;
           mm[u] = t - vv[u] * n;
-          // the plain update adds up from the mean, as the reference does
-          a[u] = PLAIN ? mean[vv[u]] : 0.0;
+          // the plain update, and where beta is 1, adds up from the mean, as the reference does
+          a[u] = PLAIN ? mean[vv[u]] : MODE == 0 ? fac[vv[u]] : 0.0;
           if (PLAIN && transm) a[u] = a[u] + tx[vv[u]];
           off[u] = mm[u] * sm;
         }
@@ -222,7 +229,7 @@ __global__ void __launch_bounds__(UPD_NT) update_f64_kernel(int n, int npts, int
           const int v = vv[u], m = mm[u];
           const double x = xp[v * n + m];
           double inc = a[u];
-          if (!PLAIN) {
+          if (!PLAIN && !(MODE == 0 && one[v])) {
             if (MODE == 1) inc = (1.0 - r.alpha) * inc + r.alpha * x;
             if (MODE == 2) inc = fac[v] * inc;
             if (transm) inc = inc + tx[v];

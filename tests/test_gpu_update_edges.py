@@ -134,3 +134,24 @@ def test_efso_edges(cuda, ne, npts, nterm):
         np.add.at(want[:, t], idx, (hdxa[idx] * w1[point]).sum(1) * rl / rd)
     _close(dj.cpu().numpy(), want)
     _close(sense.cpu().numpy(), want * dep[:, None])
+
+
+@pytest.mark.parametrize("ne,nv", [(7, 2), (31, 9), (32, 3), (40, 1), (40, 8), (50, 11), (64, 6), (101, 18), (128, 2)])
+@pytest.mark.parametrize("merged", [True, False])
+def test_beta_of_one_is_the_plain_update_bit_for_bit(cuda, ne, nv, merged):
+    import torch
+
+    from letkf_gb300.core import update_f64, update_relax_f64
+
+    rng = np.random.default_rng(ne + nv)
+    npts = 37
+    w = _t(rng.standard_normal((npts, ne, ne)) / ne, cuda)
+    tm = None if merged else _t(rng.standard_normal((npts, ne)) * 0.1, cuda)
+    xb = _t(rng.standard_normal((nv, npts, ne)) + 3.0, cuda)
+    beta = np.ones((nv, npts))
+    want = update_f64(xb, w, tm)
+    assert torch.equal(update_relax_f64(xb, w, tm)[0], want)
+    assert torch.equal(update_relax_f64(xb, w, tm, beta=_t(beta, cuda))[0], want)
+    beta[rng.uniform(size=beta.shape) < 0.4] = 0.5  # interior points beside a boundary's ramp
+    one = _t(beta == 1.0, cuda, torch.bool)
+    assert torch.equal(update_relax_f64(xb, w, tm, beta=_t(beta, cuda))[0][one], want[one])
