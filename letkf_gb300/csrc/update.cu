@@ -32,7 +32,7 @@
 namespace letkf {
 
 constexpr int UPD_NT = 128;
-constexpr int UPD_VC = 16;  // variables handled at a time
+constexpr int UPD_VC = 16;  // variables handled at a time, at most
 
 struct RelaxArgs {
   int mode;           // 0 none, 1 RTPP, 2 RTPS
@@ -45,8 +45,7 @@ struct RelaxArgs {
 
 // doubles of shared memory: W, D (RTPS), transm, x and the products of a chunk
 // of variables, mean / factor / beta / x . transm, the clipped variable
-__host__ __device__ inline size_t upd_smem_doubles(int n, int nv, int mode) {
-  const int vc = nv < UPD_VC ? nv : UPD_VC;
+static size_t upd_smem_doubles(int n, int vc, int mode) {
   const size_t d = mode == 2 ? (size_t)(n / 2 + 1) * n + (size_t)vc * n : 0;
   return (size_t)n * (n | 1) + d + n + (size_t)vc * n + 4 * (size_t)vc + n;
 }
@@ -62,17 +61,18 @@ __device__ __forceinline__ void upd_sums(int n, int sk, const double* xp, const 
 }
 
 // Points p0 .. p0+cnt-1 of arrays holding npts points; trans / transm / pao
-// are indexed from p0.  MODE and BETA (r.beta given) are compiled in: an
-// operation that is only predicated off still takes its FP64 slot.
+// are indexed from p0; vcm variables at a time.  MODE and BETA (r.beta given)
+// are compiled in: an operation that is only predicated off still takes its FP64
+// slot.
 template <int MODE, bool BETA>
-__global__ void __launch_bounds__(UPD_NT) update_f64_kernel(int n, int npts, int p0, int cnt, int nv,
+__global__ void __launch_bounds__(UPD_NT) update_f64_kernel(int n, int npts, int p0, int cnt, int nv, int vcm,
                                                              const double* __restrict__ xb,
                                                              const double* __restrict__ trans,
                                                              const double* __restrict__ transm,
                                                              const double* __restrict__ pao, RelaxArgs r, double* xa) {
   constexpr bool PLAIN = MODE == 0 && !BETA;
   extern __shared__ __align__(16) double su[];
-  const int ld = n | 1, nh = n / 2, vcm = nv < UPD_VC ? nv : UPD_VC;
+  const int ld = n | 1, nh = n / 2;
   // W(k, m) at k sk + m sm: as in memory, or transposed where the row length
   // would put the lanes' members on few banks
   const bool tr = n % 16 == 0;
@@ -123,8 +123,8 @@ __global__ void __launch_bounds__(UPD_NT) update_f64_kernel(int n, int npts, int
         if (d != 0 && (2 * d < n || (2 * d == n && j < i))) D[d * n + j] += Pp[idx];
       }
     }
-    for (int v0 = 0; v0 < nv; v0 += UPD_VC) {
-      const int vc = min(UPD_VC, nv - v0), total = vc * n;
+    for (int v0 = 0; v0 < nv; v0 += vcm) {
+      const int vc = min(vcm, nv - v0), total = vc * n;
       if (v0) __syncthreads();
       for (int t = tid; t < total; t += UPD_NT) {
         const int v = t / n;
@@ -387,7 +387,10 @@ template <int MODE, bool BETA>
 static int launch_update_as(int ne, int npts, int p0, int cnt, int nv, const double* xb, const double* trans,
                             const double* transm, const double* pao, const RelaxArgs& r, double* xa,
                             cudaStream_t stream) {
-  const size_t smem = sizeof(double) * upd_smem_doubles(ne, nv, MODE);
+  // RTPS of k = 128 leaves room for 15 variables beside W and D
+  int vc = nv < UPD_VC ? nv : UPD_VC;
+  if (sizeof(double) * upd_smem_doubles(ne, vc, MODE) > 227 * 1024) vc = UPD_VC / 2;
+  const size_t smem = sizeof(double) * upd_smem_doubles(ne, vc, MODE);
   auto kern = update_f64_kernel<MODE, BETA>;
   const cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (err != cudaSuccess) return cuda_status(err);
@@ -398,7 +401,7 @@ static int launch_update_as(int ne, int npts, int p0, int cnt, int nv, const dou
   int per_sm = (int)((size_t)(220 * 1024) / (smem + 1024));
   per_sm = per_sm < 1 ? 1 : per_sm > 8 ? 8 : per_sm;
   const int grid = cnt < nsm * per_sm ? cnt : nsm * per_sm;
-  kern<<<grid, UPD_NT, smem, stream>>>(ne, npts, p0, cnt, nv, xb, trans, transm, pao, r, xa);
+  kern<<<grid, UPD_NT, smem, stream>>>(ne, npts, p0, cnt, nv, vc, xb, trans, transm, pao, r, xa);
   note_launch();
   return cuda_status(cudaGetLastError());
 }

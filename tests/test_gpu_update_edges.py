@@ -155,3 +155,9 @@ def test_beta_of_one_is_the_plain_update_bit_for_bit(cuda, ne, nv, merged):
     beta[rng.uniform(size=beta.shape) < 0.4] = 0.5  # interior points beside a boundary's ramp
     one = _t(beta == 1.0, cuda, torch.bool)
     assert torch.equal(update_relax_f64(xb, w, tm, beta=_t(beta, cuda))[0][one], want[one])
+
+
+@pytest.mark.parametrize("ne,nv", [(127, 16), (127, 17), (128, 1), (128, 15), (128, 16), (128, 17), (128, 33)])
+def test_rtps_of_the_largest_ensembles(cuda, ne, nv):
+    """W and Pa of k = 128 leave room for fewer variables than a chunk holds."""
+    test_relaxed_update_edges(cuda, ne, nv, 2, nv - 1)
