@@ -267,6 +267,79 @@ __global__ void __launch_bounds__(UPD_NT) update_f64_kernel(int n, int npts, int
   }
 }
 
+// The plain update with merged weights (no transm) of more variables than the
+// rows kernel below takes: a CTA per point, a thread per output.  Nothing is
+// factored out of the sums here, so the general kernel's extra passes only cost
+// (320 MB of weights, at most 20,000 points: k = 20, 7 variables 172 us here and
+// 190 there, k = 33, 4 variables 257 and 270, k = 46, 8 variables 648 and 682).
+// Bound: the FP64 pipe.  W lies as in memory, or transposed where the row length
+// would put the lanes' members on two banks or one (k = 40, 4 variables: 360 ->
+// 305 us; from k = 100, two CTAs an SM, the transposing stores are no longer
+// hidden and only the latter is worth them).  The points are handed out by the
+// hardware: a grid of 8 CTAs an SM in fixed strides ends with its last CTAs alone
+// where 8 are not resident (k = 60, 4 variables: 450 us so, 360 here).
+__global__ void __launch_bounds__(UPD_NT) update_merged_kernel(int n, int npts, int p0, int cnt, int nv,
+                                                                const double* __restrict__ xb,
+                                                                const double* __restrict__ trans, double* xa) {
+  extern __shared__ __align__(16) double su[];
+  const int ld = n | 1, vcm = nv < UPD_VC ? nv : UPD_VC;
+  const bool tr = n % 16 == 0 || (n % 8 == 0 && n < 100);
+  const int sk = tr ? ld : 1, sm = tr ? 1 : n;  // W(k, m) at k sk + m sm
+  double* W = su;
+  double* xp = W + (size_t)n * ld;      // [vcm][n]
+  double* mean = xp + (size_t)vcm * n;  // [vcm]
+  const int tid = threadIdx.x;
+  for (int pl = blockIdx.x; pl < cnt; pl += gridDim.x) {
+    const int p = p0 + pl;
+    __syncthreads();
+    const double* Tp = trans + (size_t)pl * n * n;
+    if (tr) {
+      for (int idx = tid; idx < n * n; idx += UPD_NT) {
+        const int m = idx / n, k = idx - m * n;
+        W[k * ld + m] = Tp[idx];
+      }
+    } else {
+      for (int idx = tid; idx < n * n; idx += UPD_NT) W[idx] = Tp[idx];
+    }
+    for (int v0 = 0; v0 < nv; v0 += UPD_VC) {
+      const int total = min(UPD_VC, nv - v0) * n;
+      if (v0) __syncthreads();
+      for (int t = tid; t < total; t += UPD_NT) {
+        const int v = t / n;
+        xp[t] = xb[((size_t)(v0 + v) * npts + p) * n + (t - v * n)];
+      }
+      __syncthreads();
+      for (int v = tid; v * n < total; v += UPD_NT) {
+        double s = xp[v * n];
+        for (int m = 1; m < n; m++) s = s + xp[v * n + m];
+        mean[v] = s / (double)n;
+      }
+      __syncthreads();
+      for (int t = tid; t < total; t += UPD_NT) xp[t] = xp[t] - mean[t / n];
+      __syncthreads();
+      for (int t = tid; t < total; t += UPD_NT) {
+        const int v = t / n, m = t - v * n;
+        const double *x = xp + v * n, *w = W + m * sm;
+        double a = mean[v];
+        for (int k = 0; k < n; k++) a = fma(x[k], w[k * sk], a);
+        xa[((size_t)(v0 + v) * npts + p) * n + m] = a;
+      }
+    }
+  }
+}
+
+static int launch_update_merged(int ne, int npts, int p0, int cnt, int nv, const double* xb, const double* trans,
+                                double* xa, cudaStream_t stream) {
+  const int vc = nv < UPD_VC ? nv : UPD_VC;
+  const size_t smem = sizeof(double) * ((size_t)ne * (ne | 1) + (size_t)vc * ne + vc);
+  const cudaError_t err =
+      cudaFuncSetAttribute(update_merged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (err != cudaSuccess) return cuda_status(err);
+  update_merged_kernel<<<cnt, UPD_NT, smem, stream>>>(ne, npts, p0, cnt, nv, xb, trans, xa);
+  note_launch();
+  return cuda_status(cudaGetLastError());
+}
+
 // The plain update of few variables: a warp per batch of rows (variable,
 // point), no barrier.  Each lane reads its member's row of trans straight from
 // global memory, 64 consecutive bytes at a time where rows are 16-byte aligned;
@@ -277,7 +350,7 @@ __global__ void __launch_bounds__(UPD_NT) update_f64_kernel(int n, int npts, int
 // member-order mean costs as many as the products when one lane does it alone,
 // so lanes take the rows of the batch.  One variable, 100,000 points of k = 32:
 // 0.57 -> 0.22 ms, 20,000 of k = 50: 0.22 -> 0.16, 4,000 of k = 128: 0.75 ->
-// 0.16 (before: a CTA per point).  The sums are those of the kernel above in
+// 0.16 (before: a CTA per point).  The sums are those of the kernels above in
 // the same order, so the results are the same bits.
 constexpr int UPR_ROWS = 16;
 
@@ -427,13 +500,25 @@ int launch_update_f64_range(int ne, int npts_total, int p0, int cnt, int nv, con
 #define UPR_LAUNCH(NVT)                                                                                 \
   return vec ? launch_update_rows<NVT, true>(ne, npts_total, p0, cnt, xb, trans, transm, xa, stream) \
              : launch_update_rows<NVT, false>(ne, npts_total, p0, cnt, xb, trans, transm, xa, stream)
-  // A warp per batch of rows re-reads x for every member it holds, the CTA form
-  // fills the lanes over all variables: the lines where they cross, measured
-  // with n = 20 / 40 / 64 / 128 (rows against CTA, us): 4 variables 534 / 606 /
-  // 521 / 497 against 591 / 537 / 533 / 1183, 2 variables 279 / 325 / 302 / 274
-  // against 498 / 342 / 340 / 895, 6 variables
-  // (64, 128) 747 / 736 against 823 / 1503.
-  const int rows = ne <= 32 ? 4 : ne <= 55 ? 2 : 6;
+  // A warp per batch of rows re-reads x for every member it holds, the CTA forms
+  // fill the lanes over all variables: the lines where they cross, with mean
+  // weights measured with n = 20 / 40 / 64 / 128 (rows against CTA, us): 4
+  // variables 534 / 606 / 521 / 497 against 591 / 537 / 533 / 1183, 2 variables
+  // 279 / 325 / 302 / 274 against 498 / 342 / 340 / 895, 6 variables (64, 128) 747
+  // / 736 against 823 / 1503.  With merged weights, every n and 1 to 6 variables,
+  // 320 MB of weights or 20,000 points (rows, the merged form, the thread per output that both replaced): n = 20, 2
+  // variables 82 / 102 / 108, 3 106 / 101 / 109; n = 24, 3 122 / 143 / 146, 4 150 /
+  // 143 / 151; n = 32, 4 189 / 213 / 336; n = 40, 1 144 / 174 / 188, 2 228 / 216 /
+  // 221; n = 56, 2 229 / 237 / 236; n = 72, 2 258 / 280 / 298, 3 361 / 326 / 353; n =
+  // 82, 5 503 / 508 / 602, 6 599 / 553 / 615; n = 128, 6 539 / 993 / 1251.
+  const int rows = transm     ? (ne <= 32 ? 4 : ne <= 55 ? 2 : 6)
+                   : ne <= 21 ? 2
+                   : ne <= 24 ? 3
+                   : ne <= 32 ? 4
+                   : ne <= 54 ? 1
+                   : ne <= 79 ? (ne % 16 ? 2 : 4)
+                   : ne <= 82 ? 5
+                              : 6;
   if (nv <= rows) {
     if (nv == 1) UPR_LAUNCH(1);
     if (nv == 2) UPR_LAUNCH(2);
@@ -443,6 +528,9 @@ int launch_update_f64_range(int ne, int npts_total, int p0, int cnt, int nv, con
     UPR_LAUNCH(6);
   }
 #undef UPR_LAUNCH
+  // k = 128 leaves one CTA an SM: the general kernel's four sums a thread hide the FP64 latency there (7 variables
+  // 1,071 us against 1,107)
+  if (!transm && ne < 128) return launch_update_merged(ne, npts_total, p0, cnt, nv, xb, trans, xa, stream);
   const RelaxArgs r = {0, 0.0, nullptr, -1, 0.0, nullptr};
   return launch_update(ne, npts_total, p0, cnt, nv, xb, trans, transm, nullptr, r, xa, stream);
 }

@@ -161,3 +161,22 @@ def test_beta_of_one_is_the_plain_update_bit_for_bit(cuda, ne, nv, merged):
 def test_rtps_of_the_largest_ensembles(cuda, ne, nv):
     """W and Pa of k = 128 leave room for fewer variables than a chunk holds."""
     test_relaxed_update_edges(cuda, ne, nv, 2, nv - 1)
+
+
+@pytest.mark.parametrize("ne", [2, 7, 8, 15, 16, 21, 22, 24, 25, 33, 40, 46, 54, 55, 72, 79, 80, 83, 88, 96, 100, 104, 127])
+@pytest.mark.parametrize("nv", [2, 3, 4, 5, 7, 16, 17])
+def test_merged_weights_on_either_side_of_each_rule(cuda, ne, nv):
+    """The forms of the plain update with merged weights, and the general
+    kernel that the relaxed entry point takes, give the same bits."""
+    import torch
+
+    from letkf_gb300.core import update_f64, update_relax_f64
+
+    rng = np.random.default_rng(10 * ne + nv)
+    npts = 29
+    w, xb = rng.standard_normal((npts, ne, ne)) / ne, rng.standard_normal((nv, npts, ne)) + 3.0
+    dw, dx = _t(w, cuda), _t(xb, cuda)
+    xa = update_f64(dx, dw)
+    assert torch.equal(xa, update_relax_f64(dx, dw)[0])
+    mean = xb.mean(-1, keepdims=True)
+    _close(xa.cpu().numpy(), mean + np.einsum("vpk,pmk->vpm", xb - mean, w))
