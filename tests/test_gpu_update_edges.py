@@ -180,3 +180,28 @@ def test_merged_weights_on_either_side_of_each_rule(cuda, ne, nv):
     assert torch.equal(xa, update_relax_f64(dx, dw)[0])
     mean = xb.mean(-1, keepdims=True)
     _close(xa.cpu().numpy(), mean + np.einsum("vpk,pmk->vpm", xb - mean, w))
+
+
+@pytest.mark.parametrize("ne,nv,npts,merged", [(8, 1, 160_001, True), (8, 1, 160_007, False), (5, 2, 170_003, True),
+                                               (8, 3, 200_003, False), (7, 4, 90_002, False), (31, 1, 30_001, True),
+                                               (32, 1, 30_001, False), (32, 4, 40_003, False),
+                                               (58, 6, 19_501, False)])
+def test_update_f64_batches_of_points(cuda, ne, nv, npts, merged):
+    """A warp's batch of several points, up to 16 rows, the last batch short."""
+    import torch
+
+    from letkf_gb300.core import update_f64
+
+    g = torch.Generator(device=cuda).manual_seed(ne + nv)
+    r = lambda *s: torch.randn(*s, dtype=torch.float64, device=cuda, generator=g)
+    w, tm, xb = r(npts, ne, ne) / ne, r(npts, ne) * 0.1, r(nv, npts, ne) + 3.0
+    xa = update_f64(xb, w, None if merged else tm)
+    for p in range(0, npts, 10_000):
+        q = slice(p, p + 10_000)
+        x = xb[:, q].cpu().numpy()
+        mean = x.mean(-1, keepdims=True)
+        x = x - mean
+        want = mean + np.matmul(x.transpose(1, 0, 2), w[q].cpu().numpy().transpose(0, 2, 1)).transpose(1, 0, 2)
+        if not merged:
+            want = want + np.einsum("vpk,pk->vp", x, tm[q].cpu().numpy())[..., None]
+        _close(xa[:, q].cpu().numpy(), want)
