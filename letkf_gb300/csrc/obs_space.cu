@@ -111,13 +111,13 @@ struct EfsoTerms {
 // One CTA per group of neighbouring grid points: their work1 in shared memory
 // and the entries of all their lists flattened over the lanes, so short lists
 // fill the warps.  A lane sums one entry's products over the members (FP64
-// pipe: one multiply-add per member and term; the entry's rloc / rdiag is
-// applied to the sums), and the rows of the 32 observations of a warp go
+// pipe: one multiply-add per member and term; the entry's rloc / rdiag, rounded
+// once, is applied to the sums), and the rows of the 32 observations of a warp go
 // through a tile of 16 members in shared memory, read as whole lines with the
 // next tile's loads in flight.  Bound: the FP64 pipe (1.2 TFLOP/s).  A thread
 // walking its own observation's row, one point per CTA, two more products per
 // member: 30,000 points with 50 local observations of k = 64 and 3 terms took
-// 2.55 ms, now 0.78 (FP64 pipe 69 % busy).
+// 2.55 ms, now 0.72 (0.78 where rloc / rdiag was formed after the sums).
 template <int NTERM>
 __global__ void __launch_bounds__(OSA_NT) efso_djdy_kernel(int ne, int npts, int nv, int group,
                                                             const __grid_constant__ EfsoTerms tv,
@@ -157,6 +157,7 @@ __global__ void __launch_bounds__(OSA_NT) efso_djdy_kernel(int ne, int npts, int
       const int64_t l = lb + lane;
       const bool on = l < l1;
       const int ob = on ? idx[l] : -1;
+      const double s = on ? rloc[l] / rdiag[l] : 0.0;
       int q = 0;
       while (q + 1 < np && l >= lo[q + 1]) q++;
       const double* w = w1 + (size_t)q * NTERM * ne;
@@ -189,7 +190,6 @@ __global__ void __launch_bounds__(OSA_NT) efso_djdy_kernel(int ne, int npts, int
         }
       }
       if (on) {
-        const double s = 1.0 / rdiag[l] * rloc[l];
 #pragma unroll
         for (int i = 0; i < NTERM; i++) atomicAdd(&djdy[(size_t)ob * NTERM + i], acc[i] * s);
       }

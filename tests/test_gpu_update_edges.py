@@ -205,3 +205,27 @@ def test_update_f64_batches_of_points(cuda, ne, nv, npts, merged):
         if not merged:
             want = want + np.einsum("vpk,pk->vp", x, tm[q].cpu().numpy())[..., None]
         _close(xa[:, q].cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("ne", [3, 16, 40])
+def test_efso_rounds_an_entry_twice(cuda, ne):
+    """Small integers, so that the sums over the members are exact: an entry's
+    rloc / rdiag and its product with the sum are the only roundings."""
+    import torch
+
+    from letkf_gb300.core import efso
+
+    rng = np.random.default_rng(ne)
+    npts, nobs = 40, 4000
+    offs = np.linspace(0, nobs, npts + 1).astype(np.int64)
+    idx = rng.permutation(nobs).astype(np.int32)
+    rd, rl = rng.uniform(0.1, 9.0, nobs), rng.uniform(0.0, 1.0, nobs)
+    i = lambda *s: rng.integers(-9, 10, s).astype(np.float64)
+    hdxa, fcst, fcer, dep = i(nobs, ne), i(2, npts, ne), i(2, npts), i(nobs)
+    dj, _ = efso(ne, _t(offs, cuda, torch.int64), _t(idx, cuda, torch.int32), _t(rd, cuda), _t(rl, cuda),
+                 _t(hdxa, cuda), _t(fcst, cuda), _t(fcer, cuda), [0, 0], _t(dep, cuda))
+    w1 = (fcst * fcer[..., None]).sum(0)
+    point = np.repeat(np.arange(npts), np.diff(offs))
+    want = np.empty(nobs)
+    want[idx] = (hdxa[idx] * w1[point]).sum(1) * (rl / rd)
+    assert np.array_equal(dj.cpu().numpy()[:, 0], want)
