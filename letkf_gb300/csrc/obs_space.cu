@@ -117,7 +117,9 @@ struct EfsoTerms {
 // next tile's loads in flight.  Bound: the FP64 pipe (1.2 TFLOP/s).  A thread
 // walking its own observation's row, one point per CTA, two more products per
 // member: 30,000 points with 50 local observations of k = 64 and 3 terms took
-// 2.55 ms, now 0.72 (0.78 where rloc / rdiag was formed after the sums).
+// 2.55 ms, now 0.78 (FP64 pipe 69 % busy).  (rloc and rdiag loaded ahead of the
+// sums hold registers: three terms take 90 instead of 80, one CTA an SM fewer, up
+// to 20 % more time where lists are even.)
 template <int NTERM>
 __global__ void __launch_bounds__(OSA_NT) efso_djdy_kernel(int ne, int npts, int nv, int group,
                                                             const __grid_constant__ EfsoTerms tv,
@@ -157,7 +159,6 @@ __global__ void __launch_bounds__(OSA_NT) efso_djdy_kernel(int ne, int npts, int
       const int64_t l = lb + lane;
       const bool on = l < l1;
       const int ob = on ? idx[l] : -1;
-      const double s = on ? rloc[l] / rdiag[l] : 0.0;
       int q = 0;
       while (q + 1 < np && l >= lo[q + 1]) q++;
       const double* w = w1 + (size_t)q * NTERM * ne;
@@ -190,6 +191,7 @@ __global__ void __launch_bounds__(OSA_NT) efso_djdy_kernel(int ne, int npts, int
         }
       }
       if (on) {
+        const double s = rloc[l] / rdiag[l];
 #pragma unroll
         for (int i = 0; i < NTERM; i++) atomicAdd(&djdy[(size_t)ob * NTERM + i], acc[i] * s);
       }
