@@ -27,6 +27,8 @@
 // x(i) D(d,i) x(i+d mod k), D(d,i) = Pa(i,i+d) + Pa(i+d,i), d = 0..k/2, formed
 // once per point for all variables, half the products of the full form and
 // every lane busy.  RTPS, 20,000 points, k = 50, 11 variables: 7.77 -> 2.53 ms.
+#include <algorithm>
+
 #include "letkf_common.cuh"
 
 namespace letkf {
@@ -267,28 +269,34 @@ __global__ void __launch_bounds__(UPD_NT) update_f64_kernel(int n, int npts, int
   }
 }
 
-// The plain update with merged weights (no transm) of more variables than the
-// rows kernel below takes: a CTA per point, a thread per output.  Nothing is
-// factored out of the sums here, so the general kernel's extra passes only cost
-// (320 MB of weights, at most 20,000 points: k = 20, 7 variables 172 us here and
-// 190 there, k = 33, 4 variables 257 and 270, k = 46, 8 variables 648 and 682).
-// Bound: the FP64 pipe.  W lies as in memory, or transposed where the row length
-// would put the lanes' members on two banks or one (k = 40, 4 variables: 360 ->
-// 305 us; from k = 100, two CTAs an SM, the transposing stores are no longer
-// hidden and only the latter is worth them).  The points are handed out by the
-// hardware: a grid of 8 CTAs an SM in fixed strides ends with its last CTAs alone
-// where 8 are not resident (k = 60, 4 variables: 450 us so, 360 here).
-__global__ void __launch_bounds__(UPD_NT) update_merged_kernel(int n, int npts, int p0, int cnt, int nv,
-                                                                const double* __restrict__ xb,
-                                                                const double* __restrict__ trans, double* xa) {
+// The plain update of more variables than the rows kernel below takes: a CTA per
+// point, a thread per output.  TM: transm given, its product with x formed as in
+// the general kernel; the results of both are the same bits.  The general
+// kernel's extra passes and barriers cost more than what it leaves out of the
+// sums saves (320 MB of weights, at most 20,000 points, merged: k = 20, 7
+// variables 172 us here and 190 there, k = 33, 4 variables 257 and 270, k = 46, 8
+// variables 648 and 682; with transm k = 2..8, 5 variables 0.84 to 0.95 of the time
+// of a thread per output with W + transm formed in its sum, and 1.08 to 1.40
+// there).  Bound: the FP64 pipe.  W lies as in memory, or transposed where the
+// row length would put the lanes' members on two banks or one (k = 40, 4
+// variables: 360 -> 305 us; from k = 100, two CTAs an SM, the transposing stores
+// are no longer hidden and only the latter is worth them).  The points are handed
+// out by the hardware: a grid of 8 CTAs an SM in fixed strides ends with its last
+// CTAs alone where 8 are not resident (k = 60, 4 variables: 450 us so, 360 here).
+template <bool TM>
+__global__ void __launch_bounds__(UPD_NT) update_point_kernel(int n, int npts, int p0, int cnt, int nv, int vcm,
+                                                              const double* __restrict__ xb,
+                                                              const double* __restrict__ trans,
+                                                              const double* __restrict__ transm, double* xa) {
   extern __shared__ __align__(16) double su[];
-  const int ld = n | 1, vcm = nv < UPD_VC ? nv : UPD_VC;
+  const int ld = n | 1;
   const bool tr = n % 16 == 0 || (n % 8 == 0 && n < 100);
   const int sk = tr ? ld : 1, sm = tr ? 1 : n;  // W(k, m) at k sk + m sm
   double* W = su;
   double* xp = W + (size_t)n * ld;      // [vcm][n]
-  double* mean = xp + (size_t)vcm * n;  // [vcm]
-  const int tid = threadIdx.x;
+  double* mean = xp + (size_t)vcm * n;  // [vcm] each
+  double* tx = mean + vcm;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   for (int pl = blockIdx.x; pl < cnt; pl += gridDim.x) {
     const int p = p0 + pl;
     __syncthreads();
@@ -301,15 +309,15 @@ __global__ void __launch_bounds__(UPD_NT) update_merged_kernel(int n, int npts, 
     } else {
       for (int idx = tid; idx < n * n; idx += UPD_NT) W[idx] = Tp[idx];
     }
-    for (int v0 = 0; v0 < nv; v0 += UPD_VC) {
-      const int total = min(UPD_VC, nv - v0) * n;
+    for (int v0 = 0; v0 < nv; v0 += vcm) {
+      const int vc = min(vcm, nv - v0), total = vc * n;
       if (v0) __syncthreads();
       for (int t = tid; t < total; t += UPD_NT) {
         const int v = t / n;
         xp[t] = xb[((size_t)(v0 + v) * npts + p) * n + (t - v * n)];
       }
       __syncthreads();
-      for (int v = tid; v * n < total; v += UPD_NT) {
+      for (int v = tid; v < vc; v += UPD_NT) {
         double s = xp[v * n];
         for (int m = 1; m < n; m++) s = s + xp[v * n + m];
         mean[v] = s / (double)n;
@@ -317,10 +325,23 @@ __global__ void __launch_bounds__(UPD_NT) update_merged_kernel(int n, int npts, 
       __syncthreads();
       for (int t = tid; t < total; t += UPD_NT) xp[t] = xp[t] - mean[t / n];
       __syncthreads();
+      if (TM) {
+        const double* tm = transm + (size_t)pl * n;
+        for (int vb = 4 * wid; vb < vc; vb += UPD_NT / 8) {
+          const int v = min(vb + (lane >> 3), vc - 1);
+          double sx = 0.0;
+          for (int k = lane & 7; k < n; k += 8) sx = fma(xp[v * n + k], tm[k], sx);
+#pragma unroll
+          for (int o = 4; o > 0; o >>= 1) sx += __shfl_xor_sync(0xffffffffu, sx, o);
+          if ((lane & 7) == 0 && vb + (lane >> 3) < vc) tx[v] = sx;
+        }
+        __syncthreads();
+      }
       for (int t = tid; t < total; t += UPD_NT) {
         const int v = t / n, m = t - v * n;
         const double *x = xp + v * n, *w = W + m * sm;
         double a = mean[v];
+        if (TM) a = a + tx[v];
         for (int k = 0; k < n; k++) a = fma(x[k], w[k * sk], a);
         xa[((size_t)(v0 + v) * npts + p) * n + m] = a;
       }
@@ -328,14 +349,16 @@ __global__ void __launch_bounds__(UPD_NT) update_merged_kernel(int n, int npts, 
   }
 }
 
-static int launch_update_merged(int ne, int npts, int p0, int cnt, int nv, const double* xb, const double* trans,
-                                double* xa, cudaStream_t stream) {
-  const int vc = nv < UPD_VC ? nv : UPD_VC;
-  const size_t smem = sizeof(double) * ((size_t)ne * (ne | 1) + (size_t)vc * ne + vc);
-  const cudaError_t err =
-      cudaFuncSetAttribute(update_merged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+template <bool TM>
+static int launch_update_point(int ne, int npts, int p0, int cnt, int nv, const double* xb, const double* trans,
+                               const double* transm, double* xa, cudaStream_t stream) {
+  // a pass of 16 variables, or of 1,024 outputs where that is more
+  const int vc = std::min(nv, std::max(UPD_VC, 1024 / ne));
+  const size_t smem = sizeof(double) * ((size_t)ne * (ne | 1) + (size_t)vc * ne + 2 * vc);
+  auto kern = update_point_kernel<TM>;
+  const cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (err != cudaSuccess) return cuda_status(err);
-  update_merged_kernel<<<cnt, UPD_NT, smem, stream>>>(ne, npts, p0, cnt, nv, xb, trans, xa);
+  kern<<<cnt, UPD_NT, smem, stream>>>(ne, npts, p0, cnt, nv, vc, xb, trans, transm, xa);
   note_launch();
   return cuda_status(cudaGetLastError());
 }
@@ -500,25 +523,24 @@ int launch_update_f64_range(int ne, int npts_total, int p0, int cnt, int nv, con
 #define UPR_LAUNCH(NVT)                                                                                 \
   return vec ? launch_update_rows<NVT, true>(ne, npts_total, p0, cnt, xb, trans, transm, xa, stream) \
              : launch_update_rows<NVT, false>(ne, npts_total, p0, cnt, xb, trans, transm, xa, stream)
-  // A warp per batch of rows re-reads x for every member it holds, the CTA forms
-  // fill the lanes over all variables: the lines where they cross, with mean
-  // weights measured with n = 20 / 40 / 64 / 128 (rows against CTA, us): 4
-  // variables 534 / 606 / 521 / 497 against 591 / 537 / 533 / 1183, 2 variables
-  // 279 / 325 / 302 / 274 against 498 / 342 / 340 / 895, 6 variables (64, 128) 747
-  // / 736 against 823 / 1503.  With merged weights, every n and 1 to 6 variables,
-  // 320 MB of weights or 20,000 points (rows, the merged form, the thread per output that both replaced): n = 20, 2
-  // variables 82 / 102 / 108, 3 106 / 101 / 109; n = 24, 3 122 / 143 / 146, 4 150 /
-  // 143 / 151; n = 32, 4 189 / 213 / 336; n = 40, 1 144 / 174 / 188, 2 228 / 216 /
-  // 221; n = 56, 2 229 / 237 / 236; n = 72, 2 258 / 280 / 298, 3 361 / 326 / 353; n =
-  // 82, 5 503 / 508 / 602, 6 599 / 553 / 615; n = 128, 6 539 / 993 / 1251.
-  const int rows = transm     ? (ne <= 32 ? 4 : ne <= 55 ? 2 : 6)
-                   : ne <= 21 ? 2
+  // A warp per batch of rows re-reads x for every member it holds, a CTA per
+  // point fills the lanes over all variables.  The lines where they cross are
+  // drawn from every n and 1 to 20 variables, 320 MB of weights or 20,000 points;
+  // rows / point (before either: a thread per output) in us, merged weights: n =
+  // 20, 2 variables 82 / 102 (108), 3 106 / 101 (109); n = 24, 3 122 / 143 (146), 4
+  // 150 / 143 (151); n = 32, 4 189 / 213 (336); n = 40, 1 144 / 174 (188), 2 228 /
+  // 216 (221); n = 64, 3 274 / 285 (616); n = 72, 2 258 / 280 (298), 3 361 / 326
+  // (353); n = 82, 5 503 / 508 (602), 6 599 / 553 (615); n = 128, 6 539 / 993 (1251).
+  // With mean weights the same up to n = 54 (n = 8, 3 variables 0.98 / 0.84 of the
+  // time before, n = 23, 3 0.60 / 0.68, 4 0.73 / 0.69, n = 44, 2 0.65 / 0.64), then
+  // n = 62, 3 0.49 / 0.53, 4 0.50 / 0.50; n = 64, 4 0.44 / 0.47; n = 68, 2 0.53 / 0.60, 3 0.56 / 0.51; n =
+  // 77, 5 0.52 / 0.59, 6 0.59 / 0.55; n = 83, 6 0.49 / 0.53.
+  const int rows = ne <= 21   ? 2
                    : ne <= 24 ? 3
                    : ne <= 32 ? 4
                    : ne <= 54 ? 1
-                   : ne <= 79 ? (ne % 16 ? 2 : 4)
-                   : ne <= 82 ? 5
-                              : 6;
+                   : transm   ? (ne <= 64 ? (ne % 16 ? 3 : 6) : ne <= 71 ? 2 : ne <= 79 ? 5 : 6)
+                              : (ne <= 79 ? (ne % 16 ? 2 : 4) : ne <= 82 ? 5 : 6);
   if (nv <= rows) {
     if (nv == 1) UPR_LAUNCH(1);
     if (nv == 2) UPR_LAUNCH(2);
@@ -528,9 +550,14 @@ int launch_update_f64_range(int ne, int npts_total, int p0, int cnt, int nv, con
     UPR_LAUNCH(6);
   }
 #undef UPR_LAUNCH
-  // k = 128 leaves one CTA an SM: the general kernel's four sums a thread hide the FP64 latency there (7 variables
-  // 1,071 us against 1,107)
-  if (!transm && ne < 128) return launch_update_merged(ne, npts_total, p0, cnt, nv, xb, trans, xa, stream);
+  // The general kernel's four sums a thread pay where few CTAs share an SM and W
+  // is read without bank conflicts or nearly: n = 128, merged, 7 variables 1,071
+  // us against 1,107; with mean weights n = 64, 11 variables 0.96 of the point
+  // form's time, n = 88 0.94, n = 96 0.90, n = 112 0.88 (n = 62 1.10, n = 98 1.04).
+  if (transm ? ne < 64 || ne % 8 != 0 : ne < 128) {
+    if (transm) return launch_update_point<true>(ne, npts_total, p0, cnt, nv, xb, trans, transm, xa, stream);
+    return launch_update_point<false>(ne, npts_total, p0, cnt, nv, xb, trans, transm, xa, stream);
+  }
   const RelaxArgs r = {0, 0.0, nullptr, -1, 0.0, nullptr};
   return launch_update(ne, npts_total, p0, cnt, nv, xb, trans, transm, nullptr, r, xa, stream);
 }

@@ -229,3 +229,23 @@ def test_efso_rounds_an_entry_twice(cuda, ne):
     want = np.empty(nobs)
     want[idx] = (hdxa[idx] * w1[point]).sum(1) * (rl / rd)
     assert np.array_equal(dj.cpu().numpy()[:, 0], want)
+
+
+@pytest.mark.parametrize("ne", [2, 3, 7, 10, 21, 24, 25, 32, 33, 54, 55, 63, 64, 65, 71, 72, 79, 80, 88, 100])
+@pytest.mark.parametrize("nv", [2, 3, 4, 5, 6, 7, 17, 40])
+def test_mean_weights_on_either_side_of_each_rule(cuda, ne, nv):
+    """The same with mean weights."""
+    import torch
+
+    from letkf_gb300.core import update_f64, update_relax_f64
+
+    rng = np.random.default_rng(10 * ne + nv)
+    npts = 29
+    w, tm = rng.standard_normal((npts, ne, ne)) / ne, rng.standard_normal((npts, ne)) * 0.1
+    xb = rng.standard_normal((nv, npts, ne)) + 3.0
+    dw, dt, dx = _t(w, cuda), _t(tm, cuda), _t(xb, cuda)
+    xa = update_f64(dx, dw, dt)
+    assert torch.equal(xa, update_relax_f64(dx, dw, dt)[0])
+    mean = xb.mean(-1, keepdims=True)
+    x = xb - mean
+    _close(xa.cpu().numpy(), mean + np.einsum("vpk,pmk->vpm", x, w) + np.einsum("vpk,pk->vp", x, tm)[..., None])
