@@ -249,3 +249,8 @@ def test_mean_weights_on_either_side_of_each_rule(cuda, ne, nv):
     mean = xb.mean(-1, keepdims=True)
     x = xb - mean
     _close(xa.cpu().numpy(), mean + np.einsum("vpk,pmk->vpm", x, w) + np.einsum("vpk,pk->vp", x, tm)[..., None])
+
+
+@pytest.mark.parametrize("ne", [3, 8, 16, 17, 30, 32, 33])
+def test_obs_analysis_of_few_members(cuda, ne):
+    test_obs_analysis_edges(cuda, ne)
