@@ -584,11 +584,17 @@ static int launch_mixed_np(int ne, int npts, const int64_t* offs, const float* r
   auto kern = core_mixed_kernel<NP>;
   const cudaError_t err = set_smem_once(kern, bytes, done);
   if (err != cudaSuccess) return cuda_status(err);
-  int dev = 0, nsm = 0;
+  int dev = 0, nsm = 0, per_sm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  const int fit = (int)((size_t)(227 * 1024) / (bytes + 1024));
-  const int grid = npts < nsm * (fit < 1 ? 1 : fit) ? npts : nsm * (fit < 1 ? 1 : fit);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, MixedCfg<NP>::NT, bytes);
+  if (per_sm < 1) per_sm = 1;
+  // Four times what is resident: a CTA without a point to solve leaves at once,
+  // and those with one seldom have a second behind it (1,000 points of k = 50, a
+  // twentieth of them beyond the iteration: a resident grid 4.1 ms, 2.9 so).  A
+  // grid of what shared memory alone allows left its last CTAs to a wave of their
+  // own (5,000 points of k = 16, all of them beyond it: 2.7 ms, 2.1 so).
+  const int most = 4 * nsm * per_sm, grid = npts < most ? npts : most;
   kern<<<grid, MixedCfg<NP>::NT, bytes, stream>>>(ne, npts, offs, rows, rdiag, rloc, dep, parm_infl, trans, transm,
                                                    rdiag_wloc, minfl, status, 12);
   note_launch();
