@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(T8_NT, 1) sweep_tc128_kernel(SweepArgs a) {
       // beyond nr is old and not used
 #pragma unroll
       for (int g = 0; g < KH / 4; g++) {
-        const int kb = hh * KH + 4 * g;  // of the stage  // of the stage
+        const int kb = hh * KH + 4 * g;  // of the stage
         const int4 i4 = *reinterpret_cast<const int4*>(ss.pidx + o + kb);
         const float4 w4 = *reinterpret_cast<const float4*>(ss.pw + o + kb);
         const float4 d4 = *reinterpret_cast<const float4*>(ss.pd + o + kb);
