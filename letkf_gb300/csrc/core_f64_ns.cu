@@ -18,8 +18,12 @@
 //      takes the residual r to about max(1e-5 r, r^2): 1e-5 -> 1e-10 -> FP64
 //      rounding, two residuals for lambda_max / c up to about 100, three above.
 // The last residual is always FP64 against the FP64 A: FP32 decides how fast
-// the result is reached, not how good it is (error against 64-bit values
-// 5e-16 where the eigensolver form has 2e-15).
+// the result is reached.  The correction of at most 5e-10 that follows it is not
+// checked by another; measured against quadruple precision the result is no
+// further off than the eigensolver's at any conditioning (k = 40, geometric means
+// over 32 points, eigensolver / here: T 2.7e-16 / 2.8e-17 at lambda_max / c = 2,
+// 2.2e-15 / 6.9e-16 at 345, 9.8e-14 / 2.5e-14 at 8,400; wbar 7.1e-16 / 2.4e-16,
+// 8.7e-15 / 5.0e-15, 1.3e-13 / 1.3e-13).
 //
 // Bound: the FP64 pipe, 1.2 TFLOP/s on this chip against 75 in FP32, with a
 // 64-cycle latency.  The EISPACK form (core_f64.cu) walks its rotations on one
