@@ -8,6 +8,8 @@
 //    the relative-spread clip.
 //  * letkf_efso: observation sensitivity (gfs/letkf/letkf_tools.f90:547-679)
 //    over grid points with their local observation lists.
+#include <algorithm>
+
 #include "letkf_common.cuh"
 
 namespace letkf {
@@ -15,7 +17,7 @@ namespace letkf {
 constexpr int OSA_NT = 128;
 constexpr int OSA_T = 64;       // members and weights of a staged tile
 constexpr int OSA_LD = OSA_T + 1;
-constexpr int OSA_SMALL = 32;   // members of a warp's lanes
+constexpr int OSA_WARP = 128;   // members of the largest ensemble that a warp takes
 constexpr int EFSO_MAX_TERM = 8;
 constexpr int EFSO_MAX_NV = 16;
 constexpr int EFSO_MC = 16;     // members of a staged tile of 32 observations
@@ -105,36 +107,91 @@ __global__ void __launch_bounds__(OSA_NT) obs_analysis_kernel(int ne, int n, con
   }
 }
 
-// Ensembles of a warp's lanes or fewer: a warp per location, a lane per member on
-// its own row of trans (two lines), no barrier.  The sums are those of the kernel
-// above in the same order.  20,000 locations of k = 2 / 8 / 16 / 24 / 32: 92 / 99 /
-// 111 / 145 / 164 us there, 37 / 43 / 53 / 64 / 87 here; a CTA per location with a
-// thread per member, before the tile, 41 / 66 / 104 / 147.
-__global__ void __launch_bounds__(OSA_NT) obs_analysis_small_kernel(int ne, int n, const double* __restrict__ trans,
-                                                                     const double* __restrict__ ybar,
-                                                                     const double* __restrict__ hdxf, double alpha,
-                                                                     const int* __restrict__ mode, double q_sprd_max,
-                                                                     double* anal, double* amean) {
+// A warp per location, a lane per member (R of them) on its own rows of trans,
+// no barrier.  The sums are those of the kernel above in the same order.
+// A lane takes 64 consecutive bytes of its row at a time (VEC: by 16 bytes, rows
+// aligned), so that the line it is in the middle of stays in L1.  HBM for trans
+// bounds it, and the lines' way through L1 up to k = 32.  In us, a CTA per
+// location with a thread per member (before the tile) / the tile / here: 20,000
+// locations of k = 16 61 / 103 / 48, k = 32 132 / 156 / 68, k = 40 166 / 198 / 134, k =
+// 64 324 / 252 / 183, 8,000 of k = 100 242 / 269 / 234, 4,900 of k = 127 196 / 207 / 182.
+// From k = 65 a warp alone with its location takes longer than the tile's four
+// until the SMs are full of them: 600 locations of k = 100 21 / 21 / 27, 1,000 of k =
+// 96 44 / 32 / 27, of k = 101 37 / 39 / 35, of k = 127 47 / 54 / 56.
+template <int R, bool VEC>
+__global__ void __launch_bounds__(OSA_NT, 8) obs_analysis_warp_kernel(int ne, int n, const double* __restrict__ trans,
+                                                                      const double* __restrict__ ybar,
+                                                                      const double* __restrict__ hdxf, double alpha,
+                                                                      const int* __restrict__ mode, double q_sprd_max,
+                                                                      double* anal, double* amean) {
+  __shared__ __align__(16) double hs[OSA_NT / 32][32 * R];
   const int lane = threadIdx.x & 31, stride = gridDim.x * (OSA_NT / 32);
-  const bool on = lane < ne;
+  double* h = hs[threadIdx.x >> 5];
   for (int p = blockIdx.x * (OSA_NT / 32) + (threadIdx.x >> 5); p < n; p += stride) {
     const int md = mode ? mode[p] : 0;
-    const double yb = ybar[p], h = on ? hdxf[(size_t)p * ne + lane] : 0.0;
-    double a = yb + h, s = yb;
+    const double yb = ybar[p];
+    __syncwarp();
+    for (int m = lane; m < ne; m += 32) h[m] = hdxf[(size_t)p * ne + m];
+    __syncwarp();
+    double a[R], s = yb;
+#pragma unroll
+    for (int r = 0; r < R; r++) a[r] = yb + (lane + 32 * r < ne ? h[lane + 32 * r] : 0.0);
     if (md != 1) {
-      const double* w = trans + (size_t)p * ne * ne + (on ? lane : 0) * ne;
-      double v = 0.0;
-      for (int k = 0; k < ne; k++) v = fma(__shfl_sync(0xffffffffu, h, k), w[k], v);
-      if (alpha != 0.0) v = (1.0 - alpha) * v + alpha * h;
-      a = yb + v;
-      s = warp_sum(on ? a : 0.0) / (double)ne;
+      double t = 0.0;
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+        const int m = lane + 32 * r;
+        if (m >= ne) continue;
+        const double* w = trans + ((size_t)p * ne + m) * ne;
+        double v[2] = {0.0, 0.0};  // the even and odd 32s of the weights
+#pragma unroll
+        for (int q = 0; q < R; q++) {
+          const int ke = min(ne, 32 * q + 32);
+          int k = 32 * q;
+          for (; k + 8 <= ke; k += 8) {  // 64 bytes in flight
+            double x[8];
+#pragma unroll
+            for (int i = 0; i < 8; i += 2) {
+              if (VEC) {
+                const double2 u = *reinterpret_cast<const double2*>(w + k + i);
+                x[i] = u.x;
+                x[i + 1] = u.y;
+              } else {
+                x[i] = w[k + i];
+                x[i + 1] = w[k + i + 1];
+              }
+            }
+#pragma unroll
+            for (int i = 0; i < 8; i += 2) {
+              const double2 hk = *reinterpret_cast<const double2*>(h + k + i);
+              v[q & 1] = fma(hk.x, x[i], v[q & 1]);
+              v[q & 1] = fma(hk.y, x[i + 1], v[q & 1]);
+            }
+          }
+#pragma unroll 4
+          for (; k < ke; k++) v[q & 1] = fma(h[k], w[k], v[q & 1]);
+        }
+        double b = v[0] + v[1];
+        if (alpha != 0.0) b = (1.0 - alpha) * b + alpha * h[m];
+        a[r] = yb + b;
+        t = t + a[r];
+      }
+      s = warp_sum(t) / (double)ne;
       if (md == 2) {
-        const double sp = sqrt(warp_sum(on ? (a - s) * (a - s) : 0.0) / (double)(ne - 1)) / s;
-        if (sp > q_sprd_max) a = s + (a - s) * q_sprd_max / sp;
+        double sp = 0.0;
+#pragma unroll
+        for (int r = 0; r < R; r++)
+          if (lane + 32 * r < ne) sp = fma(a[r] - s, a[r] - s, sp);
+        sp = sqrt(warp_sum(sp) / (double)(ne - 1)) / s;
+        if (sp > q_sprd_max)
+#pragma unroll
+          for (int r = 0; r < R; r++) a[r] = s + (a[r] - s) * q_sprd_max / sp;
       }
     }
     if (amean && lane == 0) amean[p] = s;
-    if (on) anal[(size_t)p * ne + lane] = a;
+#pragma unroll
+    for (int r = 0; r < R; r++)
+      if (lane + 32 * r < ne) anal[(size_t)p * ne + lane + 32 * r] = a[r];
   }
 }
 
@@ -260,18 +317,20 @@ static int launch_efso(int ne, int npts, int nv, const EfsoTerms& tv, const int6
   return cuda_status(cudaGetLastError());
 }
 
+static int sm_count() {
+  int dev = 0, nsm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  return nsm;
+}
+
 __global__ void efso_sense_kernel(int64_t n, int nterm, const double* __restrict__ djdy,
                                   const double* __restrict__ obsdep, double* obsense) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) obsense[i] = djdy[i] * obsdep[i / nterm];
 }
 
-static int grid_for(int n) {
-  int dev = 0, nsm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  return n < nsm * 8 ? n : nsm * 8;
-}
+static int grid_for(int n) { return std::min(n, 8 * sm_count()); }
 
 static int have_device() {
   int nd = 0;
@@ -292,10 +351,14 @@ extern "C" int letkf_obs_analysis(int ne, int n, const double* trans, const doub
   if (ne < 2 || ne > 4096 || n < 0 || (n > 0 && (!trans || !ybar || !hdxf || !anal))) return LETKF_ERR_ARG;
   if (!have_device()) return LETKF_ERR_NOGPU;
   if (n == 0) return LETKF_OK;
-  if (ne <= OSA_SMALL) {
+  if (ne <= OSA_T || (ne <= OSA_WARP && n > 6 * sm_count())) {
+    const bool vec = ne % 2 == 0 && reinterpret_cast<uintptr_t>(trans) % 16 == 0;
+    auto kern = ne <= 32   ? (vec ? obs_analysis_warp_kernel<1, true> : obs_analysis_warp_kernel<1, false>)
+                : ne <= 64 ? (vec ? obs_analysis_warp_kernel<2, true> : obs_analysis_warp_kernel<2, false>)
+                           : (vec ? obs_analysis_warp_kernel<4, true> : obs_analysis_warp_kernel<4, false>);
     const int need = (int)(((int64_t)n + OSA_NT / 32 - 1) / (OSA_NT / 32));
-    obs_analysis_small_kernel<<<grid_for(need), OSA_NT, 0, (cudaStream_t)stream>>>(ne, n, trans, ybar, hdxf, relax_alpha,
-                                                                                    mode, q_sprd_max, anal, anal_mean);
+    kern<<<grid_for(need), OSA_NT, 0, (cudaStream_t)stream>>>(ne, n, trans, ybar, hdxf, relax_alpha, mode, q_sprd_max,
+                                                              anal, anal_mean);
     note_launch();
     return cuda_status(cudaGetLastError());
   }

@@ -254,3 +254,24 @@ def test_mean_weights_on_either_side_of_each_rule(cuda, ne, nv):
 @pytest.mark.parametrize("ne", [3, 8, 16, 17, 30, 32, 33])
 def test_obs_analysis_of_few_members(cuda, ne):
     test_obs_analysis_edges(cuda, ne)
+
+
+@pytest.mark.parametrize("ne", [33, 34, 40, 47, 64, 65, 66, 96, 97, 101, 127, 128])
+def test_obs_analysis_by_warps(cuda, ne):
+    """A warp per location, up to four members a lane, rows aligned or not; the
+    tile's sums in the same order, so few locations and many give the same bits."""
+    import torch
+
+    from letkf_gb300.core import obs_analysis
+
+    test_obs_analysis_edges(cuda, ne)
+    g = torch.Generator(device=cuda).manual_seed(ne)
+    r = lambda *s: torch.randn(*s, dtype=torch.float64, device=cuda, generator=g)
+    n = 1100
+    tr, h, y = r(n, ne, ne) / ne, r(n, ne), r(n) + 4.0
+    mode = (torch.arange(n, device=cuda) % 3).to(torch.int32)
+    anal, mean = obs_analysis(tr, y, h, 0.25, mode, 0.1)
+    for p in (0, 1, 1000):
+        q = slice(p, p + 100)
+        a, m = obs_analysis(tr[q].contiguous(), y[q].contiguous(), h[q].contiguous(), 0.25, mode[q].contiguous(), 0.1)
+        assert torch.equal(a, anal[q]) and torch.equal(m, mean[q])
