@@ -20,7 +20,8 @@ constexpr int OSA_LD = OSA_T + 1;
 constexpr int OSA_WARP = 128;   // members of the largest ensemble that a warp takes
 constexpr int EFSO_MAX_TERM = 8;
 constexpr int EFSO_MAX_NV = 16;
-constexpr int EFSO_MC = 16;     // members of a staged tile of 32 observations
+constexpr int EFSO_MC = 16;     // members of a staged tile of 32 observations, or half of them
+constexpr int EFSO_FEW = 8;     // members whose rows the lanes read by themselves
 constexpr int EFSO_GROUP = 8;   // grid points of a CTA at most
 
 // One CTA per observation location.  Bound: HBM for trans (k^2 doubles, read
@@ -211,7 +212,7 @@ struct EfsoTerms {
 // 2.55 ms, now 0.78 (FP64 pipe 69 % busy).  (rloc and rdiag loaded ahead of the
 // sums hold registers: three terms take 90 instead of 80, one CTA an SM fewer, up
 // to 20 % more time where lists are even.)
-template <int NTERM>
+template <int NTERM, int MC>
 __global__ void __launch_bounds__(OSA_NT) efso_djdy_kernel(int ne, int npts, int nv, int group,
                                                             const __grid_constant__ EfsoTerms tv,
                                                             const int64_t* __restrict__ offs,
@@ -221,10 +222,10 @@ __global__ void __launch_bounds__(OSA_NT) efso_djdy_kernel(int ne, int npts, int
                                                             const double* __restrict__ hdxa,
                                                             const double* __restrict__ fcst,
                                                             const double* __restrict__ fcer, double* djdy) {
-  extern __shared__ double w1[];  // [group][NTERM][ne], then the warps' tiles [EFSO_MC][33]
+  extern __shared__ double w1[];  // [group][NTERM][ne], then the warps' tiles [MC][33]
   __shared__ int64_t lo[EFSO_GROUP + 1];
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  double* tile = w1 + (size_t)group * NTERM * ne + wid * EFSO_MC * 33;
+  double* tile = w1 + (size_t)group * NTERM * ne + wid * MC * 33;
   const int ngroup = (npts + group - 1) / group;
   for (int g = blockIdx.x; g < ngroup; g += gridDim.x) {
     const int p0 = g * group, np = min(group, npts - p0);
@@ -256,38 +257,82 @@ __global__ void __launch_bounds__(OSA_NT) efso_djdy_kernel(int ne, int npts, int
       double acc[NTERM];
 #pragma unroll
       for (int i = 0; i < NTERM; i++) acc[i] = 0.0;
-      // rows 2 r and 2 r + 1 of the tile by the two half warps, lane % 16 the member
-      double nx[16];
-      auto load = [&](int m0) {
+      double wt = 0.0;
+      if constexpr (MC == 1) {
+        wt = on ? rloc[l] / rdiag[l] : 0.0;
+        const double* row = hdxa + (size_t)(on ? ob : 0) * ne;
+#pragma unroll 2
+        for (int m = 0; m < ne; m++) {
+          const double h = on ? row[m] : 0.0;
 #pragma unroll
-        for (int r = 0; r < 16; r++) {
-          const int o = __shfl_sync(0xffffffffu, ob, 2 * r + (lane >> 4));
-          const int m = m0 + (lane & 15);
-          nx[r] = (o >= 0 && m < ne) ? hdxa[(size_t)o * ne + m] : 0.0;
+          for (int i = 0; i < NTERM; i++) acc[i] = fma(w[i * ne + m], h, acc[i]);
         }
-      };
-      load(0);
-      for (int m0 = 0; m0 < ne; m0 += EFSO_MC) {
-        __syncwarp();
+      } else {
+        // RP rows of the tile at a time by MC lanes each, a lane a member
+        constexpr int RP = 32 / MC;
+        double nx[MC];
+        auto load = [&](int m0) {
 #pragma unroll
-        for (int r = 0; r < 16; r++) tile[(lane & 15) * 33 + 2 * r + (lane >> 4)] = nx[r];
-        __syncwarp();
-        if (m0 + EFSO_MC < ne) load(m0 + EFSO_MC);
-        const int nm = min(EFSO_MC, ne - m0);
+          for (int r = 0; r < MC; r++) {
+            const int o = __shfl_sync(0xffffffffu, ob, RP * r + lane / MC);
+            const int m = m0 + lane % MC;
+            nx[r] = (o >= 0 && m < ne) ? hdxa[(size_t)o * ne + m] : 0.0;
+          }
+        };
+        load(0);
+        for (int m0 = 0; m0 < ne; m0 += MC) {
+          __syncwarp();
+#pragma unroll
+          for (int r = 0; r < MC; r++) tile[(lane % MC) * 33 + RP * r + lane / MC] = nx[r];
+          __syncwarp();
+          if (m0 + MC < ne) load(m0 + MC);
+          const int nm = min(MC, ne - m0);
 #pragma unroll 4
-        for (int m = 0; m < nm; m++) {
-          const double h = tile[m * 33 + lane];
+          for (int m = 0; m < nm; m++) {
+            const double h = tile[m * 33 + lane];
 #pragma unroll
-          for (int i = 0; i < NTERM; i++) acc[i] = fma(w[i * ne + m0 + m], h, acc[i]);
+            for (int i = 0; i < NTERM; i++) acc[i] = fma(w[i * ne + m0 + m], h, acc[i]);
+          }
         }
       }
       if (on) {
-        const double s = rloc[l] / rdiag[l];
+        if (MC != 1) wt = rloc[l] / rdiag[l];
 #pragma unroll
-        for (int i = 0; i < NTERM; i++) atomicAdd(&djdy[(size_t)ob * NTERM + i], acc[i] * s);
+        for (int i = 0; i < NTERM; i++) atomicAdd(&djdy[(size_t)ob * NTERM + i], acc[i] * wt);
       }
     }
   }
+}
+
+static int sm_count() {
+  int dev = 0, nsm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  return nsm;
+}
+
+template <int NTERM>
+static size_t efso_smem(int ne, int group, int mc) {
+  return sizeof(double) * ((size_t)group * NTERM * ne + (mc > 1 ? (OSA_NT / 32) * mc * 33 : 0));
+}
+
+template <int NTERM, int MC>
+static int launch_efso_as(int ne, int npts, int nv, int group, const EfsoTerms& tv, const int64_t* offs, const int* idx,
+                       const double* rdiag, const double* rloc, const double* hdxa, const double* fcst,
+                       const double* fcer, double* djdy, cudaStream_t s) {
+  const size_t smem = efso_smem<NTERM>(ne, group, MC);
+  if (smem > 48 * 1024) {
+    const cudaError_t e =
+        cudaFuncSetAttribute(efso_djdy_kernel<NTERM, MC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return cuda_status(e);
+  }
+  const int nsm = sm_count();
+  const int ngroup = (npts + group - 1) / group;
+  const int grid = ngroup < nsm * 8 ? ngroup : nsm * 8;
+  efso_djdy_kernel<NTERM, MC><<<grid, OSA_NT, smem, s>>>(ne, npts, nv, group, tv, offs, idx, rdiag, rloc, hdxa, fcst,
+                                                     fcer, djdy);
+  note_launch();
+  return cuda_status(cudaGetLastError());
 }
 
 template <int NTERM>
@@ -296,32 +341,21 @@ static int launch_efso(int ne, int npts, int nv, const EfsoTerms& tv, const int6
                        const double* fcer, double* djdy, cudaStream_t s) {
   const size_t one = sizeof(double) * (size_t)NTERM * ne;
   // as many points as 24 KB of work1 hold, fewer where that would leave SMs without a group
-  int dev = 0, nsm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  const int nsm = sm_count();
   int group = (int)(24 * 1024 / one);
   group = group < 1 ? 1 : group > EFSO_GROUP ? EFSO_GROUP : group;
   const int fill = npts / (nsm * 8);
   if (group > fill) group = fill < 1 ? 1 : fill;
-  const size_t smem = group * one + sizeof(double) * (OSA_NT / 32) * EFSO_MC * 33;
-  if (smem > 48 * 1024) {
-    const cudaError_t e =
-        cudaFuncSetAttribute(efso_djdy_kernel<NTERM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return cuda_status(e);
-  }
-  const int ngroup = (npts + group - 1) / group;
-  const int grid = ngroup < nsm * 8 ? ngroup : nsm * 8;
-  efso_djdy_kernel<NTERM><<<grid, OSA_NT, smem, s>>>(ne, npts, nv, group, tv, offs, idx, rdiag, rloc, hdxa, fcst,
-                                                     fcer, djdy);
-  note_launch();
-  return cuda_status(cudaGetLastError());
-}
-
-static int sm_count() {
-  int dev = 0, nsm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  return nsm;
+  // no tile where a row is half a line or less (30,000 points with 50 entries, k = 2 / 8,
+  // 8 terms: before tiles 156 / 339 us, with one 171 / 283, here 118 / 241)
+  if (ne <= EFSO_FEW)
+    return launch_efso_as<NTERM, 1>(ne, npts, nv, group, tv, offs, idx, rdiag, rloc, hdxa, fcst, fcer, djdy, s);
+  // half a tile where a third CTA shares the SM then: k = 1024, 8 terms, 3,000 points with 50 entries 5.63 -> 3.70
+  // ms (4.18 without tiles, three CTAs an SM)
+  auto per_sm = [&](int mc) { return 227 * 1024 / (efso_smem<NTERM>(ne, group, mc) + 1024); };
+  if (per_sm(EFSO_MC) < 3 && per_sm(EFSO_MC / 2) > per_sm(EFSO_MC))
+    return launch_efso_as<NTERM, EFSO_MC / 2>(ne, npts, nv, group, tv, offs, idx, rdiag, rloc, hdxa, fcst, fcer, djdy, s);
+  return launch_efso_as<NTERM, EFSO_MC>(ne, npts, nv, group, tv, offs, idx, rdiag, rloc, hdxa, fcst, fcer, djdy, s);
 }
 
 __global__ void efso_sense_kernel(int64_t n, int nterm, const double* __restrict__ djdy,

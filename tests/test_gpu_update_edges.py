@@ -275,3 +275,10 @@ def test_obs_analysis_by_warps(cuda, ne):
         q = slice(p, p + 100)
         a, m = obs_analysis(tr[q].contiguous(), y[q].contiguous(), h[q].contiguous(), 0.25, mode[q].contiguous(), 0.1)
         assert torch.equal(a, anal[q]) and torch.equal(m, mean[q])
+
+
+@pytest.mark.parametrize("ne,npts,nterm", [(3, 2500, 3), (8, 40, 1), (8, 1300, 8), (9, 40, 8), (900, 5, 8), (1024, 7, 8),
+                                           (1024, 4, 7)])
+def test_efso_of_few_and_of_many_members(cuda, ne, npts, nterm):
+    """No tile up to eight members, half a tile where memory is short."""
+    test_efso_edges(cuda, ne, npts, nterm)
