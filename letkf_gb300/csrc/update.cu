@@ -502,12 +502,146 @@ static int launch_update_as(int ne, int npts, int p0, int cnt, int nv, const dou
   return cuda_status(cudaGetLastError());
 }
 
+// Ensembles of two to eight members: a thread per point and variable with its
+// members in registers; no barrier, no shared memory.  A CTA per point has eight
+// of its 128 lanes busy per variable, and its passes and barriers to pay for.
+// Bound: FP64 and, with many variables, the reads of each point's weights by
+// every one of them (L1).  100,000 points in us, a thread per output of a CTA per
+// point / the kernels above / here: 2 members, 20 variables, mode 0 with a beta
+// array 311 / 597 / 93; 4 members, 20 variables, plain with mean weights 295 / 316 /
+// 185, RTPS 5,509 / 1,551 / 385; 8 members, 5 variables, RTPP 737 / 404 / 144.  The plain
+// update with merged weights has the point kernel from 5 members on where the
+// variables are more than 10 (5 members: 5 variables 133 there / 72 here, 20
+// 238 / 277; 8 members 216 / 127, 363 / 477).  The operations are those of the
+// kernels above in the same order (sums over the members as their lanes add
+// them), so the results are the same bits.
+constexpr int UPD_TINY = 8;       // members, at most
+constexpr int UPD_TINY_MERGED = 4;  // and with merged weights and more than UPD_TINY_NV variables
+constexpr int UPD_TINY_NV = 10;
+constexpr int UPT_NT = 128;
+
+// x[0] + .. + x[N-1] as the butterfly of eight lanes, or of a warp, adds them
+template <int N>
+__device__ __forceinline__ double upt_sum(const double (&x)[N]) {
+  double t[N < 4 ? N : 4];
+#pragma unroll
+  for (int i = 0; i < N && i < 4; i++) t[i] = i + 4 < N ? x[i] + x[i + 4 < N ? i + 4 : 0] : x[i];
+  if constexpr (N == 2) return t[0] + t[1];
+  if constexpr (N == 3) return (t[0] + t[2]) + t[1];
+  if constexpr (N >= 4) return (t[0] + t[2]) + (t[1] + t[3]);
+}
+
+template <int N, int MODE>
+__global__ void __launch_bounds__(UPT_NT) update_tiny_kernel(int npts, int p0, int cnt, int nv,
+                                                             const double* __restrict__ xb,
+                                                             const double* __restrict__ trans,
+                                                             const double* __restrict__ transm,
+                                                             const double* __restrict__ pao, RelaxArgs r, double* xa) {
+  const int64_t total = (int64_t)cnt * nv;
+  for (int64_t t = (int64_t)blockIdx.x * UPT_NT + threadIdx.x; t < total; t += (int64_t)gridDim.x * UPT_NT) {
+    const int v = (int)(t / cnt), pl = (int)(t - (int64_t)v * cnt);
+    const size_t at = ((size_t)v * npts + p0 + pl) * N;
+    double x[N], y[N], s[N];
+#pragma unroll
+    for (int m = 0; m < N; m++) x[m] = xb[at + m];
+    double mean = x[0];
+#pragma unroll
+    for (int m = 1; m < N; m++) mean = mean + x[m];
+    mean = mean / (double)N;
+#pragma unroll
+    for (int m = 0; m < N; m++) x[m] = x[m] - mean;
+    double tx = 0.0;
+    if (transm) {
+#pragma unroll
+      for (int m = 0; m < N; m++) s[m] = __dmul_rn(x[m], transm[(size_t)pl * N + m]);
+      tx = upt_sum<N>(s);
+    }
+    const double b = r.beta ? r.beta[(size_t)v * npts + p0 + pl] : 1.0;
+    double fac = 1.0;
+    if (MODE == 2) {
+      const double* P = pao + (size_t)pl * N * N;
+#pragma unroll
+      for (int i = 0; i < N; i++) {  // pairs (i, i + d mod N), as the general kernel's D
+        double a = 0.0;
+#pragma unroll
+        for (int d = 0; 2 * d <= N; d++) {
+          const int j = (i + d) % N;
+          if (2 * d == N && i > j) continue;
+          const double dd = d == 0 ? P[i * N + i] : P[i * N + j] + P[j * N + i];
+          a = fma(dd, x[j], a);
+        }
+        s[i] = __dmul_rn(a, x[i]);
+      }
+      const double va = upt_sum<N>(s);
+#pragma unroll
+      for (int i = 0; i < N; i++) s[i] = __dmul_rn(x[i], x[i]);
+      const double vg = upt_sum<N>(s);
+      if (b != 0.0 && vg > 0.0 && va > 0.0) fac = r.alpha * sqrt(vg / (va * (double)(N - 1))) - r.alpha + 1.0;
+      if (r.rtps_infl) r.rtps_infl[(size_t)v * npts + p0 + pl] = fac;
+    }
+    const double* W = trans + (size_t)pl * N * N;  // W(k, m) at m N + k
+    const bool plain = MODE == 0 && b == 1.0;
+#pragma unroll
+    for (int m = 0; m < N; m++) {
+      double a = plain ? (transm ? mean + tx : mean) : 0.0;
+#pragma unroll
+      for (int k = 0; k < N; k++) a = fma(x[k], W[m * N + k], a);
+      if (!plain) {
+        if (MODE == 1) a = (1.0 - r.alpha) * a + r.alpha * x[m];
+        if (MODE == 2) a = fac * a;
+        if (transm) a = a + tx;
+        if (r.beta) a = b == 0.0 ? x[m] : b == 1.0 ? a : b * a + (1.0 - b) * x[m];
+        a = mean + a;
+      }
+      y[m] = a;
+    }
+    if (r.q_sprd_max > 0.0 && v == r.q_var) {
+      const double qm = upt_sum<N>(y) / (double)N;
+#pragma unroll
+      for (int m = 0; m < N; m++) s[m] = __dmul_rn(y[m] - qm, y[m] - qm);
+      const double sp = sqrt(upt_sum<N>(s) / (double)(N - 1)) / qm;
+      const double f = r.q_sprd_max / sp;
+#pragma unroll
+      for (int m = 0; m < N; m++)
+        if (sp > r.q_sprd_max) y[m] = qm + (y[m] - qm) * f;
+    }
+#pragma unroll
+    for (int m = 0; m < N; m++) xa[at + m] = y[m];
+  }
+}
+
+template <int MODE>
+static int launch_update_tiny(int ne, int npts, int p0, int cnt, int nv, const double* xb, const double* trans,
+                              const double* transm, const double* pao, const RelaxArgs& r, double* xa,
+                              cudaStream_t stream) {
+  decltype(&update_tiny_kernel<2, MODE>) kern = nullptr;
+  switch (ne) {
+    case 2: kern = update_tiny_kernel<2, MODE>; break;
+    case 3: kern = update_tiny_kernel<3, MODE>; break;
+    case 4: kern = update_tiny_kernel<4, MODE>; break;
+    case 5: kern = update_tiny_kernel<5, MODE>; break;
+    case 6: kern = update_tiny_kernel<6, MODE>; break;
+    case 7: kern = update_tiny_kernel<7, MODE>; break;
+    case 8: kern = update_tiny_kernel<8, MODE>; break;
+  }
+  const int64_t need = ((int64_t)cnt * nv + UPT_NT - 1) / UPT_NT;
+  kern<<<(unsigned)std::min<int64_t>(need, 1 << 20), UPT_NT, 0, stream>>>(npts, p0, cnt, nv, xb, trans, transm, pao, r,
+                                                                          xa);
+  note_launch();
+  return cuda_status(cudaGetLastError());
+}
+
 static int launch_update(int ne, int npts, int p0, int cnt, int nv, const double* xb, const double* trans,
                          const double* transm, const double* pao, const RelaxArgs& r, double* xa,
                          cudaStream_t stream) {
 #define UPD_AS(MODE)                                                                                             \
   return r.beta ? launch_update_as<MODE, true>(ne, npts, p0, cnt, nv, xb, trans, transm, pao, r, xa, stream) \
                 : launch_update_as<MODE, false>(ne, npts, p0, cnt, nv, xb, trans, transm, pao, r, xa, stream)
+  if (ne <= UPD_TINY) {
+    if (r.mode == 2) return launch_update_tiny<2>(ne, npts, p0, cnt, nv, xb, trans, transm, pao, r, xa, stream);
+    if (r.mode == 1) return launch_update_tiny<1>(ne, npts, p0, cnt, nv, xb, trans, transm, pao, r, xa, stream);
+    return launch_update_tiny<0>(ne, npts, p0, cnt, nv, xb, trans, transm, pao, r, xa, stream);
+  }
   if (r.mode == 2) UPD_AS(2);
   if (r.mode == 1) UPD_AS(1);
   UPD_AS(0);
@@ -519,6 +653,9 @@ int launch_update_f64_range(int ne, int npts_total, int p0, int cnt, int nv, con
   if (ne < 2 || npts_total < 0 || p0 < 0 || cnt < 0 || p0 + cnt > npts_total || nv < 1) return LETKF_ERR_ARG;
   if (ne > LETKF_MAX_NE) return LETKF_ERR_CAPACITY;
   if (cnt == 0) return LETKF_OK;
+  const RelaxArgs plain = {0, 0.0, nullptr, -1, 0.0, nullptr};
+  if (ne <= (transm || nv <= UPD_TINY_NV ? UPD_TINY : UPD_TINY_MERGED))
+    return launch_update(ne, npts_total, p0, cnt, nv, xb, trans, transm, nullptr, plain, xa, stream);
   const bool vec = ne % 2 == 0 && reinterpret_cast<uintptr_t>(trans) % 16 == 0;
 #define UPR_LAUNCH(NVT)                                                                                 \
   return vec ? launch_update_rows<NVT, true>(ne, npts_total, p0, cnt, xb, trans, transm, xa, stream) \
@@ -558,8 +695,7 @@ int launch_update_f64_range(int ne, int npts_total, int p0, int cnt, int nv, con
     if (transm) return launch_update_point<true>(ne, npts_total, p0, cnt, nv, xb, trans, transm, xa, stream);
     return launch_update_point<false>(ne, npts_total, p0, cnt, nv, xb, trans, transm, xa, stream);
   }
-  const RelaxArgs r = {0, 0.0, nullptr, -1, 0.0, nullptr};
-  return launch_update(ne, npts_total, p0, cnt, nv, xb, trans, transm, nullptr, r, xa, stream);
+  return launch_update(ne, npts_total, p0, cnt, nv, xb, trans, transm, nullptr, plain, xa, stream);
 }
 
 int launch_update_f64(int ne, int npts, int nv, const double* xb, const double* trans, const double* transm,

@@ -282,3 +282,14 @@ def test_obs_analysis_by_warps(cuda, ne):
 def test_efso_of_few_and_of_many_members(cuda, ne, npts, nterm):
     """No tile up to eight members, half a tile where memory is short."""
     test_efso_edges(cuda, ne, npts, nterm)
+
+
+@pytest.mark.parametrize("ne,nv", [(2, 1), (2, 41), (3, 6), (4, 11), (5, 1), (5, 17), (6, 3), (7, 16), (8, 10), (8, 11),
+                                   (9, 10)])
+@pytest.mark.parametrize("mode", [0, 1, 2])
+def test_small_ensembles_by_threads(cuda, ne, nv, mode):
+    """A thread per point and variable up to eight members, either side of its rules."""
+    test_relaxed_update_edges(cuda, ne, nv, mode, nv - 1)
+    for merged in (True, False):
+        test_update_f64_edges(cuda, ne, nv, merged, 301)
+        test_beta_of_one_is_the_plain_update_bit_for_bit(cuda, ne, nv, merged)
