@@ -678,7 +678,20 @@ int launch_update_f64_range(int ne, int npts_total, int p0, int cnt, int nv, con
                    : ne <= 54 ? 1
                    : transm   ? (ne <= 64 ? (ne % 16 ? 3 : 6) : ne <= 71 ? 2 : ne <= 79 ? 5 : 6)
                               : (ne <= 79 ? (ne % 16 ? 2 : 4) : ne <= 82 ? 5 : 6);
-  if (nv <= rows) {
+  // Few points: a warp takes the same time for the rows of one point as of all
+  // that fit, a CTA per point divides them, so up to some waves of its resident
+  // CTAs the latter is faster.  rows / point, merged weights (before either) in us: n =
+  // 80, 3 variables, 600 points 39 / 33 (50), 1,000 58 / 60 (97); n = 100, 1 variable,
+  // 300 27 / 17 (19), 450 28 / 31 (33); 6 variables, 1 point 113 / 33 (33), 600 115 /
+  // 80 (82); n = 128, 1 variable, 150 33 / 23 (23), 300 33 / 41 (41), 3 variables, 300
+  // 76 / 66 (78), 450 76 / 97 (115); rows that are not 16-byte aligned take longer: n =
+  // 127, 1 variable, 450 52 / 50 (52), 600 52 / 69 (76).
+  int dev = 0, nsm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  const int resident = (int)(227 * 1024 / (sizeof(double) * (size_t)ne * (ne + nv) + 1024));
+  const int waves = !vec ? 3 : nv > 2 ? 2 : 1;
+  if (nv <= rows && cnt > nsm * std::min(4, waves * resident)) {
     if (nv == 1) UPR_LAUNCH(1);
     if (nv == 2) UPR_LAUNCH(2);
     if (nv == 3) UPR_LAUNCH(3);

@@ -293,3 +293,29 @@ def test_small_ensembles_by_threads(cuda, ne, nv, mode):
     for merged in (True, False):
         test_update_f64_edges(cuda, ne, nv, merged, 301)
         test_beta_of_one_is_the_plain_update_bit_for_bit(cuda, ne, nv, merged)
+
+
+@pytest.mark.parametrize("ne,nv", [(9, 1), (20, 2), (24, 3), (32, 4), (54, 1), (63, 2), (64, 4), (82, 5), (101, 1),
+                                   (101, 6), (127, 3), (128, 1), (128, 3), (128, 6)])
+@pytest.mark.parametrize("merged", [True, False])
+def test_few_points_and_many_have_the_same_bits(cuda, ne, nv, merged):
+    """Batches of rows from a number of points on, a CTA per point below it."""
+    import torch
+
+    from letkf_gb300.core import update_f64
+
+    g = torch.Generator(device=cuda).manual_seed(ne + nv)
+    r = lambda *s: torch.randn(*s, dtype=torch.float64, device=cuda, generator=g)
+    npts = 701
+    w, xb = r(npts, ne, ne) / ne, r(nv, npts, ne) + 3.0
+    tm = None if merged else r(npts, ne) * 0.1
+    xa = update_f64(xb, w, tm)
+    for p in (0, 1, 131, 700):
+        q = slice(p, min(p + 130, npts))
+        part = update_f64(xb[:, q].contiguous(), w[q].contiguous(), None if merged else tm[q].contiguous())
+        assert torch.equal(part, xa[:, q])
+    x, m = xb[:, :50].cpu().numpy(), xb[:, :50].mean(-1, keepdim=True).cpu().numpy()
+    want = m + np.einsum("vpk,pmk->vpm", x - m, w[:50].cpu().numpy())
+    if not merged:
+        want = want + np.einsum("vpk,pk->vp", x - m, tm[:50].cpu().numpy())[..., None]
+    _close(xa[:, :50].cpu().numpy(), want)
