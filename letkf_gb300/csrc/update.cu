@@ -352,9 +352,13 @@ __global__ void __launch_bounds__(UPD_NT) update_point_kernel(int n, int npts, i
 template <bool TM>
 static int launch_update_point(int ne, int npts, int p0, int cnt, int nv, const double* xb, const double* trans,
                                const double* transm, double* xa, cudaStream_t stream) {
-  // a pass of 16 variables, or of 1,024 outputs where that is more
-  const int vc = std::min(nv, std::max(UPD_VC, 1024 / ne));
-  const size_t smem = sizeof(double) * ((size_t)ne * (ne | 1) + (size_t)vc * ne + 2 * vc);
+  // a pass of 16 variables, or of 1,024 outputs where that is more; all of them where no fewer CTAs share an SM then
+  // (k = 100, 20 variables, merged, 3,000 points: 1,250 us in passes of 16 and 4, 1,163 in one)
+  auto bytes = [&](int vc) { return sizeof(double) * ((size_t)ne * (ne | 1) + (size_t)vc * ne + 2 * vc); };
+  auto per_sm = [&](int vc) { return 227 * 1024 / (bytes(vc) + 1024); };
+  int vc = std::min(nv, std::max(UPD_VC, 1024 / ne));
+  if (nv <= 2 * UPD_VC && per_sm(nv) == per_sm(vc)) vc = nv;
+  const size_t smem = bytes(vc);
   auto kern = update_point_kernel<TM>;
   const cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (err != cudaSuccess) return cuda_status(err);

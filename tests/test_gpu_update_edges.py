@@ -319,3 +319,9 @@ def test_few_points_and_many_have_the_same_bits(cuda, ne, nv, merged):
     if not merged:
         want = want + np.einsum("vpk,pk->vp", x - m, tm[:50].cpu().numpy())[..., None]
     _close(xa[:, :50].cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("ne,nv", [(60, 17), (72, 32), (90, 20), (100, 20), (100, 33), (127, 17)])
+def test_more_variables_than_a_pass(cuda, ne, nv):
+    for merged in (True, False):
+        test_update_f64_edges(cuda, ne, nv, merged, 19)
