@@ -314,6 +314,17 @@ __device__ bool mn_newton_schulz(float* Y, float* Z, float* T, float* red, int t
   return false;
 }
 
+// A point that the iteration is not tried for leaves its Gram matrix (lower
+// triangle), b, p1 and p3 (above the diagonal) in its place in trans: the
+// eigensolver forming them again took up to 18 % of small batches with long
+// lists (1,000 points of k = 20 with 300 to 500 observations, three in ten left
+// to it: 521 us with one kernel for both, 613 with the Gram twice, 538 so).
+constexpr int MN_PENDING_GRAM = -LETKF_PENDING;  // of status, until the eigensolver's launch
+constexpr int MN_GRAM_MIN = 5;  // fewest members whose rows 0 and 1 hold the n + 2 values above the diagonal
+
+// place of value e < n + 2 above the diagonal: row 0 from column 1, row 1 from column 2
+__device__ __forceinline__ int mn_spare(int n, int e) { return e < n - 1 ? 1 + e : e + 3; }
+
 template <int NP>
 __global__ void __launch_bounds__(Mn<NP>::TP* Mn<NP>::PPC, MnCfg<NP>::MINB) core_mixed_ns_kernel(
     int n, int npts, const int64_t* __restrict__ offs, const float* __restrict__ rows,
@@ -434,6 +445,7 @@ __global__ void __launch_bounds__(Mn<NP>::TP* Mn<NP>::PPC, MnCfg<NP>::MINB) core
     const double trace = (double)mn_sum32<NP, (NP <= 32 ? 32 : NP <= 64 ? 64 : 128)>(g, 0.f);
     mn_sync<NP>();
     bool ok = c > 0.f && trace < 1.0e6 * (double)c;
+    const bool tried = ok;
     float s = 1.f;
     if (ok) {
       // s = min(Gershgorin, Frobenius) >= lambda_max of the matrix padded to NV
@@ -458,7 +470,16 @@ __global__ void __launch_bounds__(Mn<NP>::TP* Mn<NP>::PPC, MnCfg<NP>::MINB) core
       ok = mn_newton_schulz<NP>(Y, Z, T, red, tp, 0.9f * c * inv_s, c * inv_s, NV - NP);
     }
     if (!ok) {  // uniform over the point's threads: left to the eigensolver
-      if (tp == 0) status[p] = LETKF_PENDING;
+      // with its sums, where the iteration has not overwritten them
+      const bool gram = n >= MN_GRAM_MIN && !tried;
+      if (gram) {
+        for (int idx = tp; idx < n * n; idx += TP) {
+          const int i = idx / n, j = idx - i * n;
+          if (j <= i) Tp[idx] = i == j ? g[i] : Y[i * NP + j];
+        }
+        for (int e = tp; e < n + 2; e += TP) Tp[mn_spare(n, e)] = e < n ? bv[e] : e == n ? p1 : p3;
+      }
+      if (tp == 0) status[p] = gram ? MN_PENDING_GRAM : LETKF_PENDING;
       mn_sync<NP>();
       continue;
     }
@@ -505,33 +526,47 @@ __global__ void __launch_bounds__(MixedCfg<NP>::NT) core_mixed_kernel(
   extern __shared__ __align__(16) float sm[];
   const int tid = threadIdx.x;
   for (int p = blockIdx.x; p < npts; p += gridDim.x) {
-    if (status[p] != LETKF_PENDING) continue;
+    const int pending = status[p];
+    if (pending != LETKF_PENDING && pending != MN_PENDING_GRAM) continue;
     __syncthreads();  // every thread has read the status before it is set
     const int64_t r0 = offs[p];
     const int L = (int)(offs[p + 1] - r0);
     double infl = parm_infl[p];
     float* T = trans + (size_t)p * n * n;
     GramAcc<NP> acc;
-    acc.zero();
-    for (int c0 = 0; c0 < L; c0 += S::CH) {
-      const int nr = min(S::CH, L - c0);
-      __syncthreads();
-      for (int t = tid; t < S::CH * NP; t += C::NT) {
-        const int r = t / NP, m = t - r * NP;
-        sm[S::Y + t] = (r < nr && m < n) ? rows[(size_t)(r0 + c0 + r) * n + m] : 0.f;
+    double trace;
+    if (pending == MN_PENDING_GRAM) {
+      for (int idx = tid; idx < NP * NP; idx += C::NT) {
+        const int i = idx / NP, j = idx - i * NP;
+        sm[S::A + idx] = i < n && j < n ? T[i < j ? j * n + i : i * n + j] : 0.f;
       }
-      if (tid < nr) {
-        const float rd = rdiag[r0 + c0 + tid], rl = rloc[r0 + c0 + tid];
-        sm[S::WR + tid] = rdiag_wloc ? 1.f / rd : rl / rd;
-        sm[S::DR + tid] = dep[r0 + c0 + tid];
-        sm[S::RL + tid] = rl;
+      for (int i = tid; i < NP; i += C::NT) sm[S::B + i] = i < n ? T[mn_spare(n, i)] : 0.f;
+      acc.p1 = T[mn_spare(n, n)];
+      acc.p3 = T[mn_spare(n, n + 1)];
+      __syncthreads();
+      trace = gram_trace<NP>(sm);
+    } else {
+      acc.zero();
+      for (int c0 = 0; c0 < L; c0 += S::CH) {
+        const int nr = min(S::CH, L - c0);
+        __syncthreads();
+        for (int t = tid; t < S::CH * NP; t += C::NT) {
+          const int r = t / NP, m = t - r * NP;
+          sm[S::Y + t] = (r < nr && m < n) ? rows[(size_t)(r0 + c0 + r) * n + m] : 0.f;
+        }
+        if (tid < nr) {
+          const float rd = rdiag[r0 + c0 + tid], rl = rloc[r0 + c0 + tid];
+          sm[S::WR + tid] = rdiag_wloc ? 1.f / rd : rl / rd;
+          sm[S::DR + tid] = dep[r0 + c0 + tid];
+          sm[S::RL + tid] = rl;
+        }
+        __syncthreads();
+        for (int t = tid; t < nr * NP; t += C::NT) sm[S::YW + t] = sm[S::Y + t] * sm[S::WR + t / NP];
+        __syncthreads();
+        gram_chunk<NP>(sm, nr, acc);
       }
-      __syncthreads();
-      for (int t = tid; t < nr * NP; t += C::NT) sm[S::YW + t] = sm[S::Y + t] * sm[S::WR + t / NP];
-      __syncthreads();
-      gram_chunk<NP>(sm, nr, acc);
+      trace = gram_finish<NP>(sm, acc);
     }
-    const double trace = gram_finish<NP>(sm, acc);
     if (minfl > 0.0 && infl < minfl) infl = minfl;
     const float c = (float)((double)(n - 1) / infl);
     for (int i = tid; i < NP; i += C::NT) sm[S::A + i * NP + i] += c;

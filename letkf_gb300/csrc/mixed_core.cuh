@@ -124,6 +124,16 @@ __device__ __forceinline__ void gram_chunk(const float* sm, int nr, GramAcc<NP>&
   }
 }
 
+// trace of sm[A] in every thread
+template <int NP>
+__device__ __forceinline__ double gram_trace(float* sm) {
+  using C = MixedCfg<NP>;
+  using S = MixedSmem<NP>;
+  float tr = 0.f;
+  for (int i = threadIdx.x; i < NP; i += C::NT) tr += sm[S::A + i * NP + i];
+  return (double)block_sum<float, C::NT>(tr, sm + S::RED);
+}
+
 // Write the Gram tiles into sm[A] (symmetrised from the lower triangle), the
 // departure product into sm[B], reduce the inflation sums into acc.p1 / acc.p3
 // of every thread, and return trace(Gram) in FP64 (all threads).
@@ -152,13 +162,10 @@ __device__ __forceinline__ double gram_finish(float* sm, GramAcc<NP>& acc) {
     const int lo = i < j ? i : j, hi = i < j ? j : i;
     A[lo * NP + hi] = A[hi * NP + lo];
   }
-  float tr = 0.f;
-  for (int i = tid; i < NP; i += C::NT) tr += A[i * NP + i];
-  float* red = sm + S::RED;
-  const float trace = block_sum<float, C::NT>(tr, red);
-  acc.p1 = block_sum<float, C::NT>(acc.p1, red);
-  acc.p3 = block_sum<float, C::NT>(acc.p3, red);
-  return (double)trace;
+  const double trace = gram_trace<NP>(sm);
+  acc.p1 = block_sum<float, C::NT>(acc.p1, sm + S::RED);
+  acc.p3 = block_sum<float, C::NT>(acc.p3, sm + S::RED);
+  return trace;
 }
 
 // Parallel cyclic Jacobi on sm[A] (symmetric, NP x NP), eigenvectors into
