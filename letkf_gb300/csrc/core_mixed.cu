@@ -5,8 +5,8 @@
 //       mtx_eigen's truncation cannot act): W = sqrt((k-1)/s) (A/s)^(-1/2) by
 //       the spectrum-scaled Newton-Schulz iteration, wbar = Z (Z b) / s.
 //   core_mixed_kernel      the points the first launch leaves (status
-//       LETKF_PENDING): the parallel Jacobi eigensolver with the reference's
-//       truncation.
+//       LETKF_PENDING, or MN_PENDING_GRAM with their sums in trans): the
+//       parallel Jacobi eigensolver with the reference's truncation.
 // Outputs FP32 trans / transm with the semantics of
 // common/common_letkf.f90:50-243 (transm present: trans = T, transm = wbar;
 // absent: trans = T + wbar 1^T).

@@ -690,9 +690,8 @@ static int largek_core(int ne, int npts, const int64_t* offs, const float* rows,
   A(&pt, sizeof(LkPoint) * B);
   int st = ok ? LETKF_OK : LETKF_ERR_CUDA;
   if (st == LETKF_OK) st = cuda_status(cudaMemsetAsync(err, 0, sizeof(int), s));
-  // without any observation the points need no product: 8 points of k = 129
-  // 416 us
-  // before the list sums had launches of their own, 456 since, 385 so
+  // without any observation the points need no product: 8 points of k = 129 416
+  // us before the list sums had launches of their own, 456 since, 385 so
   const bool any = nrows > 0;
   if (st == LETKF_OK && any) {
     lk_weights_kernel<<<(unsigned)((nrows + 255) / 256), 256, 0, s>>>(nrows, rdiag, rloc, rdiag_wloc, w);

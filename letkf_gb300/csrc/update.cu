@@ -11,13 +11,17 @@
 // beta + (1 - beta) I, xa = mean + xb' T; beta == 0 leaves mean + xb'; optional
 // clipping of the relative spread of one variable (Q_SPRD_MAX).
 //
-// One CTA per point, one kernel for both entry points (mode 0 where beta is 1,
-// no array or an element of it, is the plain update bit for bit).  The factors
-// that do not depend on k stay out of the sum: t(m) = sum_k x(k) W(k,m) and
-// sum_k x(k) transm(k) once, then xa = mean + beta (fac t + tx) + (1 - beta)
+// update_f64_kernel has one CTA per point and serves both entry points (mode 0
+// where beta is 1, no array or an element of it, is the plain update bit for
+// bit); forms for few members, few variables or few points follow it, with the
+// same operations in the same order.  The factors that do not depend on k stay out
+// of the sum: t(m) = sum_k x(k) W(k,m) and sum_k x(k) transm(k) once, then xa = mean + beta (fac t + tx) + (1 - beta)
 // x(m): one multiply-add per element of W and variable where forming each weight
 // first took five FP64 operations, and increments added up before they meet the
-// mean.
+// mean, in every form: with the mean first each of k additions rounds at its size
+// (error of the plain update against exact arithmetic, merged weights, of the rms
+// value: k = 8 1.5e-16 so and 8.1e-17 here, k = 40 2.9e-16 and 9.4e-17, k = 100 4.3e-16
+// and 1.3e-16).
 //
 // Bound: the FP64 pipe (1.2 TFLOP/s; a warp instruction takes 16 cycles of an
 // SM), so lanes are kept full: outputs (variable, member) are flattened over
@@ -72,7 +76,6 @@ __global__ void __launch_bounds__(UPD_NT) update_f64_kernel(int n, int npts, int
                                                              const double* __restrict__ trans,
                                                              const double* __restrict__ transm,
                                                              const double* __restrict__ pao, RelaxArgs r, double* xa) {
-  constexpr bool PLAIN = MODE == 0 && !BETA;
   extern __shared__ __align__(16) double su[];
   const int ld = n | 1, nh = n / 2;
   // W(k, m) at k sk + m sm: as in memory, or transposed where the row length
@@ -89,7 +92,6 @@ __global__ void __launch_bounds__(UPD_NT) update_f64_kernel(int n, int npts, int
   double* bet = fac + vcm;
   double* tx = bet + vcm;
   double* qv = tx + vcm;                   // [n]
-  __shared__ int one[UPD_VC];              // mode 0 with a beta array: beta is 1
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   for (int pl = blockIdx.x; pl < cnt; pl += gridDim.x) {
     const int p = p0 + pl;
@@ -139,10 +141,6 @@ __global__ void __launch_bounds__(UPD_NT) update_f64_kernel(int n, int npts, int
         mean[v] = s / (double)n;
         if (BETA) bet[v] = r.beta[(size_t)(v0 + v) * npts + p];
         fac[v] = 1.0;
-        if (MODE == 0 && BETA) {
-          one[v] = bet[v] == 1.0;
-          fac[v] = one[v] ? mean[v] : 0.0;  // what the sum of an output starts from
-        }
       }
       __syncthreads();
       for (int t = tid; t < total; t += UPD_NT) xp[t] = xp[t] - mean[t / n];
@@ -188,7 +186,6 @@ __global__ void __launch_bounds__(UPD_NT) update_f64_kernel(int n, int npts, int
           }
           if ((lane & 7) == 0 && vb + (lane >> 3) < vc) {
             tx[v] = sx;
-            if (MODE == 0 && BETA && one[v]) fac[v] = mean[v] + sx;
             if (MODE == 2) {  // beta == 0 skips weight_RTPS (factor 1)
               double f = 1.0;
               if ((!BETA || bet[v] != 0.0) && vg > 0.0 && va > 0.0)
@@ -211,9 +208,7 @@ __global__ void __launch_bounds__(UPD_NT) update_f64_kernel(int n, int npts, int
           const int t = min(32 * (c0 + u * (UPD_NT / 32)) + lane, total - 1);
           vv[u] = t / n;
           mm[u] = t - vv[u] * n;
-          // the plain update, and where beta is 1, adds up from the mean, as the reference does
-          a[u] = PLAIN ? mean[vv[u]] : MODE == 0 ? fac[vv[u]] : 0.0;
-          if (PLAIN && transm) a[u] = a[u] + tx[vv[u]];
+          a[u] = 0.0;
           off[u] = mm[u] * sm;
         }
         // one loop per count: a multiply-add that is only predicated off takes its FP64 slot
@@ -231,17 +226,14 @@ __global__ void __launch_bounds__(UPD_NT) update_f64_kernel(int n, int npts, int
           const int v = vv[u], m = mm[u];
           const double x = xp[v * n + m];
           double inc = a[u];
-          if (!PLAIN && !(MODE == 0 && one[v])) {
-            if (MODE == 1) inc = (1.0 - r.alpha) * inc + r.alpha * x;
-            if (MODE == 2) inc = fac[v] * inc;
-            if (transm) inc = inc + tx[v];
-            if (BETA) {
-              const double b = bet[v];
-              inc = b == 0.0 ? x : b == 1.0 ? inc : b * inc + (1.0 - b) * x;
-            }
-            inc = mean[v] + inc;
+          if (MODE == 1) inc = (1.0 - r.alpha) * inc + r.alpha * x;
+          if (MODE == 2) inc = fac[v] * inc;
+          if (transm) inc = inc + tx[v];
+          if (BETA) {
+            const double b = bet[v];
+            inc = b == 0.0 ? x : b == 1.0 ? inc : b * inc + (1.0 - b) * x;
           }
-          const double y = inc;
+          const double y = mean[v] + inc;
           if (clip && v0 + v == r.q_var)
             qv[m] = y;
           else
@@ -340,10 +332,10 @@ __global__ void __launch_bounds__(UPD_NT) update_point_kernel(int n, int npts, i
       for (int t = tid; t < total; t += UPD_NT) {
         const int v = t / n, m = t - v * n;
         const double *x = xp + v * n, *w = W + m * sm;
-        double a = mean[v];
-        if (TM) a = a + tx[v];
+        double a = 0.0;
         for (int k = 0; k < n; k++) a = fma(x[k], w[k * sk], a);
-        xa[((size_t)(v0 + v) * npts + p) * n + m] = a;
+        if (TM) a = a + tx[v];
+        xa[((size_t)(v0 + v) * npts + p) * n + m] = mean[v] + a;
       }
     }
   }
@@ -389,8 +381,9 @@ __global__ void __launch_bounds__(UPD_NT, 8) update_rows_kernel(int n, int npts,
   // pb points of NVT rows each in a batch
   extern __shared__ __align__(16) double su[];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, ld = n | 1;
-  double* xs = su + (size_t)wid * pb * NVT * (ld + 1);  // [point][variable][ld]
-  double* tx = xs + pb * NVT * ld;
+  double* xs = su + (size_t)wid * pb * NVT * (ld + 2);  // [point][variable][ld]
+  double* tx = xs + pb * NVT * ld;                      // [point][variable] each
+  double* ms = tx + pb * NVT;
   const int nbatch = (cnt + pb - 1) / pb;
   for (int b = blockIdx.x * (UPD_NT / 32) + wid; b < nbatch; b += gridDim.x * (UPD_NT / 32)) {
     const int q0 = b * pb, nq = min(pb, cnt - q0), nr = nq * NVT;
@@ -406,6 +399,7 @@ __global__ void __launch_bounds__(UPD_NT, 8) update_rows_kernel(int n, int npts,
       double s = x[0];
       for (int m = 1; m < n; m++) s = s + x[m];
       mean = s / (double)n;
+      ms[lane] = mean;
     }
     for (int r = 0; r < nr; r++) {
       const double mr = __shfl_sync(0xffffffffu, mean, r);
@@ -426,14 +420,11 @@ __global__ void __launch_bounds__(UPD_NT, 8) update_rows_kernel(int n, int npts,
     }
     for (int q = 0; q < nq; q++) {
       const double* x = xs + q * NVT * ld;
-      double mr[NVT];
-#pragma unroll
-      for (int v = 0; v < NVT; v++) mr[v] = __shfl_sync(0xffffffffu, mean, q * NVT + v);
       for (int m = lane; m < n; m += 32) {
         const double* w = trans + ((size_t)(q0 + q) * n + m) * n;
         double a[NVT];
 #pragma unroll
-        for (int v = 0; v < NVT; v++) a[v] = transm ? mr[v] + tx[q * NVT + v] : mr[v];
+        for (int v = 0; v < NVT; v++) a[v] = 0.0;
         int k = 0;
         if (VEC) {
           for (; k + 8 <= n; k += 8) {
@@ -456,7 +447,8 @@ __global__ void __launch_bounds__(UPD_NT, 8) update_rows_kernel(int n, int npts,
           for (int v = 0; v < NVT; v++) a[v] = fma(x[v * ld + k], t, a[v]);
         }
 #pragma unroll
-        for (int v = 0; v < NVT; v++) xa[((size_t)v * npts + p0 + q0 + q) * n + m] = a[v];
+        for (int v = 0; v < NVT; v++)
+          xa[((size_t)v * npts + p0 + q0 + q) * n + m] = ms[q * NVT + v] + (transm ? a[v] + tx[q * NVT + v] : a[v]);
       }
     }
   }
@@ -467,7 +459,7 @@ static int launch_update_rows(int ne, int npts, int p0, int cnt, const double* x
                               const double* transm, double* xa, cudaStream_t stream) {
   static std::atomic<uint32_t> done{0};
   const cudaError_t err = set_smem_once(update_rows_kernel<NVT, VEC>,
-                                        sizeof(double) * (UPD_NT / 32) * (size_t)(UPR_ROWS * (LETKF_MAX_NE + 1) + UPR_ROWS), done);
+                                        sizeof(double) * (UPD_NT / 32) * (size_t)(UPR_ROWS * (LETKF_MAX_NE + 1) + 2 * UPR_ROWS), done);
   if (err != cudaSuccess) return cuda_status(err);
   int dev = 0, nsm = 0;
   cudaGetDevice(&dev);
@@ -475,7 +467,7 @@ static int launch_update_rows(int ne, int npts, int p0, int cnt, const double* x
   // full batches only where every SM then still has two rounds of warps
   int pb = cnt / (nsm * 64);
   pb = pb < 1 ? 1 : pb > UPR_ROWS / NVT ? UPR_ROWS / NVT : pb;
-  const size_t smem = sizeof(double) * (UPD_NT / 32) * (size_t)pb * NVT * ((ne | 1) + 1);
+  const size_t smem = sizeof(double) * (UPD_NT / 32) * (size_t)pb * NVT * ((ne | 1) + 2);
   const int need = (cnt + pb * (UPD_NT / 32) - 1) / (pb * (UPD_NT / 32));
   const int grid = need < nsm * 8 ? need : nsm * 8;
   update_rows_kernel<NVT, VEC><<<grid, UPD_NT, smem, stream>>>(ne, npts, p0, cnt, pb, xb, trans, transm, xa);
@@ -584,20 +576,16 @@ __global__ void __launch_bounds__(UPT_NT) update_tiny_kernel(int npts, int p0, i
       if (r.rtps_infl) r.rtps_infl[(size_t)v * npts + p0 + pl] = fac;
     }
     const double* W = trans + (size_t)pl * N * N;  // W(k, m) at m N + k
-    const bool plain = MODE == 0 && b == 1.0;
 #pragma unroll
     for (int m = 0; m < N; m++) {
-      double a = plain ? (transm ? mean + tx : mean) : 0.0;
+      double a = 0.0;
 #pragma unroll
       for (int k = 0; k < N; k++) a = fma(x[k], W[m * N + k], a);
-      if (!plain) {
-        if (MODE == 1) a = (1.0 - r.alpha) * a + r.alpha * x[m];
-        if (MODE == 2) a = fac * a;
-        if (transm) a = a + tx;
-        if (r.beta) a = b == 0.0 ? x[m] : b == 1.0 ? a : b * a + (1.0 - b) * x[m];
-        a = mean + a;
-      }
-      y[m] = a;
+      if (MODE == 1) a = (1.0 - r.alpha) * a + r.alpha * x[m];
+      if (MODE == 2) a = fac * a;
+      if (transm) a = a + tx;
+      if (r.beta) a = b == 0.0 ? x[m] : b == 1.0 ? a : b * a + (1.0 - b) * x[m];
+      y[m] = mean + a;
     }
     if (r.q_sprd_max > 0.0 && v == r.q_var) {
       const double qm = upt_sum<N>(y) / (double)N;
