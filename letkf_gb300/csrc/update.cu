@@ -15,11 +15,11 @@
 // where beta is 1, no array or an element of it, is the plain update bit for
 // bit); forms for few members, few variables or few points follow it, with the
 // same operations in the same order.  The factors that do not depend on k stay out
-// of the sum: t(m) = sum_k x(k) W(k,m) and sum_k x(k) transm(k) once, then xa = mean + beta (fac t + tx) + (1 - beta)
-// x(m): one multiply-add per element of W and variable where forming each weight
-// first took five FP64 operations, and increments added up before they meet the
-// mean, in every form: with the mean first each of k additions rounds at its size
-// (error of the plain update against exact arithmetic, merged weights, of the rms
+// of the sum: t(m) = sum_k x(k) W(k,m) and sum_k x(k) transm(k) once, then xa =
+// mean + beta (fac t + tx) + (1 - beta) x(m): one multiply-add per element of W and
+// variable where forming each weight first took five FP64 operations, and
+// increments added up before they meet the mean, in every form: with the mean
+// first each of k additions rounds at its size (error of the plain update against exact arithmetic, merged weights, of the rms
 // value: k = 8 1.5e-16 so and 8.1e-17 here, k = 40 2.9e-16 and 9.4e-17, k = 100 4.3e-16
 // and 1.3e-16).
 //
@@ -67,17 +67,18 @@ __device__ __forceinline__ void upd_sums(int n, int sk, const double* xp, const 
 }
 
 // Points p0 .. p0+cnt-1 of arrays holding npts points; trans / transm / pao
-// are indexed from p0; vcm variables at a time.  MODE and BETA (r.beta given)
+// are indexed from p0; CAP variables at a time.  MODE and BETA (r.beta given)
 // are compiled in: an operation that is only predicated off still takes its FP64
-// slot.
-template <int MODE, bool BETA>
-__global__ void __launch_bounds__(UPD_NT) update_f64_kernel(int n, int npts, int p0, int cnt, int nv, int vcm,
+// slot; CAP is because a loop of unknown step costs up to 7 % (k = 50, one
+// variable, beta given, 6,000 points: 88 us with it compiled in, 95 without).
+template <int MODE, bool BETA, int CAP>
+__global__ void __launch_bounds__(UPD_NT) update_f64_kernel(int n, int npts, int p0, int cnt, int nv,
                                                              const double* __restrict__ xb,
                                                              const double* __restrict__ trans,
                                                              const double* __restrict__ transm,
                                                              const double* __restrict__ pao, RelaxArgs r, double* xa) {
   extern __shared__ __align__(16) double su[];
-  const int ld = n | 1, nh = n / 2;
+  const int ld = n | 1, nh = n / 2, vcm = nv < CAP ? nv : CAP;
   // W(k, m) at k sk + m sm: as in memory, or transposed where the row length
   // would put the lanes' members on few banks
   const bool tr = n % 16 == 0;
@@ -127,8 +128,8 @@ __global__ void __launch_bounds__(UPD_NT) update_f64_kernel(int n, int npts, int
         if (d != 0 && (2 * d < n || (2 * d == n && j < i))) D[d * n + j] += Pp[idx];
       }
     }
-    for (int v0 = 0; v0 < nv; v0 += vcm) {
-      const int vc = min(vcm, nv - v0), total = vc * n;
+    for (int v0 = 0; v0 < nv; v0 += CAP) {
+      const int vc = min(CAP, nv - v0), total = vc * n;
       if (v0) __syncthreads();
       for (int t = tid; t < total; t += UPD_NT) {
         const int v = t / n;
@@ -483,7 +484,9 @@ static int launch_update_as(int ne, int npts, int p0, int cnt, int nv, const dou
   int vc = nv < UPD_VC ? nv : UPD_VC;
   if (sizeof(double) * upd_smem_doubles(ne, vc, MODE) > 227 * 1024) vc = UPD_VC / 2;
   const size_t smem = sizeof(double) * upd_smem_doubles(ne, vc, MODE);
-  auto kern = update_f64_kernel<MODE, BETA>;
+  auto kern = update_f64_kernel<MODE, BETA, UPD_VC>;
+  if constexpr (MODE == 2)
+    if (vc < nv && vc < UPD_VC) kern = update_f64_kernel<MODE, BETA, UPD_VC / 2>;
   const cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (err != cudaSuccess) return cuda_status(err);
   int dev = 0, nsm = 0;
@@ -493,7 +496,7 @@ static int launch_update_as(int ne, int npts, int p0, int cnt, int nv, const dou
   int per_sm = (int)((size_t)(220 * 1024) / (smem + 1024));
   per_sm = per_sm < 1 ? 1 : per_sm > 8 ? 8 : per_sm;
   const int grid = cnt < nsm * per_sm ? cnt : nsm * per_sm;
-  kern<<<grid, UPD_NT, smem, stream>>>(ne, npts, p0, cnt, nv, vc, xb, trans, transm, pao, r, xa);
+  kern<<<grid, UPD_NT, smem, stream>>>(ne, npts, p0, cnt, nv, xb, trans, transm, pao, r, xa);
   note_launch();
   return cuda_status(cudaGetLastError());
 }
@@ -581,7 +584,7 @@ __global__ void __launch_bounds__(UPT_NT) update_tiny_kernel(int npts, int p0, i
       double a = 0.0;
 #pragma unroll
       for (int k = 0; k < N; k++) a = fma(x[k], W[m * N + k], a);
-      if (MODE == 1) a = (1.0 - r.alpha) * a + r.alpha * x[m];
+      if (MODE == 1) a = fma(r.alpha, x[m], __dmul_rn(1.0 - r.alpha, a));  // as the compiler has it above
       if (MODE == 2) a = fac * a;
       if (transm) a = a + tx;
       if (r.beta) a = b == 0.0 ? x[m] : b == 1.0 ? a : b * a + (1.0 - b) * x[m];
